@@ -18,8 +18,7 @@ struct DevModel {
   int poly_canon;  // coefficients in canonical order: use the generated polynomials
   float h, inv_h, r_cut, ro2_scale;
   const float4* spl0;  // [S*S][nint][4][2][C/2]: channel-pair planes
-  const float4* spl1;      // [npairs][nint][n_instr][2][C/2]: channel-pair planes (adjoint)
-  const float4* spl1_fwd;  // [npairs][nint][n_instr][C]: per-channel cubics (forward)
+  const float4* spl1_fwd;  // [npairs][nint][n_instr][C]: per-channel cubics
   const int* mono0;
   int mono0_off[10];
   const float* coef0;  // [S][nLM][T0][C]
@@ -78,9 +77,9 @@ struct DevModel {
   // sched[0..1]; 0 launches one block per atom.  pgrid is read on the host only.
   int* sched;
   int pgrid[8];
-  // L_max = 2 layer-1 kernels: channel slices per node (one block each) and the offset
-  // between the per-slice partial edge forces in f1 (0: one slice)
+  // L_max = 2 layer-1 forward: channel slices per node (one block each)
   int l2_split;
+  // layer-1 adjoint: the offset between the partial edge forces of its 32-channel slices
   long f1_stride;
   // the engine's status word (mapped host memory): a bounded wait that gave up sets bit 0
   unsigned* status;
@@ -154,11 +153,11 @@ __device__ __forceinline__ fix64 to_fixed(float v) {
   const float tb = fmaf(va, 4096.0f, kMagic);
   const float vb = fmaf(-(tb - kMagic), 1.0f / 4096.0f, va);  // va - b 2^-12
   const float tc = fmaf(vb, 17179869184.0f, kMagic);
-  const int a = __float_as_int(ta) - 0x4B400000, b = __float_as_int(tb) - 0x4B400000,
-            c = __float_as_int(tc) - 0x4B400000;
-  // a 2^44 + b 2^22 + c
-  return (static_cast<fix64>(static_cast<long long>(a)) << 44) + (static_cast<fix64>(static_cast<long long>(b)) << 22) +
-         static_cast<fix64>(static_cast<long long>(c));
+  // a 2^44 + b 2^22 + c, modulo 2^64: the words hold 0x4B400000 (kMagic's) more than a, b
+  // and c, taken off as one constant
+  constexpr fix64 kWord = 0x4B400000ull, kBias = (kWord << 44) + (kWord << 22) + kWord;
+  const unsigned a = __float_as_uint(ta), b = __float_as_uint(tb), c = __float_as_uint(tc);
+  return (static_cast<fix64>(a << 12) << 32) + ((static_cast<fix64>(b) << 22) + c) - kBias;
 }
 __device__ __forceinline__ void add_fixed(fix64* dst, float v) { atomicAdd(dst, to_fixed(v)); }
 // q 2^-34 as a float without float64 arithmetic (whose conversions run on this part's

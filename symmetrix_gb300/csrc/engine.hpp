@@ -80,7 +80,7 @@ struct smx_engine {
   float *A0 = nullptr, *M0 = nullptr, *H1 = nullptr, *Phi1 = nullptr, *A1 = nullptr, *M1 = nullptr, *H2 = nullptr;
   float *A0_adj = nullptr, *M0_adj = nullptr, *H1_adj = nullptr, *Phi1_adj = nullptr, *A1_adj = nullptr;
   float *M1_adj = nullptr, *H2_adj = nullptr;
-  double* f1 = nullptr;  // layer-1 edge forces (float64 accumulation)
+  float* f1 = nullptr;  // layer-1 edge forces, one partial sum per 32-channel slice
   smx::fix64* H1_adj_fx = nullptr;  // H1_adj accumulator (fixed point: order-independent sums)
   // precision form: bf16 GEMM operands (M0 and H1_adj as [N*nLM][C]; Phi1 and A1_adj
   // regrouped per l as [N*(2l+1)][n_eta*C] and [N*(2l+1)][C])
@@ -157,7 +157,6 @@ struct smx_engine {
     m.r_cut = pm.r_cut;
     m.ro2_scale = pm.ro2_scale;
     m.spl0 = reinterpret_cast<const float4*>(upload(pm.spl0));
-    m.spl1 = reinterpret_cast<const float4*>(upload(pm.spl1));
     m.spl1_fwd = reinterpret_cast<const float4*>(upload(pm.spl1_fwd));
     m.mono0 = upload(pm.mono0);
     for (int q = 0; q < 10; ++q) m.mono0_off[q] = q < static_cast<int>(pm.mono0_off.size()) ? pm.mono0_off[q] : pm.mono0_off.back();
@@ -332,9 +331,8 @@ struct smx_engine {
     A1_adj = dalloc<float>(nN * 16 * C);
     M1_adj = dalloc<float>(nN * C);
     H2_adj = dalloc<float>(nN * C);
-    // L_max = 2 with two channel slices: one f1 slice each
-    dm.f1_stride = l2_split_max > 1 ? 3 * nE : 0;
-    f1 = dalloc<double>(3 * nE * l2_split_max);
+    dm.f1_stride = 3 * nE;
+    f1 = dalloc<float>(3 * nE * (C >> 5));
     zbl_e = dalloc<float>(nN);
     first = dalloc<int>(nN + 1);
     ntype = dalloc<int>(nN);
@@ -524,17 +522,16 @@ struct smx_engine {
     for (int k = 0; k < smx::kAkCount; ++k) dm.pgrid[k] = mode ? pfull[k] : 0;
   }
 
-  // the persistent grids of the layer-1 kernels follow their block shape
+  // the persistent grid of the layer-1 forward follows its block shape
   void set_l2_split(int ns) {
     dm.l2_split = ns;
     int nsm = 0, per_sm[smx::kAkCount] = {};
     check(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device), "cudaDeviceGetAttribute");
     smx::layer1_residency(dm, per_sm);
-    for (int k : {smx::kAkLayer1Fwd, smx::kAkLayer1Rev}) {
-      const bool on = dm.pgrid[k] > 0;
-      pfull[k] = per_sm[k] * nsm;
-      if (on) dm.pgrid[k] = pfull[k];
-    }
+    const int k = smx::kAkLayer1Fwd;
+    const bool on = dm.pgrid[k] > 0;
+    pfull[k] = per_sm[k] * nsm;
+    if (on) dm.pgrid[k] = pfull[k];
   }
 
   void tune_sched(const smx::EdgeIn& in, double* out_e, double* out_f, cudaStream_t s, int n1) {
@@ -559,17 +556,16 @@ struct smx_engine {
       const int q = kStageOf[k];
       dm.pgrid[k] = best[1][q] < best[0][q] ? pfull[k] : 0;
     }
-    if (l2_split_max > 1) {  // channel slices of the L_max = 2 layer-1 kernels: stages 2 and 6
+    if (l2_split_max > 1) {  // channel slices of the L_max = 2 layer-1 forward: stage 2
       float t[3] = {1e30f, 1e30f, 1e30f};
       for (int rep = 0; rep < 2; ++rep)
         for (int ns = 1; ns <= l2_split_max; ++ns) {
           set_l2_split(ns);
           run_pass(in, out_e, out_f, s, n1);
           check(cudaEventSynchronize(ev[kStages]), "autotune");
-          float a = 0.0f, b = 0.0f;
+          float a = 0.0f;
           check(cudaEventElapsedTime(&a, ev[2], ev[3]), "cudaEventElapsedTime");
-          check(cudaEventElapsedTime(&b, ev[6], ev[7]), "cudaEventElapsedTime");
-          t[ns] = std::min(t[ns], a + b);
+          t[ns] = std::min(t[ns], a);
         }
       set_l2_split(t[1] <= t[2] ? 1 : 2);
     }
@@ -662,7 +658,7 @@ struct smx_engine {
     smx::launch_rows_to_fixed(H1_adj, H1_adj_fx, nh, zero_h1adj, s);
     smx::launch_layer1_rev(m, in, H1, Phi1_adj, H1_adj_fx, f1, s);
     smx::launch_fixed_rows(H1_adj_fx, H1_adj, nullptr, in.N * static_cast<long>(dm.nLM), dm.C, 1, dm.nLM, s);
-    smx::launch_forces_from_f1(forces, f1, dm.f1_stride, dm.l2_split, 3 * E, zero_dxyz, s);
+    smx::launch_forces_from_f1(forces, f1, dm.f1_stride, dm.C >> 5, 3 * E, zero_dxyz, s);
   }
 
   // The full forward + adjoint pass on device-resident inputs (tuning the atom schedule

@@ -332,7 +332,7 @@ __global__ void __launch_bounds__(256) k_contract0_rev(DevModel m, const int* __
 // this edge computes.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void layer0_rev_atom(const DevModel& m, const EdgeIn& in, const float* __restrict__ A0_adj,
-                                                const double* __restrict__ f1, double* __restrict__ forces, int i) {
+                                                const float* __restrict__ f1, double* __restrict__ forces, int i) {
   __shared__ L0Stage<true> st;
   __shared__ float sF[kEdgeChunk][8][3];
   const int C = m.C, C2 = C >> 1;
@@ -415,11 +415,17 @@ __device__ __forceinline__ void layer0_rev_atom(const DevModel& m, const EdgeIn&
         const double g = static_cast<double>(m.dens_c[0][i]) * static_cast<double>(d) / r;
         for (int a = 0; a < 3; ++a) s[a] -= g * in.xyz[3 * e + a];
       }
+      if (m.dens_spl[1] && local) {  // and through the layer-1 one (mace.cpp:744-749)
+        float v, d;
+        const double r = in.r[e];
+        dens_eval(m, 1, ti, in.ntype_e[e], static_cast<float>(r), v, d);
+        const double g = static_cast<double>(m.dens_c[1][i]) * static_cast<double>(d) / r;
+        for (int a = 0; a < 3; ++a) s[a] -= g * in.xyz[3 * e + a];
+      }
       for (int a = 0; a < 3; ++a) {
         double f = 0.0;
         if (local) {
-          f = f1[3 * e + a];
-          for (int h = 1; h < m.l2_split; ++h) f += f1[h * m.f1_stride + 3 * e + a];  // channel slices (L_max = 2)
+          for (int h = 0; h < C >> 5; ++h) f += static_cast<double>(f1[h * m.f1_stride + 3 * e + a]);  // channel slices
         }
         forces[3 * e + a] = -(s[a] + f);
       }
@@ -429,7 +435,7 @@ __device__ __forceinline__ void layer0_rev_atom(const DevModel& m, const EdgeIn&
 
 template <bool P>
 __global__ void __launch_bounds__(128) k_layer0_rev(DevModel m, EdgeIn in, const float* __restrict__ A0_adj,
-                                                    const double* __restrict__ f1, double* __restrict__ forces) {
+                                                    const float* __restrict__ f1, double* __restrict__ forces) {
   pdl_begin();
   AtomCursor cur{P ? m.sched : nullptr, in.N, 0};
   for (int b = cur.first(); b < in.N; b = cur.next())
@@ -471,7 +477,7 @@ void launch_layer0_fwd(const DevModel& m, const EdgeIn& in, float* A0, float* M0
   });
 }
 
-void launch_layer0_rev(const DevModel& m, const EdgeIn& in, const float* A0, const float* M0_adj, const double* f1,
+void launch_layer0_rev(const DevModel& m, const EdgeIn& in, const float* A0, const float* M0_adj, const float* f1,
                        float* A0_adj, double* forces, cudaStream_t s) {
   if (in.N <= 0) return;
   DevModel mk;

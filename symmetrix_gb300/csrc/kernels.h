@@ -16,16 +16,17 @@ void layer0_residency(const DevModel& m, int* per_sm);
 void layer1_residency(const DevModel& m, int* per_sm);
 void node_tail_residency(const DevModel& m, int* per_sm);
 void launch_layer0_fwd(const DevModel& m, const EdgeIn& in, float* A0, float* M0, float* zbl_e, cudaStream_t s);
-void launch_layer0_rev(const DevModel& m, const EdgeIn& in, const float* A0, const float* M0_adj, const double* f1,
+void launch_layer0_rev(const DevModel& m, const EdgeIn& in, const float* A0, const float* M0_adj, const float* f1,
                        float* A0_adj, double* forces, cudaStream_t s);
 
 // k_layer1.cu
 cudaError_t init_layer1_kernels(const DevModel& m);
-int layer1_block(int C);
 void launch_layer1_fwd(const DevModel& m, const EdgeIn& in, const float* H1, float* Phi1, cudaStream_t s);
 // H1_adj: fixed-point accumulator (see to_fixed), seeded by launch_node_tail
+// k_layer1_rev.cu: f1 receives the edge forces' sums over each 32-channel slice, f1_stride apart
+int layer1_rev_residency(const DevModel& m);
 void launch_layer1_rev(const DevModel& m, const EdgeIn& in, const float* H1, const float* dPhi1, fix64* H1_adj,
-                       double* f1, cudaStream_t s);
+                       float* f1, cudaStream_t s);
 
 // k_node.cu
 // One segment of a row-gathered GEMM  Y[rows, ncols] = X[rows, K] @ B[K, ncols].
@@ -59,7 +60,7 @@ void launch_fixed_rows(const fix64* src, float* dst, __nv_bfloat16* bf, long row
 // single-stage calls: dst = fixed-point copy of src (zero: dst = 0); forces = (zero ? 0 :
 // forces) - the sum of the nslices f1 slices (stride apart), n = 3 * edges
 void launch_rows_to_fixed(const float* src, fix64* dst, long n, bool zero, cudaStream_t s);
-void launch_forces_from_f1(double* forces, const double* f1, long stride, int nslices, long n, bool zero,
+void launch_forces_from_f1(double* forces, const float* f1, long stride, int nslices, long n, bool zero,
                            cudaStream_t s);
 void launch_scan_first(const int* num_neigh, int N, int* first, cudaStream_t s);
 // input check of the host API (bits of the flags word)
