@@ -17,6 +17,7 @@ struct DevModel {
   int S, C, L_max, nLM, n_lme, n_instr, n_p, nint, T0, T1, n_hidden;
   int poly_canon;  // coefficients in canonical order: use the generated polynomials
   float h, inv_h, r_cut, ro2_scale;
+  double hd;  // knot spacing of the radial splines in float64 (spline_at)
   const float4* spl0;  // [S*S][nint][4][2][C/2]: channel-pair planes
   const float4* spl1_fwd;  // [npairs][nint][n_instr][C]: per-channel cubics
   const int* mono0;
@@ -36,9 +37,9 @@ struct DevModel {
   const int* cg_rev_off;
   const int* cg_rev_lme;
   const float* cg_rev_v;
-  // the same table padded to two terms per path, (lme, float bits of the value), zero
-  // terms as (0, 0); nullptr when some path has more terms
-  const int2* cg_rev_pad;
+  // the coefficients of path p's terms in the canonical zero pattern (cg_canon.h), 0 where
+  // there is none; nullptr when the model's table has another pattern
+  const float2* cg_val;
   int lme_off[4], num_e[4];
   const float* A1W[4];
   const float* A1W_T[4];
@@ -77,8 +78,6 @@ struct DevModel {
   // sched[0..1]; 0 launches one block per atom.  pgrid is read on the host only.
   int* sched;
   int pgrid[8];
-  // L_max = 2 layer-1 forward: channel slices per node (one block each)
-  int l2_split;
   // layer-1 adjoint: the offset between the partial edge forces of its 32-channel slices
   long f1_stride;
   // the engine's status word (mapped host memory): a bounded wait that gave up sets bit 0
@@ -139,6 +138,13 @@ struct AtomCursor {
 // |H1_adj| < 2^29 (5.4e8, far above any model's dE/dH1: O(1)); resolution 2^-34
 // (5.8e-11, far below the float32 rounding of a term).
 using fix64 = unsigned long long;
+// a 2^44 + b 2^22 + c, modulo 2^64, from the floats whose words hold 0x4B400000 (that of
+// 1.5 2^23) more than a, b and c: the excess is taken off as one constant
+__device__ __forceinline__ fix64 fixed_words(float ta, float tb, float tc) {
+  constexpr fix64 kWord = 0x4B400000ull, kBias = (kWord << 44) + (kWord << 22) + kWord;
+  const unsigned a = __float_as_uint(ta), b = __float_as_uint(tb), c = __float_as_uint(tc);
+  return (static_cast<fix64>(a << 12) << 32) + ((static_cast<fix64>(b) << 22) + c) - kBias;
+}
 // round(v 2^34) as an int64, round-to-nearest-even, for |v| < 2^29, in three exact FP32
 // steps and no conversion instruction (whose issue cost is several times these): v is
 // split as a 2^10 + b 2^-12 + c 2^-34 with a, b, c integers of at most 22 bits, each
@@ -153,13 +159,21 @@ __device__ __forceinline__ fix64 to_fixed(float v) {
   const float tb = fmaf(va, 4096.0f, kMagic);
   const float vb = fmaf(-(tb - kMagic), 1.0f / 4096.0f, va);  // va - b 2^-12
   const float tc = fmaf(vb, 17179869184.0f, kMagic);
-  // a 2^44 + b 2^22 + c, modulo 2^64: the words hold 0x4B400000 (kMagic's) more than a, b
-  // and c, taken off as one constant
-  constexpr fix64 kWord = 0x4B400000ull, kBias = (kWord << 44) + (kWord << 22) + kWord;
-  const unsigned a = __float_as_uint(ta), b = __float_as_uint(tb), c = __float_as_uint(tc);
-  return (static_cast<fix64>(a << 12) << 32) + ((static_cast<fix64>(b) << 22) + c) - kBias;
+  return fixed_words(ta, tb, tc);
 }
 __device__ __forceinline__ void add_fixed(fix64* dst, float v) { atomicAdd(dst, to_fixed(v)); }
+// two values at once, the same steps in packed FP32
+__device__ __forceinline__ void add_fixed2(fix64* d0, fix64* d1, float2 v) {
+  const float2 magic = make_float2(12582912.0f, 12582912.0f), neg = make_float2(-12582912.0f, -12582912.0f);
+  auto dup = [](float x) { return make_float2(x, x); };
+  const float2 ta = __ffma2_rn(v, dup(1.0f / 1024.0f), magic);
+  const float2 va = __ffma2_rn(__fadd2_rn(ta, neg), dup(-1024.0f), v);
+  const float2 tb = __ffma2_rn(va, dup(4096.0f), magic);
+  const float2 vb = __ffma2_rn(__fadd2_rn(tb, neg), dup(-1.0f / 4096.0f), va);
+  const float2 tc = __ffma2_rn(vb, dup(17179869184.0f), magic);
+  atomicAdd(d0, fixed_words(ta.x, tb.x, tc.x));
+  atomicAdd(d1, fixed_words(ta.y, tb.y, tc.y));
+}
 // q 2^-34 as a float without float64 arithmetic (whose conversions run on this part's
 // slow float64 pipe): q = a 2^44 + b 2^22 + c with a signed, b and c in [0, 2^22), all
 // exact as floats; t = a 2^10 + b 2^-12 is exact when |q 2^-34| < 2^10 (then |a 2^22 + b|
@@ -291,6 +305,17 @@ struct EdgeIn {
   __device__ __forceinline__ int atom_at(int b) const { return order ? order[b] : b; }
   __device__ __forceinline__ int end(int i) const { return last ? last[i] : first[i + 1]; }
 };
+
+// The spline interval of edge length r and the offset inside it, rounded once: formed from a
+// float32 r it would carry half an ulp of r (1.2e-7 at 2 A), which the radials' slope turns
+// into the largest single error of the forces (400-atom box after 205 MD steps, rms against
+// float64: 6.6e-7 eV/A from the float32 r, 4.6e-7 from the float64 one).
+__device__ __forceinline__ int spline_at(const DevModel& m, double r, float& x) {
+  int iv = static_cast<int>(static_cast<float>(r) * m.inv_h);
+  iv = iv < 0 ? 0 : (iv >= m.nint ? m.nint - 1 : iv);
+  x = static_cast<float>(fma(-static_cast<double>(iv), m.hd, r));
+  return iv;
+}
 
 // Canonical layer-1 tensor-product instructions (l1 from Y_lm, l2 from H1),
 // ordered by output l; the loader reorders model data to this order.

@@ -153,6 +153,7 @@ struct smx_engine {
     m.poly_canon = pm.poly_canon;
     m.n_hidden = pm.n_hidden;
     m.h = pm.h;
+    m.hd = hm.spl_h;
     m.inv_h = static_cast<float>(1.0 / hm.spl_h);
     m.r_cut = pm.r_cut;
     m.ro2_scale = pm.ro2_scale;
@@ -193,24 +194,12 @@ struct smx_engine {
       cg_fwd_pad_keep = m.cg_fwd_pad;
       cg_fwd_kp_keep = m.cg_fwd_kp;
     }
-    {  // two-term padded copy: the adjoint kernels then gather g with independent loads
-      const int np = static_cast<int>(pm.cg_rev_off.size()) - 1;
-      bool fits = np > 0;
-      for (int p = 0; p < np && fits; ++p) fits = pm.cg_rev_off[p + 1] - pm.cg_rev_off[p] <= 2;
-      m.cg_rev_pad = nullptr;
-      if (fits) {
-        std::vector<int> pad(static_cast<size_t>(4) * np, 0);
-        for (int p = 0; p < np; ++p)
-          for (int q = pm.cg_rev_off[p], t = 0; q < pm.cg_rev_off[p + 1]; ++q, ++t) {
-            float v = pm.cg_rev_v[q];
-            int bits;
-            std::memcpy(&bits, &v, sizeof(bits));
-            pad[4 * p + 2 * t] = pm.cg_rev_lme[q];
-            pad[4 * p + 2 * t + 1] = bits;
-          }
-        m.cg_rev_pad = reinterpret_cast<const int2*>(upload(pad));
-      }
-      cg_rev_pad_keep = m.cg_rev_pad;
+    {  // the coefficients in the canonical zero pattern, when the table fits it
+      std::vector<float> val;
+      m.cg_val = smx::canonical_cg(pm.L_max, pm.cg_rev_off, pm.cg_rev_lme, pm.cg_rev_v, pm.lme_off, pm.num_e, val)
+                     ? reinterpret_cast<const float2*>(upload(val))
+                     : nullptr;
+      cg_val_keep = m.cg_val;
     }
     for (int l = 0; l < 4; ++l) {
       m.lme_off[l] = pm.lme_off[l];
@@ -229,10 +218,6 @@ struct smx_engine {
     m.has_zbl = pm.has_zbl;
     m.op_m0 = m.op_phi1 = m.op_a1adj = nullptr;
     m.tc_terms = tc_terms;
-    // two blocks per node (half the channels each) let two L_max = 2 layer-1 blocks share
-    // an SM: one computes while the other waits at a barrier
-    l2_split_max = (pm.L_max == 2 && pm.C >= 64) ? 2 : 1;
-    m.l2_split = l2_split_max;
     m.f1_stride = 0;
     m.zbl_p = pm.zbl_p;
     for (int q = 0; q < 4; ++q) m.zbl_c[q] = pm.zbl_c[q];
@@ -482,14 +467,15 @@ struct smx_engine {
     smx::launch_umma_gemms(g, ng, status_dev, s, test);
   }
 
-  // padded Clebsch-Gordan tables (option "cg_padded" 0 switches the kernels to the
-  // compressed-row walk, which models with longer rows always use)
-  const int2 *cg_fwd_pad_keep = nullptr, *cg_rev_pad_keep = nullptr;
+  // canonical and padded Clebsch-Gordan tables (option "cg_padded" 0 switches the kernels to
+  // the compressed-row walk, which models with other tables always use)
+  const int2* cg_fwd_pad_keep = nullptr;
+  const float2* cg_val_keep = nullptr;
   int cg_fwd_kp_keep = 0;
   void use_cg_padded(bool on) {
     dm.cg_fwd_pad = on ? cg_fwd_pad_keep : nullptr;
     dm.cg_fwd_kp = on ? cg_fwd_kp_keep : 0;
-    dm.cg_rev_pad = on ? cg_rev_pad_keep : nullptr;
+    dm.cg_val = on ? cg_val_keep : nullptr;
   }
 
   // ---- centre-atom order of the edge kernels ----
@@ -513,25 +499,11 @@ struct smx_engine {
   // (alternating, two passes each, per-stage CUDA events) and keeps the faster per
   // kernel; the two layer-0 adjoint kernels share one stage and are switched together.
   int pfull[smx::kAkCount] = {};
-  // L_max = 2 layer-1 kernels: channel slices per node, 1 or (from 64 channels) 2, tuned
-  int l2_split_max = 1;
   int sched_force = -1;  // -1: tune; 0: one block per atom; 1: persistent
   bool sched_tuned = false;
 
   void sched_set(int mode) {
     for (int k = 0; k < smx::kAkCount; ++k) dm.pgrid[k] = mode ? pfull[k] : 0;
-  }
-
-  // the persistent grid of the layer-1 forward follows its block shape
-  void set_l2_split(int ns) {
-    dm.l2_split = ns;
-    int nsm = 0, per_sm[smx::kAkCount] = {};
-    check(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device), "cudaDeviceGetAttribute");
-    smx::layer1_residency(dm, per_sm);
-    const int k = smx::kAkLayer1Fwd;
-    const bool on = dm.pgrid[k] > 0;
-    pfull[k] = per_sm[k] * nsm;
-    if (on) dm.pgrid[k] = pfull[k];
   }
 
   void tune_sched(const smx::EdgeIn& in, double* out_e, double* out_f, cudaStream_t s, int n1) {
@@ -555,19 +527,6 @@ struct smx_engine {
     for (int k = 0; k < smx::kAkCount; ++k) {
       const int q = kStageOf[k];
       dm.pgrid[k] = best[1][q] < best[0][q] ? pfull[k] : 0;
-    }
-    if (l2_split_max > 1) {  // channel slices of the L_max = 2 layer-1 forward: stage 2
-      float t[3] = {1e30f, 1e30f, 1e30f};
-      for (int rep = 0; rep < 2; ++rep)
-        for (int ns = 1; ns <= l2_split_max; ++ns) {
-          set_l2_split(ns);
-          run_pass(in, out_e, out_f, s, n1);
-          check(cudaEventSynchronize(ev[kStages]), "autotune");
-          float a = 0.0f;
-          check(cudaEventElapsedTime(&a, ev[2], ev[3]), "cudaEventElapsedTime");
-          t[ns] = std::min(t[ns], a);
-        }
-      set_l2_split(t[1] <= t[2] ? 1 : 2);
     }
     profile = prof;
     sched_tuned = true;

@@ -86,9 +86,7 @@ __device__ __forceinline__ void stage_l0(const DevModel& m, const EdgeIn& in, in
       const float inv = 1.0f / rr;
       st.u[t] = make_float4(vx * inv, vy * inv, vz * inv, 0.0f);
     }
-    int iv = static_cast<int>(rr * m.inv_h);
-    iv = iv < 0 ? 0 : (iv >= m.nint ? m.nint - 1 : iv);
-    st.x[t] = rr - static_cast<float>(iv) * m.h;
+    const int iv = spline_at(m, in.r[e], st.x[t]);
     active = rr < m.r_cut;
     st.row[t] = active ? (ti * m.S + in.ntype_e[e]) * m.nint + iv : -1;
   }

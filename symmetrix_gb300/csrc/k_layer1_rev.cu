@@ -14,60 +14,67 @@
 // the radial term are summed over the lanes four edges at a time through shared memory, and
 // only these sums meet dY_a/dx.
 //
-// What bounds it: issue slots and the packed dependencies between them (64% of the cycles
-// issue, at 12 warps per SM and 168 registers; 255 registers without the spills of 50 bytes,
-// 8 warps: 0.55 -> 0.58 ms).  Against one block per node with two instruction halves of
-// channel pairs, which met at a barrier for every edge (8 warps per SM, 47% of the cycles
-// issuing, four FMAs per path): 4096 atoms, 128 channels, 213k edges 0.733 -> 0.533 ms;
-// L_max = 2, 2197 atoms, 178k edges 2.12 -> 1.15 ms.
+// What bounds it: issue slots (64 to 70% of the cycles issue, at 12 warps per SM and 168
+// registers; 255 registers, 8 warps: 0.55 -> 0.58 ms).  Against one block per node with two
+// instruction halves of channel pairs, which met at a barrier for every edge (8 warps per SM,
+// 47% of the cycles issuing, four FMAs on each of the 88 paths): 4096 atoms, 128 channels,
+// 213k edges 0.733 -> 0.533 ms, and without the paths that reach no output 0.47 ms; L_max = 2,
+// 2197 atoms, 178k edges 2.12 -> 1.15 -> 0.97 ms.
 //
-// L_max = 2 (17 instructions, 243 paths): three instruction groups in turn, by the l of
-// H1: {0, 1} (the ten instructions of L_max = 1) and two halves of l = 2, so that a group's
-// g fits the registers and the H1_adj rows of l = 0, 1 are added once, those of l = 2 twice.
+// L_max = 2 (17 instructions): three instruction groups in turn (layer1.cuh), so that a
+// group's g fits the registers; the H1_adj rows of l = 0, 1 are added once, those of l = 2
+// twice.  (One launch per group, 16 warps per SM for the two of l = 2: the same time.)
 #include <cuda_runtime.h>
 
 #include <algorithm>
 
-#include "device.cuh"
 #include "kernels.h"
+#include "layer1.cuh"
 
 namespace smx {
 
 namespace {
 
-// instruction groups, ordered by l1 (Y_00 = 1: an l1 = 0 instruction has u = g and no dE/dY)
-__host__ __device__ constexpr int rev_groups(int LMAX) { return LMAX == 1 ? 1 : 3; }
-__host__ __device__ constexpr int rev_count(int LMAX, int G) { return G == 0 ? 10 : (G == 1 ? 3 : 4); }
-__host__ __device__ constexpr int rev_ins(int LMAX, int G, int i) {
-  constexpr int a[10] = {0, 3, 2, 1, 6, 5, 4, 9, 8, 7};
-  constexpr int b[10] = {0, 4, 3, 1, 9, 8, 5, 14, 13, 10}, b1[3] = {6, 2, 7}, b2[4] = {11, 15, 12, 16};
-  return LMAX == 1 ? a[i] : (G == 0 ? b[i] : (G == 1 ? b1[i] : b2[i]));
+// has an earlier instruction of the group, or an earlier used path of this one, touched
+// dE/dY_a of its l1 (component b and on of instruction i come next)?
+template <int LMAX, int G, bool CANON>
+__host__ __device__ constexpr bool dY_started(int i, int a, int b) {
+  const int q = grp_ins(LMAX, G, i);
+  for (int w = 0; w <= i; ++w) {
+    const int qw = grp_ins(LMAX, G, w);
+    if (ins_l1(LMAX, qw) != ins_l1(LMAX, q)) continue;
+    for (int v = 0; v < (w < i ? 2 * ins_l2(LMAX, qw) + 1 : b); ++v)
+      if (path_used<LMAX, CANON>(qw, a, v)) return true;
+  }
+  return false;
 }
-// the H1 rows [row0, row0 + rows) that group G reads and adds to
-__host__ __device__ constexpr int rev_row0(int G) { return G == 0 ? 0 : 4; }
-__host__ __device__ constexpr int rev_rows(int G) { return G == 0 ? 4 : 5; }
-__host__ __device__ constexpr int ins_paths(int LMAX, int q) {
-  return (2 * ins_l1(LMAX, q) + 1) * (2 * ins_l2(LMAX, q) + 1);
+// is dE/dY_c touched by the group at all?
+template <int LMAX, int G, bool CANON>
+__host__ __device__ constexpr bool dY_used(int c) {
+  for (int w = 0; w < grp_count(G); ++w) {
+    const int q = grp_ins(LMAX, G, w), l1 = ins_l1(LMAX, q);
+    if (l1 == 0 || c < l1 * l1 || c >= (l1 + 1) * (l1 + 1)) continue;
+    for (int b = 0; b < 2 * ins_l2(LMAX, q) + 1; ++b)
+      if (path_used<LMAX, CANON>(q, c - l1 * l1, b)) return true;
+  }
+  return false;
 }
-// offset of the group's i-th instruction in its path list
-template <int LMAX, int G>
-__host__ __device__ constexpr int rev_goff(int i) {
-  int s = 0;
-  for (int w = 0; w < i; ++w) s += ins_paths(LMAX, rev_ins(LMAX, G, w));
-  return s;
+// is there a used path (q, a' < a, b)?
+template <int LMAX, bool CANON>
+__host__ __device__ constexpr bool u_started(int q, int a, int b) {
+  for (int v = 0; v < a; ++v)
+    if (path_used<LMAX, CANON>(q, v, b)) return true;
+  return false;
 }
-// is the i-th instruction the first of its group with its l1 (l2)?
-template <int LMAX, int G>
-__host__ __device__ constexpr bool rev_first_l1(int i) {
-  for (int w = 0; w < i; ++w)
-    if (ins_l1(LMAX, rev_ins(LMAX, G, w)) == ins_l1(LMAX, rev_ins(LMAX, G, i))) return false;
-  return true;
-}
-template <int LMAX, int G>
-__host__ __device__ constexpr bool rev_first_l2(int i) {
-  for (int w = 0; w < i; ++w)
-    if (ins_l2(LMAX, rev_ins(LMAX, G, w)) == ins_l2(LMAX, rev_ins(LMAX, G, i))) return false;
-  return true;
+// has an earlier instruction of the group added to H1_adj row l2^2 + b of instruction i?
+template <int LMAX, int G, bool CANON>
+__host__ __device__ constexpr bool row_started(int i, int b) {
+  const int q = grp_ins(LMAX, G, i);
+  for (int w = 0; w < i; ++w) {
+    const int qw = grp_ins(LMAX, G, w);
+    if (ins_l2(LMAX, qw) == ins_l2(LMAX, q) && u_started<LMAX, CANON>(qw, 2 * ins_l1(LMAX, qw) + 1, b)) return true;
+  }
+  return false;
 }
 
 constexpr int kSumEdges = 4;  // edges summed over the lanes at a time
@@ -75,39 +82,23 @@ constexpr int kSumRow = 33;   // row pitch of their terms: 32 rows read at one c
 
 // shared memory of one warp
 struct RevSmem {
-  float Y[kEdgeChunk][16];   // Y_lm of the staged edges; then (dE/dR term, dE/dY_1 .. dE/dY_15)
-  int4 meta[kEdgeChunk];     // offset inside the spline interval (float bits), spline row, j
+  EdgeStage st;   // Y rows: once an edge is done, (dE/dr term, dE/dY_1 .. dE/dY_15) in their place
   float2 buf[1];             // [kSumEdges * 8][kSumRow] per-lane terms; before the edges: dPhi1 rows
 };
 
-__device__ __forceinline__ void async_copy4(float* dst, const float* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(static_cast<unsigned>(__cvta_generic_to_shared(dst))),
-               "l"(src)
-               : "memory");
-}
-__device__ __forceinline__ void async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-
 // One edge, group G, this lane's channel; c: the edge's cubics, replaced by those of the
 // next edge (cn); t: this lane's slot of the edge in RevSmem::buf.
-template <int LMAX, int G>
+template <int LMAX, int G, bool CANON>
 __device__ __forceinline__ void rev_edge(const float* g, float4* c, const float4* __restrict__ cn, int C, float x,
                                          const float* Y, const float* h, float* hadj, float2* t) {
   float y[16];
-#pragma unroll
-  for (int v = 0; v < 4; ++v) {
-    const float4 f = *reinterpret_cast<const float4*>(Y + 4 * v);
-    y[4 * v] = f.x;
-    y[4 * v + 1] = f.y;
-    y[4 * v + 2] = f.z;
-    y[4 * v + 3] = f.w;
-  }
-  constexpr int r0 = rev_row0(G);
+  read_Y(Y, y);
+  constexpr int r0 = grp_row0(G);
   float dY[16], dr = 0.0f;
-  static_for<rev_count(LMAX, G)>([&](auto ic) {
+  static_for<grp_count(G)>([&](auto ic) {
     constexpr int i = decltype(ic)::value;
-    constexpr int q = rev_ins(LMAX, G, i);
-    constexpr int l1 = ins_l1(LMAX, q), l2 = ins_l2(LMAX, q), g0 = rev_goff<LMAX, G>(i), nb = 2 * l2 + 1;
-    constexpr bool first1 = rev_first_l1<LMAX, G>(i), first2 = rev_first_l2<LMAX, G>(i);
+    constexpr int q = grp_ins(LMAX, G, i);
+    constexpr int l1 = ins_l1(LMAX, q), l2 = ins_l2(LMAX, q), nb = 2 * l2 + 1;
     // value and derivative by the two-row Horner scheme
     float R = fmaf(c[i].w, x, c[i].z);
     float Rd = fmaf(c[i].w, x, R);
@@ -118,28 +109,30 @@ __device__ __forceinline__ void rev_edge(const float* g, float4* c, const float4
     float us[nb], rh[nb];
 #pragma unroll
     for (int b = 0; b < nb; ++b) rh[b] = R * h[l2 * l2 - r0 + b];
-#pragma unroll
-    for (int a = 0; a < 2 * l1 + 1; ++a) {
-#pragma unroll
-      for (int b = 0; b < nb; ++b) {
-        const float gp = g[g0 + a * nb + b];
-        if constexpr (l1 == 0) {
-          us[b] = gp;
-        } else {
-          us[b] = a == 0 ? gp * y[l1 * l1] : fmaf(gp, y[l1 * l1 + a], us[b]);
-          dY[l1 * l1 + a] = (first1 && b == 0) ? gp * rh[b] : fmaf(gp, rh[b], dY[l1 * l1 + a]);
-        }
+    for_paths<LMAX, G, CANON, i>([&](auto ac, auto bc, auto pc) {
+      constexpr int a = decltype(ac)::value, b = decltype(bc)::value;
+      const float gp = g[decltype(pc)::value];
+      if constexpr (l1 == 0) {
+        us[b] = gp;
+      } else {
+        us[b] = u_started<LMAX, CANON>(q, a, b) ? fmaf(gp, y[l1 * l1 + a], us[b]) : gp * y[l1 * l1 + a];
+        float& d = dY[l1 * l1 + a];
+        d = dY_started<LMAX, G, CANON>(i, a, b) ? fmaf(gp, rh[b], d) : gp * rh[b];
       }
-    }
-    float w = us[0] * h[l2 * l2 - r0];
-#pragma unroll
-    for (int b = 1; b < nb; ++b) w = fmaf(us[b], h[l2 * l2 - r0 + b], w);
+    });
+    float w = 0.0f;
+    static_for<nb>([&](auto bc) {
+      constexpr int b = decltype(bc)::value;
+      if constexpr (u_started<LMAX, CANON>(q, 2 * l1 + 1, b)) {
+        w = fmaf(us[b], h[l2 * l2 - r0 + b], w);
+        float& o = hadj[l2 * l2 - r0 + b];
+        o = row_started<LMAX, G, CANON>(i, b) ? fmaf(R, us[b], o) : R * us[b];
+      }
+    });
     dr = i == 0 ? w * Rd : fmaf(w, Rd, dr);
-#pragma unroll
-    for (int b = 0; b < nb; ++b) {
-      float& o = hadj[l2 * l2 - r0 + b];
-      o = first2 ? R * us[b] : fmaf(R, us[b], o);
-    }
+  });
+  static_for<16>([&](auto cc) {
+    if constexpr (decltype(cc)::value > 0 && !dY_used<LMAX, G, CANON>(decltype(cc)::value)) dY[decltype(cc)::value] = 0.0f;
   });
   t[0] = make_float2(dr, dY[1]);
 #pragma unroll
@@ -161,56 +154,50 @@ __device__ __forceinline__ void rev_sums(RevSmem& s, int a0, int n) {
       p2 = __fadd2_rn(p2, row[i + 2]);
       p3 = __fadd2_rn(p3, row[i + 3]);
     }
-    *reinterpret_cast<float2*>(&s.Y[a0 + e][2 * v]) = __fadd2_rn(__fadd2_rn(p0, p1), __fadd2_rn(p2, p3));
+    *reinterpret_cast<float2*>(&s.st.Y[a0 + e][2 * v]) = __fadd2_rn(__fadd2_rn(p0, p1), __fadd2_rn(p2, p3));
   }
   __syncwarp();
 }
 
-// Group G over the edges of chunks `split` apart; `add`: the edge forces of an earlier group
+// Group G over the edges of chunks `split` apart; the edge forces of the earlier groups
 // of the same warp are in f1 already.
-template <int LMAX, int G, int CT>
+template <int LMAX, int G, int CT, bool CANON>
 __device__ __forceinline__ void rev_group(const DevModel& m, const EdgeIn& in, const float* __restrict__ H1,
                                           const float* __restrict__ dPhi1, fix64* __restrict__ H1_adj,
                                           float* __restrict__ f1, RevSmem& s, int i, int k, int part, int split,
                                           int cs) {
   constexpr int NI = ins_count(LMAX), NL2 = (LMAX + 1) * (LMAX + 1);
-  constexpr int NQ = rev_count(LMAX, G), NP = rev_goff<LMAX, G>(NQ), NR = rev_rows(G), r0 = rev_row0(G);
+  constexpr int NQ = grp_count(G), NP = grp_off<LMAX, G, CANON>(NQ), NR = grp_rows(G), r0 = grp_row0(G);
   const int C = CT > 0 ? CT : m.C;
   const int lane = threadIdx.x & 31;
   const int ti = in.node_type[i];
   const int e0 = in.first[i], e1 = in.end(i);
-  // g of this lane's channel from the node's dPhi1 rows
-  float g[NP];
-  float* sD = reinterpret_cast<float*>(s.buf);  // [n_lme][32]
-  __syncwarp();
-  for (int lme = 0; lme < m.n_lme; ++lme)  // (a lane reads only its own column back)
-    async_copy4(sD + lme * 32 + lane, dPhi1 + (static_cast<size_t>(i) * m.n_lme + lme) * C + k);
-  // this lane's edge of a chunk; the first chunk's loads overlap the copies
-  float vx, vy, vz, rr;
-  int tj, nj;
-  auto load = [&](int eb) {
-    const long e = min(eb + lane, e1 - 1);
-    vx = static_cast<float>(in.xyz[3 * e]);
-    vy = static_cast<float>(in.xyz[3 * e + 1]);
-    vz = static_cast<float>(in.xyz[3 * e + 2]);
-    rr = static_cast<float>(in.r[e]);
-    tj = in.ntype_e[e];
-    nj = in.nidx[e];
-  };
-  load(e0 + part * cs);
-  async_wait();
-  if (m.cg_rev_pad) {  // two terms per path, all loads independent
+  float g[NP];  // of this lane's channel, from the node's dPhi1 rows
+  LaneEdge ed;
+  ed.load(m, in, min(e0 + part * cs + lane, e1 - 1));
+  if constexpr (CANON) {  // one or two terms per path, from the instruction's rows
     static_for<NQ>([&](auto ic) {
       constexpr int w = decltype(ic)::value;
-      constexpr int q = rev_ins(LMAX, G, w), p0 = ins_poff(LMAX, q), g0 = rev_goff<LMAX, G>(w);
+      constexpr int q = grp_ins(LMAX, G, w), l = ins_l(LMAX, q), p0 = ins_poff(LMAX, q), nb = 2 * ins_l2(LMAX, q) + 1;
+      float D[2 * l + 1];
 #pragma unroll
-      for (int p = 0; p < ins_paths(LMAX, q); ++p) {
-        const int4 tt = __ldg(reinterpret_cast<const int4*>(m.cg_rev_pad) + p0 + p);
-        g[g0 + p] = fmaf(__int_as_float(tt.w), sD[tt.z * 32 + lane], __int_as_float(tt.y) * sD[tt.x * 32 + lane]);
-      }
+      for (int v = 0; v < 2 * l + 1; ++v)
+        D[v] = __ldg(dPhi1 + (static_cast<size_t>(i) * l1_rows(LMAX) + ins_row(LMAX, q) + v * ins_ne(LMAX, l)) * C + k);
+      for_paths<LMAX, G, CANON, w>([&](auto ac, auto bc, auto pc) {
+        constexpr int p = p0 + decltype(ac)::value * nb + decltype(bc)::value;
+        const float2 cg = __ldg(m.cg_val + p);
+        float v = cg.x * D[cg_m(LMAX, p, 0)];
+        if constexpr (cg_m(LMAX, p, 1) >= 0) v = fmaf(cg.y, D[cg_m(LMAX, p, 1)], v);
+        g[decltype(pc)::value] = v;
+      });
     });
-  } else {  // any number of terms: all paths first, through the compressed rows
-    float* sP = sD + m.n_lme * 32;  // [NP][32]
+  } else {  // any table: all paths first, through the compressed rows
+    float* sD = reinterpret_cast<float*>(s.buf);  // [n_lme][32]; a lane reads only its own column
+    float* sP = sD + m.n_lme * 32;                // [n_p][32]
+    __syncwarp();
+    for (int lme = 0; lme < m.n_lme; ++lme)
+      async_copy4(sD + lme * 32 + lane, dPhi1 + (static_cast<size_t>(i) * m.n_lme + lme) * C + k);
+    async_wait();
     for (int p = 0; p < m.n_p; ++p) {
       float v = 0.0f;
       for (int t = __ldg(m.cg_rev_off + p), t1 = __ldg(m.cg_rev_off + p + 1); t < t1; ++t)
@@ -219,48 +206,36 @@ __device__ __forceinline__ void rev_group(const DevModel& m, const EdgeIn& in, c
     }
     static_for<NQ>([&](auto ic) {
       constexpr int w = decltype(ic)::value;
-      constexpr int q = rev_ins(LMAX, G, w), p0 = ins_poff(LMAX, q), g0 = rev_goff<LMAX, G>(w);
+      constexpr int q = grp_ins(LMAX, G, w), p0 = ins_poff(LMAX, q), g0 = grp_off<LMAX, G, CANON>(w);
 #pragma unroll
       for (int p = 0; p < ins_paths(LMAX, q); ++p) g[g0 + p] = sP[(p0 + p) * 32 + lane];
     });
+    __syncwarp();
   }
   for (int eb = e0 + part * cs; eb < e1; eb += split * cs) {
     const int ne = min(cs, e1 - eb);
     const long e = static_cast<long>(eb) + lane;
-    if (eb > e0 + part * cs) load(eb);
-    const bool active = lane < ne && rr < m.r_cut;
-    const unsigned ball = __ballot_sync(0xffffffffu, active);
-    const int na = __popc(ball), pos = __popc(ball & ((1u << lane) - 1u));
-    __syncwarp();  // the last chunk's sums have been read
-    if (active) {  // (inactive edges are left out of the staged list)
-      float Y[16];
-      sph_harm16<false>(vx, vy, vz, Y, nullptr);
-#pragma unroll
-      for (int v = 0; v < 4; ++v)
-        *reinterpret_cast<float4*>(&s.Y[pos][4 * v]) = make_float4(Y[4 * v], Y[4 * v + 1], Y[4 * v + 2], Y[4 * v + 3]);
-      int iv = static_cast<int>(rr * m.inv_h);
-      iv = iv < 0 ? 0 : (iv >= m.nint ? m.nint - 1 : iv);
-      const int a = ti < tj ? ti : tj, b = ti < tj ? tj : ti;
-      s.meta[pos] = make_int4(__float_as_int(rr - static_cast<float>(iv) * m.h),
-                              (a * (2 * m.S - a - 1) / 2 + b) * m.nint + iv, nj, 0);
-    }
-    __syncwarp();
+    if (eb > e0 + part * cs) ed.load(m, in, min(eb + lane, e1 - 1));
+    const bool active = lane < ne && ed.r < m.r_cut;
+    int na;
+    const int pos = stage_rows(m, s.st, ed, ti, active, na);
     if (na > 0) {
       float4 c[NQ];
       float h[NR];
-      int4 mt = s.meta[0];
+      int4 mt = s.st.meta[0];
       {
         const float4* cp = m.spl1_fwd + static_cast<size_t>(mt.y) * NI * C + k;
         static_for<NQ>([&](auto ic) {
           constexpr int w = decltype(ic)::value;
-          c[w] = __ldg(cp + rev_ins(LMAX, G, w) * C);
+          c[w] = __ldg(cp + grp_ins(LMAX, G, w) * C);
         });
         const float* hp = H1 + (static_cast<size_t>(mt.z) * NL2 + r0) * C + k;
 #pragma unroll
         for (int b = 0; b < NR; ++b) h[b] = __ldg(hp + b * C);
       }
+      stage_Y(s.st, ed, active, pos);
       for (int a = 0; a < na; ++a) {
-        const int4 mn = s.meta[min(a + 1, na - 1)];
+        const int4 mn = s.st.meta[min(a + 1, na - 1)];
         const float4* cn = m.spl1_fwd + static_cast<size_t>(mn.y) * NI * C + k;
         float hv[NR], hadj[NR];
         const float* hp = H1 + (static_cast<size_t>(mn.z) * NL2 + r0) * C + k;
@@ -269,11 +244,12 @@ __device__ __forceinline__ void rev_group(const DevModel& m, const EdgeIn& in, c
           hv[b] = h[b];
           h[b] = __ldg(hp + b * C);
         }
-        rev_edge<LMAX, G>(g, c, cn, C, __int_as_float(mt.x), s.Y[a], hv, hadj,
+        rev_edge<LMAX, G, CANON>(g, c, cn, C, __int_as_float(mt.x), s.st.Y[a], hv, hadj,
                           s.buf + (a % kSumEdges) * 8 * kSumRow + lane);
         fix64* dst = H1_adj + (static_cast<size_t>(mt.z) * NL2 + r0) * C + k;
 #pragma unroll
-        for (int b = 0; b < NR; ++b) add_fixed(dst + b * C, hadj[b]);
+        for (int b = 0; b + 1 < NR; b += 2) add_fixed2(dst + b * C, dst + (b + 1) * C, make_float2(hadj[b], hadj[b + 1]));
+        if constexpr (NR % 2) add_fixed(dst + (NR - 1) * C, hadj[NR - 1]);
         mt = mn;
         if (a % kSumEdges == kSumEdges - 1 || a == na - 1)
           rev_sums(s, a - a % kSumEdges, a % kSumEdges + 1);
@@ -283,12 +259,12 @@ __device__ __forceinline__ void rev_group(const DevModel& m, const EdgeIn& in, c
       float fx = 0.0f, fy = 0.0f, fz = 0.0f;
       if (active) {
         float Y[16], D[48];
-        sph_harm16<true>(vx, vy, vz, Y, D);
-        const float* S = s.Y[pos];
-        const float d = S[0] / rr;
-        fx = d * vx;
-        fy = d * vy;
-        fz = d * vz;
+        sph_harm16<true>(ed.vx, ed.vy, ed.vz, Y, D);
+        const float* S = s.st.Y[pos];
+        const float d = S[0] / ed.r;
+        fx = d * ed.vx;
+        fy = d * ed.vy;
+        fz = d * ed.vz;
 #pragma unroll
         for (int q = 1; q < 16; ++q) {
           fx = fmaf(S[q], D[q], fx);
@@ -305,7 +281,7 @@ __device__ __forceinline__ void rev_group(const DevModel& m, const EdgeIn& in, c
 }
 
 // item: (node, 32-channel slice, part of the node's edges), parts fastest
-template <int LMAX, int CT>
+template <int LMAX, int CT, bool CANON>
 __device__ __forceinline__ void rev_item(const DevModel& m, const EdgeIn& in, const float* __restrict__ H1,
                                          const float* __restrict__ dPhi1, fix64* __restrict__ H1_adj,
                                          float* __restrict__ f1, RevSmem& s, int item, int split, int cs) {
@@ -315,16 +291,16 @@ __device__ __forceinline__ void rev_item(const DevModel& m, const EdgeIn& in, co
   if (in.first[i] + part * cs >= in.end(i)) return;
   const int k = slice * 32 + (threadIdx.x & 31);
   float* f1s = f1 + slice * m.f1_stride;
-  rev_group<LMAX, 0, CT>(m, in, H1, dPhi1, H1_adj, f1s, s, i, k, part, split, cs);
+  rev_group<LMAX, 0, CT, CANON>(m, in, H1, dPhi1, H1_adj, f1s, s, i, k, part, split, cs);
   if constexpr (LMAX == 2) {
-    rev_group<LMAX, 1, CT>(m, in, H1, dPhi1, H1_adj, f1s, s, i, k, part, split, cs);
-    rev_group<LMAX, 2, CT>(m, in, H1, dPhi1, H1_adj, f1s, s, i, k, part, split, cs);
+    rev_group<LMAX, 1, CT, CANON>(m, in, H1, dPhi1, H1_adj, f1s, s, i, k, part, split, cs);
+    rev_group<LMAX, 2, CT, CANON>(m, in, H1, dPhi1, H1_adj, f1s, s, i, k, part, split, cs);
   }
 }
 
 }  // namespace
 
-template <int LMAX, int CT, bool P>
+template <int LMAX, int CT, bool CANON, bool P>
 __global__ void __launch_bounds__(32, 12) k_layer1_rev(DevModel m, EdgeIn in, const float* __restrict__ H1,
                                                       const float* __restrict__ dPhi1, fix64* __restrict__ H1_adj,
                                                       float* __restrict__ f1, int split, int cs) {
@@ -334,28 +310,11 @@ __global__ void __launch_bounds__(32, 12) k_layer1_rev(DevModel m, EdgeIn in, co
   const int n = in.N * split * ((CT > 0 ? CT : m.C) >> 5);
   AtomCursor cur{P ? m.sched : nullptr, n, 0};
   for (int b = cur.first(); b < n; b = cur.next())
-    rev_item<LMAX, CT>(m, in, H1, dPhi1, H1_adj, f1, s, b, split, cs);
+    rev_item<LMAX, CT, CANON>(m, in, H1, dPhi1, H1_adj, f1, s, b, split, cs);
   cur.done();
 }
 
 namespace {
-
-// channel counts with a compile-time specialisation (addresses fold to immediates)
-template <typename F>
-void dispatch_rev(const DevModel& m, F&& f) {
-  auto by_c = [&](auto lc) {
-    switch (m.C) {
-      case 32: f(lc, std::integral_constant<int, 32>{}); break;
-      case 64: f(lc, std::integral_constant<int, 64>{}); break;
-      case 128: f(lc, std::integral_constant<int, 128>{}); break;
-      default: f(lc, std::integral_constant<int, 0>{}); break;
-    }
-  };
-  if (m.L_max == 2)
-    by_c(std::integral_constant<int, 2>{});
-  else
-    by_c(std::integral_constant<int, 1>{});
-}
 
 // Warps the chip holds at once (12 per SM).  A node's edges are split over `split` warps
 // while all parts still fit at once, each part paying the g prologue again, and over two
@@ -364,7 +323,7 @@ void dispatch_rev(const DevModel& m, F&& f) {
 constexpr long kSlots = 12 * 152;
 
 size_t rev_smem(const DevModel& m) {
-  const size_t rows = m.n_lme + (m.cg_rev_pad ? 0 : m.n_p);
+  const size_t rows = m.cg_val ? 0 : m.n_lme + m.n_p;
   return offsetof(RevSmem, buf) + std::max<size_t>(sizeof(float2) * kSumEdges * 8 * kSumRow, sizeof(float) * 32 * rows);
 }
 
@@ -379,20 +338,21 @@ void launch_layer1_rev(const DevModel& m, const EdgeIn& in, const float* H1, con
   const int cs = split == 1 ? kEdgeChunk : (split <= 2 ? 16 : (split <= 8 ? 8 : 4));
   DevModel mk;
   const int grid = atom_grid(m, kAkLayer1Rev, static_cast<int>(items * split), mk);
-  dispatch_rev(m, [&](auto lc, auto cc) {
+  dispatch_layer1(m, [&](auto lc, auto cc, auto nc) {
     constexpr int LM = decltype(lc)::value, CT = decltype(cc)::value;
+    constexpr bool CANON = decltype(nc)::value;
     if (mk.sched)
-      launch_pdl(k_layer1_rev<LM, CT, true>, grid, 32, rev_smem(m), s, mk, in, H1, dPhi1, H1_adj, f1, split, cs);
+      launch_pdl(k_layer1_rev<LM, CT, CANON, true>, grid, 32, rev_smem(m), s, mk, in, H1, dPhi1, H1_adj, f1, split, cs);
     else
-      launch_pdl(k_layer1_rev<LM, CT, false>, grid, 32, rev_smem(m), s, mk, in, H1, dPhi1, H1_adj, f1, split, cs);
+      launch_pdl(k_layer1_rev<LM, CT, CANON, false>, grid, 32, rev_smem(m), s, mk, in, H1, dPhi1, H1_adj, f1, split, cs);
   });
 }
 
 int layer1_rev_residency(const DevModel& m) {
   int r = 0;
-  dispatch_rev(m, [&](auto lc, auto cc) {
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, k_layer1_rev<decltype(lc)::value, decltype(cc)::value, true>, 32,
-                                                  rev_smem(m));
+  dispatch_layer1(m, [&](auto lc, auto cc, auto nc) {
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+        &r, k_layer1_rev<decltype(lc)::value, decltype(cc)::value, decltype(nc)::value, true>, 32, rev_smem(m));
   });
   return r;
 }

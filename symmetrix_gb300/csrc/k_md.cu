@@ -309,11 +309,12 @@ __global__ void k_edge_geometry_packed(int N, const int* __restrict__ first, con
       dx = pos[3 * j] + sh.x * box.x - px;
       dy = pos[3 * j + 1] + sh.y * box.y - py;
       dz = pos[3 * j + 2] + sh.z * box.z - pz;
-      // the length in float32 (the evaluator reads r as a float; float64 arithmetic runs
-      // on this part's slow float64 pipe)
-      const float fx = static_cast<float>(dx), fy = static_cast<float>(dy), fz = static_cast<float>(dz);
-      const float rf = sqrtf(fmaf(fx, fx, fmaf(fy, fy, fz * fz)));
-      re = rf;
+      // the float32 root and one Newton step on the float64 r^2: the float64 length to
+      // ~1e-15, without the float64 root (its arithmetic runs on this part's slow pipe)
+      const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
+      const float rf = sqrtf(static_cast<float>(r2));
+      const double rd = rf;
+      re = rf > 0.0f ? rd + static_cast<double>(__fdividef(static_cast<float>(fma(-rd, rd, r2)), rf + rf)) : 0.0;
       active = rf < r_cut_f;
     }
     const unsigned ball = __ballot_sync(0xffffffffu, active);

@@ -4,6 +4,8 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <vector>
+
 #include "device.cuh"
 
 namespace smx {
@@ -20,6 +22,10 @@ void launch_layer0_rev(const DevModel& m, const EdgeIn& in, const float* A0, con
                        float* A0_adj, double* forces, cudaStream_t s);
 
 // k_layer1.cu
+// The Clebsch-Gordan values (paths x 2) of a model's compressed path rows in the canonical
+// zero pattern; false when the table has a term outside it.
+bool canonical_cg(int L_max, const std::vector<int>& off, const std::vector<int>& lme, const std::vector<float>& v,
+                  const int* lme_off, const int* num_e, std::vector<float>& val);
 cudaError_t init_layer1_kernels(const DevModel& m);
 void launch_layer1_fwd(const DevModel& m, const EdgeIn& in, const float* H1, float* Phi1, cudaStream_t s);
 // H1_adj: fixed-point accumulator (see to_fixed), seeded by launch_node_tail

@@ -1,6 +1,12 @@
-"""The layer-1 adjoint (k_layer1_rev.cu): edge counts around its sum batches (4 edges) and
-staging chunks (8, 16 and 32 edges), both edge splits, both CG tables, every instruction
-group; and the fixed-point conversion it adds H1_adj terms with (CPU)."""
+"""The layer-1 forward and adjoint (k_layer1.cu, k_layer1_rev.cu): edge counts around the
+adjoint's sum batches (4 edges) and the staging chunks (4 to 32 edges), nodes of one and of
+several warps, every instruction group, and the Clebsch-Gordan tables: the canonical zero
+pattern, its general form and a table outside the pattern; the pattern's generated source
+and the fixed-point conversion of the H1_adj terms (CPU)."""
+import importlib.util
+import os
+import sys
+
 import numpy as np
 import pytest
 
@@ -23,34 +29,55 @@ def clusters(sizes, seed, S):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("C,L_max,padded", [(32, 1, 1), (96, 1, 0), (128, 1, 1), (64, 2, 1), (32, 2, 0)])
-def test_edge_counts_and_splits(engine_lib, tmp_path, C, L_max, padded):
+@pytest.mark.parametrize("C,L_max,table", [(32, 1, "canonical"), (96, 1, "rows"), (128, 1, "canonical"),
+                                           (64, 2, "canonical"), (32, 2, "rows"), (64, 1, "other"), (96, 2, "other")])
+def test_edge_counts_and_splits(engine_lib, tmp_path, C, L_max, table):
     from oracle.pyoracle import Evaluator
     from symmetrix_gb300 import MACE
     from symmetrix_gb300.synth.model import make_model, write_model
     from symmetrix_gb300.synth.structures import neighbor_list
-    path = write_model(make_model(num_channels=C, species=("H", "C", "O"), r_cut=5.0, L_max=L_max, num_knots=60,
-                                  seed=5, avg_num_neighbors=40.0), str(tmp_path / "m.json"))
+    model = make_model(num_channels=C, species=("H", "C", "O"), r_cut=5.0, L_max=L_max, num_knots=60, seed=5,
+                       avg_num_neighbors=40.0)
+    if table == "other":  # one term on a path that reaches no output in the canonical pattern
+        unused = sorted(set(range(max(model["Phi1_lelm1lm2"]) + 1)) - set(model["Phi1_lelm1lm2"]))[0]
+        model["Phi1_lme"].append(0)
+        model["Phi1_lelm1lm2"].append(unused)
+        model["Phi1_clebsch_gordan"].append(0.3)
+    path = write_model(model, str(tmp_path / "m.json"))
     pos, species = clusters([1, 2, 4, 5, 6, 9, 10, 17, 18, 33, 34], 3, 3)
     nl = neighbor_list(pos, 5.0)
     a = edge_args(species, nl)
     m = MACE(path)
-    m.set_option("cg_padded", padded)
+    m.set_option("cg_padded", 0 if table == "rows" else 1)
     m.compute_node_energies_forces(*a)
-    e, f, h = m.node_energies, m.node_forces, m.H1_adj
+    e, f, h, phi = m.node_energies, m.node_forces, m.H1_adj, m.Phi1
     ref = Evaluator(path, "port")
     ref.compute_node_energies_forces(*a)
     # float32 sums of a few hundred terms against float64: 1e-5 of the largest component
-    for got, want in ((e, ref.node_energies), (f, ref.node_forces), (h, ref.get("H1_adj"))):
+    for got, want in ((e, ref.node_energies), (f, ref.node_forces), (h, ref.get("H1_adj")), (phi, ref.get("Phi1"))):
         assert np.abs(got - want).max() <= 1e-5 * max(1.0, np.abs(want).max())
-    # many copies: the edges of a node stay with one warp; the same bits
+    # many copies: the edges of a node stay with one warp
     n, E = len(species), len(nl["r"])
-    copies = 1 + 3000 // (n * C // 32)
-    rep = [np.tile(nl["neigh_indices"], copies) + np.repeat(np.arange(copies) * n, E)]
-    m.compute_node_energies_forces(n * copies, np.tile(species, copies), np.tile(nl["num_neigh"], copies), rep[0],
+    copies = 1 + 2 * 12 * 152 // (n * C // 32)
+    rep = np.tile(nl["neigh_indices"], copies) + np.repeat(np.arange(copies) * n, E)
+    m.compute_node_energies_forces(n * copies, np.tile(species, copies), np.tile(nl["num_neigh"], copies), rep,
                                    np.tile(a[4], copies), np.tile(nl["xyz"], (copies, 1)), np.tile(nl["r"], copies))
-    assert np.array_equal(m.node_forces.reshape(copies, -1), np.tile(f, (copies, 1)))
-    assert np.array_equal(m.H1_adj.reshape(copies, -1), np.tile(h, (copies, 1)))
+    for got, want in ((m.node_forces, ref.node_forces), (m.Phi1, ref.get("Phi1")), (m.H1_adj, ref.get("H1_adj"))):
+        assert np.abs(got.reshape(copies, -1) - want).max() <= 1e-5 * max(1.0, np.abs(want).max())
+
+
+def test_generated_pattern_is_current(tmp_path):
+    csrc = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "symmetrix_gb300", "csrc")
+    spec = importlib.util.spec_from_file_location("gen_cg", os.path.join(csrc, "gen_cg.py"))
+    gen = importlib.util.module_from_spec(spec)
+    keep, sys.dont_write_bytecode = sys.dont_write_bytecode, True
+    try:
+        spec.loader.exec_module(gen)
+    finally:
+        sys.dont_write_bytecode = keep
+    gen.main(out_dir=str(tmp_path))
+    with open(os.path.join(csrc, "cg_canon.h")) as f, open(tmp_path / "cg_canon.h") as g:
+        assert f.read() == g.read()
 
 
 def test_to_fixed_is_the_rounding_of_v_2_to_34():
