@@ -63,6 +63,9 @@ struct smx_engine {
   // (K contiguous, split_wterms(tc_terms) bf16 split terms concatenated along K: see tc_operand)
   const __nv_bfloat16 *W_H1 = nullptr, *W_M0adj = nullptr, *W_A1[4] = {}, *W_Phi1adj[4] = {};
   bool tc_H1 = false, tc_A1[4] = {}, tc_Phi1adj[4] = {};
+  // float32 tensor-core GEMMs: three bf16 terms per weight (see f32_operand)
+  const __nv_bfloat16 *W32_H1[3] = {}, *W32_M0adj[3] = {}, *W32_A1[4] = {}, *W32_Phi1adj[4] = {};
+  bool tc32 = false;
   // 1: bf16 operands; 2: weights split hi + lo (x_hi W_hi + x_hi W_lo); 3: both
   // split (x_hi W_hi + x_lo W_hi + x_hi W_lo: close to float32 operand precision)
   int tc_terms = 3;
@@ -112,6 +115,27 @@ struct smx_engine {
         std::memcpy(&hf, &hu, 4);
         const uint16_t lo = smx::bf16_bits(w - hf);
         for (int t = 0; t < WT; ++t) b[(static_cast<size_t>(n) * WT + t) * K + k] = t == 0 ? hi : lo;
+      }
+    return reinterpret_cast<const __nv_bfloat16*>(upload(b));
+  }
+
+  // B operand of a float32 tensor-core GEMM from a row-major float [nrows][K] matrix: row n
+  // holds (W0 | W1 | W2), each the bf16 rounding of what the ones before it leave, padded
+  // with zeros to whole k-blocks
+  const __nv_bfloat16* f32_operand(const float* W, int nrows, int K) {
+    const size_t Kp = smx::umma_f32_kp(K);
+    std::vector<uint16_t> b(nrows * 3 * Kp, 0);
+    for (int n = 0; n < nrows; ++n)
+      for (int k = 0; k < K; ++k) {
+        float w = W[static_cast<size_t>(n) * K + k];
+        for (int t = 0; t < 3; ++t) {
+          const uint16_t h = smx::bf16_bits(w);
+          b[(static_cast<size_t>(n) * 3 + t) * Kp + k] = h;
+          const uint32_t hu = static_cast<uint32_t>(h) << 16;
+          float hf;
+          std::memcpy(&hf, &hu, 4);
+          w -= hf;
+        }
       }
     return reinterpret_cast<const __nv_bfloat16*>(upload(b));
   }
@@ -248,8 +272,24 @@ struct smx_engine {
         m.pgrid[k] = sched_force == 1 ? pfull[k] : 0;
       }
     }
+    check(smx::init_umma_kernels(), "cudaFuncSetAttribute");
+    // Float32 GEMMs on the tensor cores from 64 channels (two k-blocks or more in A1); at 32
+    // the SIMT kernel is as fast or faster (5000 x 96 x 96: 12.2 us each).  A rule on the
+    // model alone, so that a molecule gives the same bits in a batch and by itself.
+    tc32 = pm.C >= 64 && smx::umma_f32_supported(pm.C, pm.C);
+    if (tc32) {
+      const int C = pm.C;
+      for (int L = 0; L <= pm.L_max; ++L) {
+        W32_H1[L] = f32_operand(pm.H1W_T.data() + static_cast<size_t>(L) * C * C, C, C);
+        W32_M0adj[L] = f32_operand(pm.H1W.data() + static_cast<size_t>(L) * C * C, C, C);
+      }
+      for (int l = 0; l < 4; ++l) {
+        if (pm.num_e[l] == 0) continue;
+        W32_A1[l] = f32_operand(pm.A1W_T[l].data(), C, pm.num_e[l] * C);
+        W32_Phi1adj[l] = f32_operand(pm.A1W[l].data(), pm.num_e[l] * C, C);
+      }
+    }
     if (precision == SMX_PRECISION_BF16) {
-      check(smx::init_umma_kernels(), "cudaFuncSetAttribute");
       const int C = pm.C;
       // (three split products, the most the tc_terms option allows)
       tc_H1 = smx::umma_supported(C, C, 3) && pm.L_max == 1;
@@ -441,6 +481,15 @@ struct smx_engine {
     tc_cfg[gid] = bestc;
     tc_tuned[gid] = true;
     tc_tuned_us[gid] = best * 1000.0f / 3.0f;
+  }
+
+  // float32 GEMMs: on the tensor cores (B: the segments' split weights) or the SIMT kernel
+  void gemm32(const smx::GemmBatch& b, const __nv_bfloat16* const* B, cudaStream_t s) {
+    if (b.n == 0) return;
+    if (tc32)
+      smx::launch_umma_f32(b, B, status_dev, s);
+    else
+      smx::launch_gemm(b, s);
   }
 
   // The M0_adj GEMM (L_max 1) as two segments, one per L block: X rows grouped by L
@@ -698,7 +747,7 @@ struct smx_engine {
       for (int L = 0; L <= dm.L_max; ++L)
         b.s[b.n++] = seg_rows(M0, H1, dm.H1W + static_cast<size_t>(L) * C * C, N, 2 * L + 1, C, C,
                               static_cast<long>(dm.nLM) * C, L * L * C, C, static_cast<long>(dm.nLM) * C, L * L * C, C);
-      smx::launch_gemm(b, s);
+      gemm32(b, W32_H1, s);
     }
     mark(2, s);
     smx::launch_layer1_fwd(dm, in1, H1, Phi1_out, s);
@@ -717,12 +766,15 @@ struct smx_engine {
         }
       run_tc(1, g, ng, true, s);
       smx::GemmBatch b{};
+      const __nv_bfloat16* B[4] = {};
       for (int l = 0; l < 4; ++l)
-        if (dm.num_e[l] > 0 && !tc_A1[l])
+        if (dm.num_e[l] > 0 && !tc_A1[l]) {
+          B[b.n] = W32_A1[l];
           b.s[b.n++] = seg_rows(Phi1, A1, dm.A1W[l], N1, 2 * l + 1, dm.num_e[l] * C, C,
                                 static_cast<long>(dm.n_lme) * C, dm.lme_off[l] * C, dm.num_e[l] * C,
                                 16L * C, l * l * C, C);
-      smx::launch_gemm(b, s);
+        }
+      gemm32(b, B, s);
     }
     mark(4, s);
     smx::launch_node_tail(dm, in.node_type, N1, A1, H1, M1, H2, A1adj_out, H1_adj_fx, M1_adj, H2_adj,
@@ -743,11 +795,14 @@ struct smx_engine {
         }
       run_tc(2, g, ng, true, s);
       smx::GemmBatch b{};
+      const __nv_bfloat16* B[4] = {};
       for (int l = 0; l < 4; ++l)
-        if (dm.num_e[l] > 0 && !tc_Phi1adj[l])
+        if (dm.num_e[l] > 0 && !tc_Phi1adj[l]) {
+          B[b.n] = W32_Phi1adj[l];
           b.s[b.n++] = seg_rows(A1_adj, Phi1_adj, dm.A1W_T[l], N1, 2 * l + 1, C, dm.num_e[l] * C, 16L * C, l * l * C,
                                 C, static_cast<long>(dm.n_lme) * C, dm.lme_off[l] * C, dm.num_e[l] * C);
-      smx::launch_gemm(b, s);
+        }
+      gemm32(b, B, s);
     }
     mark(6, s);
     smx::launch_layer1_rev(dm, in1, H1, Phi1_adj, H1_adj_fx, f1, s);
@@ -764,7 +819,7 @@ struct smx_engine {
       for (int L = 0; L <= dm.L_max; ++L)
         b.s[b.n++] = seg_rows(H1_adj, M0_adj, dm.H1W_T + static_cast<size_t>(L) * C * C, N, 2 * L + 1, C, C,
                               static_cast<long>(dm.nLM) * C, L * L * C, C, static_cast<long>(dm.nLM) * C, L * L * C, C);
-      smx::launch_gemm(b, s);
+      gemm32(b, W32_M0adj, s);
     }
     mark(8, s);
     smx::launch_layer0_rev(dm, in, A0, M0_adj, f1, A0_adj, out_f, s);

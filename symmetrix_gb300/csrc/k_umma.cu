@@ -201,6 +201,229 @@ __global__ void __launch_bounds__(128, 1) k_umma_gemm(const __grid_constant__ Um
   if (warp == 0) sm100::tmem_dealloc(tmem, ncols);
 }
 
+// ---------------------------------------------------------------------------
+// Float32 GEMMs:  Y[rows, N] = X[rows, K] . B[N, K]^T with float32 X, split in the kernel.
+//
+// x = x0 + x1 + x2 and w = w0 + w1 + w2 in bf16 (24 bits: what float32 holds), six products:
+// x0 w0 into one accumulator, x0 w1, x1 w0, x1 w1, x0 w2, x2 w0 into another that the
+// epilogue adds, so that the small products are not rounded at the size of the large one.
+// The tensor core's running sum is cut towards zero at every step, measured as a shrinking of
+// the result by 1.2e-8 per 16-wide step for terms of random sign (2e-8 for terms of one
+// sign), where a chain of FMAs errs either way and grows with the root of K.  So above
+// K = 128 the k-blocks alternate between two accumulators of x0 w0, and the epilogue gives
+// the mean loss back.  Error against float64 (2-norm; this kernel : the SIMT one, random
+// terms): K = 128 0.7e-7 : 2.0e-7, K = 384 1.0e-7 : 3.5e-7, K = 640 1.6e-7 : 4.5e-7; terms of
+// one sign: 0.8e-7 : 1.6e-7, 1.2e-7 : 2.9e-7, 2.2e-7 : 3.5e-7.
+// Eight warps read the float32 rows where the producers left them (the row map of the SIMT
+// GEMM) and split them into the swizzled operand layout, a k-block ahead in registers; one
+// thread of a ninth brings the weights' terms by TMA and issues the MMAs.
+// ---------------------------------------------------------------------------
+struct F32SegDev {
+  CUtensorMap tb;
+  GemmSeg g;
+  int NT, tiles_m, tiles_n, mains, stages;  // mains: accumulators of x0 w0
+};
+struct F32GroupDev {
+  F32SegDev s[4];
+};
+constexpr int kF32Split = 256;                // threads that split X and store Y
+constexpr int kF32Threads = kF32Split + 32;   // and a warp whose first lane issues TMA and MMAs
+constexpr float kStepLoss = 1.2e-8f;  // mean relative loss of an accumulator per MMA step
+constexpr uint32_t kATerm = kTileM * kBoxK * 2;  // bytes of one X term of a k-block
+
+__device__ __forceinline__ float bf16_lo(uint32_t p) { return __uint_as_float(p << 16); }
+__device__ __forceinline__ float bf16_hi(uint32_t p) { return __uint_as_float(p & 0xffff0000u); }
+__device__ __forceinline__ uint32_t bf16_pair(float a, float b) {
+  const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
+  return *reinterpret_cast<const uint32_t*>(&v);
+}
+// the remainder of v after its leading term; an infinite v has none (v - v is NaN)
+__device__ __forceinline__ float rest(float v, float lead) {
+  const float d = v - lead;
+  return d == d ? d : 0.0f;
+}
+
+// Up to K = 128 two CTAs per SM with one stage each (96 KB, 256 TMEM columns) overlap one's
+// splitting and stores with the other's MMAs; above, one CTA with two stages and 512 columns.
+__global__ void __launch_bounds__(kF32Threads, 2) k_umma_f32(const __grid_constant__ F32GroupDev grp,
+                                                             unsigned* status) {
+  pdl_begin();
+  const F32SegDev& seg = grp.s[blockIdx.z];
+  const GemmSeg& g = seg.g;
+  const int tile_n = static_cast<int>(blockIdx.x % static_cast<unsigned>(seg.tiles_n));
+  const int tile_m = static_cast<int>(blockIdx.x / static_cast<unsigned>(seg.tiles_n));
+  if (tile_m >= seg.tiles_m) return;
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ uint64_t full[kStages], split[kStages], empty[kStages], bar_mma;
+  __shared__ uint32_t tmem_base;
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  const int NT = seg.NT, S = seg.stages;
+  const int KB = (g.K + kBoxK - 1) / kBoxK, Kp = KB * kBoxK;
+  const uint32_t b_bytes = static_cast<uint32_t>(NT) * kBoxK * 2, stage_bytes = 3 * kATerm + 3 * b_bytes;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int m0 = tile_m * kTileM, n0 = tile_n * NT;
+  const uint32_t used = static_cast<uint32_t>((seg.mains + 1) * NT);
+  const uint32_t ncols = used <= 64 ? 64u : (used <= 128 ? 128u : (used <= 256 ? 256u : 512u));
+  if (tid == 0) {
+    for (int s = 0; s < S; ++s) {
+      sm100::mbar_init(&full[s], 1);
+      sm100::mbar_init(&split[s], kF32Split);
+      sm100::mbar_init(&empty[s], 1);
+    }
+    sm100::mbar_init(&bar_mma, 1);
+    sm100::fence_mbar_init();
+  }
+  if (warp == 0) {
+    sm100::tmem_alloc(&tmem_base, ncols);
+    sm100::tmem_relinquish();
+  }
+  __shared__ long x_row[kTileM];  // offsets of the tile's rows, -1 past the end
+  if (tid < kTileM) {
+    const int r = m0 + tid, node = r / g.rpn, sub = r - node * g.rpn;
+    x_row[tid] = r < g.rows ? node * g.x_ns + g.x_off + static_cast<long>(sub) * g.x_rs : -1;
+  }
+  sm100::tc_fence_before();
+  __syncthreads();
+  sm100::tc_fence_after();
+  const uint32_t tmem = tmem_base;
+
+  // a k-block row is 16 float4: a warp reads two rows at a time, 16 rows in all; this thread
+  // has float4 c of rows warp * 16 + lane / 16 + 2 j
+  const int c = lane & 15, row0 = warp * 16 + (lane >> 4);
+  float4 v[8];
+  auto load = [&](int kb) {
+    const int k = kb * kBoxK + 4 * c;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const long o = x_row[row0 + 2 * j];
+      v[j] = o >= 0 && k < g.K ? __ldg(reinterpret_cast<const float4*>(g.X + o + k)) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+  };
+  bool ok = true, issued = false;
+  int loads = 0;
+  if (tid < kF32Split) {
+    load(0);
+    for (int kb = 0; kb < KB; ++kb) {
+      const int s = kb % S;
+      if (kb >= S && !sm100::mbar_wait(&empty[s], ((kb / S) - 1) & 1)) {  // the stage's last MMAs are done
+        ok = false;
+        break;
+      }
+      uint8_t* st = smem + static_cast<size_t>(s) * stage_bytes;
+      // 16-byte group q (8 elements) of row r sits at slot q ^ (r & 7) of its 128-byte row
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int row = row0 + 2 * j;
+        uint8_t* a = st + row * 128 + ((c >> 1) ^ (row & 7)) * 16 + (c & 1) * 8;
+        float4 x = v[j];
+#pragma unroll
+        for (int t = 0; t < 3; ++t) {
+          const uint2 w = make_uint2(bf16_pair(x.x, x.y), bf16_pair(x.z, x.w));
+          *reinterpret_cast<uint2*>(a + t * kATerm) = w;
+          if (t < 2)
+            x = make_float4(rest(x.x, bf16_lo(w.x)), rest(x.y, bf16_hi(w.x)), rest(x.z, bf16_lo(w.y)),
+                            rest(x.w, bf16_hi(w.y)));
+        }
+      }
+      sm100::fence_async_shared();
+      sm100::mbar_arrive(&split[s]);
+      if (kb + 1 < KB) load(kb + 1);
+    }
+  } else if (tid == kF32Split) {
+    const uint32_t idesc = sm100::idesc_bf16_f32(kTileM, NT);
+    auto weights = [&](int kb) {  // into the stage of k-block kb, which must be free
+      uint8_t* st = smem + static_cast<size_t>(kb % S) * stage_bytes + 3 * kATerm;
+      sm100::mbar_arrive_expect_tx(&full[kb % S], 3 * b_bytes);
+      for (int u = 0; u < 3; ++u)
+        sm100::tma_load_2d(st + u * b_bytes, &seg.tb, u * Kp + kb * kBoxK, n0, &full[kb % S]);
+      ++loads;
+    };
+    for (int kb = 0; kb < KB && kb < S; ++kb) weights(kb);
+    for (int kb = 0; kb < KB; ++kb) {
+      const int s = kb % S;
+      // (with one stage: this k-block's weights, once the last one's MMAs are done)
+      if (S == 1 && kb > 0) {
+        if (!(ok = sm100::mbar_wait(&empty[0], (kb - 1) & 1))) break;
+        weights(kb);
+      }
+      ok = sm100::mbar_wait(&full[s], (kb / S) & 1) && sm100::mbar_wait(&split[s], (kb / S) & 1);
+      if (!ok) break;
+      sm100::tc_fence_after();
+      const uint32_t x0 = sm100::smem_u32(smem + static_cast<size_t>(s) * stage_bytes), w0 = x0 + 3 * kATerm;
+#pragma unroll
+      for (int k = 0; k < kBoxK / 16; ++k) {
+        auto mma = [&](uint32_t d, int xt, int wt, uint32_t acc) {
+          sm100::umma_bf16(d, sm100::sdesc_sw128(x0 + xt * kATerm + k * 32),
+                           sm100::sdesc_sw128(w0 + wt * b_bytes + k * 32), idesc, acc);
+        };
+        const uint32_t corr = tmem + seg.mains * NT;
+        mma(tmem + (kb % seg.mains) * NT, 0, 0, kb >= seg.mains || k != 0 ? 1u : 0u);
+        mma(corr, 0, 2, (kb | k) != 0 ? 1u : 0u);
+        mma(corr, 2, 0, 1u);
+        mma(corr, 1, 1, 1u);
+        mma(corr, 0, 1, 1u);
+        mma(corr, 1, 0, 1u);
+      }
+      sm100::umma_commit(&empty[s]);
+      issued = true;
+      // while these run: the weights that follow those of the k-block before
+      if (S > 1 && kb > 0 && kb - 1 + S < KB) {
+        if (!(ok = sm100::mbar_wait(&empty[(kb - 1) % S], ((kb - 1) / S) & 1))) break;
+        weights(kb - 1 + S);
+      }
+    }
+    if (issued) sm100::umma_commit(&bar_mma);
+  }
+  const int all_ok = __syncthreads_and(ok ? 1 : 0);
+  const int any_mma = __syncthreads_or(issued ? 1 : 0);
+  bool done = false;
+  if (any_mma) done = sm100::mbar_wait(&bar_mma, 0);
+  const int all_done = __syncthreads_and((done && all_ok) ? 1 : 0);
+  sm100::tc_fence_after();
+  if (all_done && tid < kF32Split) {
+    // warp w reads the accumulator lanes 32 (w mod 4) and every other 32-column chunk; rows
+    // leave through a swizzled 4 KB tile per warp, as in k_umma_gemm
+    const int quarter = warp & 3, r = m0 + quarter * 32 + lane;
+    const bool write = r < g.rows;
+    const long base = write ? static_cast<long>(r / g.rpn) * g.y_ns + g.y_off + static_cast<long>(r % g.rpn) * g.y_rs + n0
+                            : 0;
+    float* stg = reinterpret_cast<float*>(smem) + warp * 32 * 32;
+    const int sub = lane >> 3, c4 = lane & 7;
+    const uint32_t t0 = tmem + (static_cast<uint32_t>(quarter * 32) << 16);
+    const float loss = kStepLoss * static_cast<float>((KB + seg.mains - 1) / seg.mains * (kBoxK / 16));
+    for (int c0 = (warp >> 2) * 32; c0 < NT; c0 += 64) {
+      // mains + (corrections + loss mains)
+      float a[32], b[32];
+      sm100::tmem_ld32(t0 + static_cast<uint32_t>(seg.mains * NT + c0), a);
+      for (int w = seg.mains - 1; w >= 0; --w) {
+        sm100::tmem_ld32(t0 + static_cast<uint32_t>(w * NT + c0), b);
+#pragma unroll
+        for (int q = 0; q < 32; ++q) a[q] = b[q] + fmaf(loss, b[q], a[q]);
+      }
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        reinterpret_cast<float4*>(stg + lane * 32)[q ^ (lane & 7)] =
+            make_float4(a[4 * q], a[4 * q + 1], a[4 * q + 2], a[4 * q + 3]);
+      __syncwarp();
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int t = 4 * j + sub;
+        const long yb = __shfl_sync(0xffffffffu, base, t);
+        const int w = __shfl_sync(0xffffffffu, write ? 1 : 0, t);
+        const float4 val = reinterpret_cast<const float4*>(stg + t * 32)[c4 ^ (t & 7)];
+        if (w) reinterpret_cast<float4*>(g.Y + yb + c0)[c4] = val;
+      }
+      __syncwarp();
+    }
+  } else if (!all_done && tid == kF32Split) {
+    record_timeout(status);
+    for (int kb = loads - S > 0 ? loads - S : 0; kb < loads; ++kb) sm100::mbar_wait(&full[kb % S], (kb / S) & 1);
+  }
+  sm100::tc_fence_before();
+  __syncthreads();
+  if (warp == 0) sm100::tmem_dealloc(tmem, ncols);
+}
+
 using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                    const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                    CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -252,7 +475,53 @@ bool umma_supported(int K, int NT, int terms) {
          umma_smem_bytes(K, NT, 1, terms) <= kMaxDynSmem;
 }
 
+namespace {
+
+// x0 w0 accumulators, and ring stages (see k_umma_f32)
+int f32_mains(int K) { return K > 2 * kBoxK ? 2 : 1; }
+// N-tile: the widest of 128, 96, 64, 32 that divides the columns
+int f32_tile_n(int ncols) {
+  for (int nt : {128, 96, 64})
+    if (ncols % nt == 0) return nt;
+  return 32;
+}
+size_t f32_smem_bytes(int NT, int stages) {
+  return static_cast<size_t>(stages) * (3 * kATerm + 3 * static_cast<size_t>(NT) * kBoxK * 2) + 1024;
+}
+}  // namespace
+
+bool umma_f32_supported(int K, int ncols) { return K > 0 && K % 32 == 0 && ncols > 0 && ncols % 32 == 0; }
+
+int umma_f32_kp(int K) { return (K + kBoxK - 1) / kBoxK * kBoxK; }
+
+void launch_umma_f32(const GemmBatch& b, const __nv_bfloat16* const* B, unsigned* status, cudaStream_t s) {
+  F32GroupDev grp;
+  std::memset(&grp, 0, sizeof(grp));
+  long gx = 0;
+  size_t smem = 0;
+  int used = 0;
+  for (int q = 0; q < b.n; ++q) {
+    const GemmSeg& g = b.s[q];
+    if (!umma_f32_supported(g.K, g.ncols)) throw std::invalid_argument("unsupported tensor-core GEMM shape");
+    if (g.rows <= 0) continue;
+    F32SegDev& d = grp.s[used++];
+    d.g = g;
+    d.NT = f32_tile_n(g.ncols);
+    d.mains = d.stages = f32_mains(g.K);
+    d.tb = make_map(B[q], g.ncols, 3 * umma_f32_kp(g.K), d.NT);
+    d.tiles_m = (g.rows + kTileM - 1) / kTileM;
+    d.tiles_n = g.ncols / d.NT;
+    gx = std::max(gx, static_cast<long>(d.tiles_m) * d.tiles_n);
+    smem = std::max(smem, f32_smem_bytes(d.NT, d.stages));
+  }
+  if (used == 0) return;
+  launch_pdl(k_umma_f32, dim3(static_cast<unsigned>(gx), 1, used), kF32Threads, smem, s, grp, status);
+}
+
 cudaError_t init_umma_kernels() {
+  const cudaError_t e = cudaFuncSetAttribute(k_umma_f32, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             static_cast<int>(f32_smem_bytes(128, 2)));
+  if (e != cudaSuccess) return e;
   return cudaFuncSetAttribute(k_umma_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               static_cast<int>(kMaxDynSmem));
 }

@@ -112,6 +112,12 @@ struct UmmaGemm {
 // wait gives up after 2 ms: the launch records a timeout in *status and writes nothing)
 void launch_umma_gemms(const UmmaGemm* g, int n, unsigned* status, cudaStream_t s, bool test_timeout = false);
 
+// The batch's GEMMs in float32 on the tensor cores; B[q]: segment q's weights as three bf16
+// terms, [ncols][3][umma_f32_kp(K)], zero behind K (GemmSeg::B is not read).
+bool umma_f32_supported(int K, int ncols);
+int umma_f32_kp(int K);
+void launch_umma_f32(const GemmBatch& b, const __nv_bfloat16* const* B, unsigned* status, cudaStream_t s);
+
 // k_md.cu
 void launch_wrap(int N, double3 box, int3 periodic, double* pos, cudaStream_t s);
 void launch_cell_list(const double* pos, int N, double3 box, int3 nc, int* cell, int* cell_count, int* cell_start,

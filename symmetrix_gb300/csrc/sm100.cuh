@@ -64,6 +64,11 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint64
   return true;
 }
 
+// make this thread's shared-memory writes visible to the async proxy (tcgen05 operands)
+__device__ __forceinline__ void fence_async_shared() {
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+}
+
 // ---- TMA --------------------------------------------------------------------
 // 2-D tile load of the box at (x, y) (x innermost, in elements) into shared memory,
 // completing transaction bytes on bar.
