@@ -361,11 +361,16 @@ __device__ __forceinline__ float spline_der(const float4 c, float x) {
 // Condon-Shortley phase, times 2 sqrt(pi) (libsymmetrix/source/mace.cpp:118-148).
 // Each Y_lm = s P_lm(u) with P_lm homogeneous of degree l and u the unit vector;
 // the gradient with respect to v is s (grad P_lm(u) - l P_lm(u) u) / |v|.
+// Every product and sum is an explicit intrinsic: which of them the compiler fuses would
+// otherwise depend on the kernel around the call, and the kernels' schedules (one block per
+// node, persistent grids) are to give the same bits.
 template <bool GRAD>
 __device__ __forceinline__ void sph_harm16(float vx, float vy, float vz, float* Y, float* G /*[3][16]*/) {
-  const float r2 = vx * vx + vy * vy + vz * vz;
+  auto mul = [](float a, float b) { return __fmul_rn(a, b); };
+  auto fma = [](float a, float b, float c) { return __fmaf_rn(a, b, c); };
+  const float r2 = fma(vz, vz, fma(vy, vy, mul(vx, vx)));
   const float inv_r = rsqrtf(r2);
-  const float X = vz * inv_r, Yv = vx * inv_r, Z = vy * inv_r;  // shuffled unit vector
+  const float X = mul(vz, inv_r), Yv = mul(vx, inv_r), Z = mul(vy, inv_r);  // shuffled unit vector
   // 2 sqrt(pi) times the orthonormal normalisation constants
   const float s0 = 1.0f;
   const float s1 = 1.7320508075688772f;                      // sqrt(3)
@@ -377,23 +382,25 @@ __device__ __forceinline__ void sph_harm16(float vx, float vy, float vz, float* 
   const float s3c = 1.620185174601965f;                      // sqrt(21/8)
   const float s3d = 1.3228756555322954f;                     // sqrt(7)/2
   const float s3e = 5.123475382979799f;                      // sqrt(105)/2
-  const float XX = X * X, YY = Yv * Yv, ZZ = Z * Z;
+  const float XX = mul(X, X), YY = mul(Yv, Yv), ZZ = mul(Z, Z), XY = mul(X, Yv), YZ = mul(Yv, Z), XZ = mul(X, Z);
+  const float dXY = __fsub_rn(XX, YY), sXY = __fadd_rn(XX, YY);
+  const float c4 = fma(4.0f, ZZ, -sXY);  // 4 Z^2 - X^2 - Y^2
   Y[0] = s0;
-  Y[1] = s1 * Yv;
-  Y[2] = s1 * Z;
-  Y[3] = s1 * X;
-  Y[4] = s2a * X * Yv;
-  Y[5] = s2a * Yv * Z;
-  Y[6] = s2b * (2.0f * ZZ - XX - YY);
-  Y[7] = s2a * X * Z;
-  Y[8] = s2c * (XX - YY);
-  Y[9] = s3a * Yv * (3.0f * XX - YY);
-  Y[10] = s3b * X * Yv * Z;
-  Y[11] = s3c * Yv * (4.0f * ZZ - XX - YY);
-  Y[12] = s3d * Z * (2.0f * ZZ - 3.0f * XX - 3.0f * YY);
-  Y[13] = s3c * X * (4.0f * ZZ - XX - YY);
-  Y[14] = s3e * Z * (XX - YY);
-  Y[15] = s3a * X * (XX - 3.0f * YY);
+  Y[1] = mul(s1, Yv);
+  Y[2] = mul(s1, Z);
+  Y[3] = mul(s1, X);
+  Y[4] = mul(s2a, XY);
+  Y[5] = mul(s2a, YZ);
+  Y[6] = mul(s2b, fma(2.0f, ZZ, -sXY));
+  Y[7] = mul(s2a, XZ);
+  Y[8] = mul(s2c, dXY);
+  Y[9] = mul(mul(s3a, Yv), fma(3.0f, XX, -YY));
+  Y[10] = mul(mul(s3b, XY), Z);
+  Y[11] = mul(mul(s3c, Yv), c4);
+  Y[12] = mul(mul(s3d, Z), fma(2.0f, ZZ, mul(-3.0f, sXY)));
+  Y[13] = mul(mul(s3c, X), c4);
+  Y[14] = mul(mul(s3e, Z), dXY);
+  Y[15] = mul(mul(s3a, X), fma(-3.0f, YY, XX));
   if constexpr (GRAD) {
     // dP/d(X, Y, Z) in shuffled axes
     float D[3][16];
@@ -404,26 +411,27 @@ __device__ __forceinline__ void sph_harm16(float vx, float vy, float vz, float* 
     D[1][1] = s1;
     D[2][2] = s1;
     D[0][3] = s1;
-    D[0][4] = s2a * Yv; D[1][4] = s2a * X;
-    D[1][5] = s2a * Z;  D[2][5] = s2a * Yv;
-    D[0][6] = -2.0f * s2b * X; D[1][6] = -2.0f * s2b * Yv; D[2][6] = 4.0f * s2b * Z;
-    D[0][7] = s2a * Z; D[2][7] = s2a * X;
-    D[0][8] = 2.0f * s2c * X; D[1][8] = -2.0f * s2c * Yv;
-    D[0][9] = 6.0f * s3a * X * Yv; D[1][9] = 3.0f * s3a * (XX - YY);
-    D[0][10] = s3b * Yv * Z; D[1][10] = s3b * X * Z; D[2][10] = s3b * X * Yv;
-    D[0][11] = -2.0f * s3c * X * Yv; D[1][11] = s3c * (4.0f * ZZ - XX - 3.0f * YY); D[2][11] = 8.0f * s3c * Yv * Z;
-    D[0][12] = -6.0f * s3d * X * Z; D[1][12] = -6.0f * s3d * Yv * Z; D[2][12] = s3d * (6.0f * ZZ - 3.0f * XX - 3.0f * YY);
-    D[0][13] = s3c * (4.0f * ZZ - 3.0f * XX - YY); D[1][13] = -2.0f * s3c * X * Yv; D[2][13] = 8.0f * s3c * X * Z;
-    D[0][14] = 2.0f * s3e * X * Z; D[1][14] = -2.0f * s3e * Yv * Z; D[2][14] = s3e * (XX - YY);
-    D[0][15] = 3.0f * s3a * (XX - YY); D[1][15] = -6.0f * s3a * X * Yv;
+    D[0][4] = mul(s2a, Yv); D[1][4] = mul(s2a, X);
+    D[1][5] = mul(s2a, Z);  D[2][5] = mul(s2a, Yv);
+    D[0][6] = mul(-2.0f * s2b, X); D[1][6] = mul(-2.0f * s2b, Yv); D[2][6] = mul(4.0f * s2b, Z);
+    D[0][7] = mul(s2a, Z); D[2][7] = mul(s2a, X);
+    D[0][8] = mul(2.0f * s2c, X); D[1][8] = mul(-2.0f * s2c, Yv);
+    D[0][9] = mul(6.0f * s3a, XY); D[1][9] = mul(3.0f * s3a, dXY);
+    D[0][10] = mul(s3b, YZ); D[1][10] = mul(s3b, XZ); D[2][10] = mul(s3b, XY);
+    D[0][11] = mul(-2.0f * s3c, XY); D[1][11] = mul(s3c, fma(-2.0f, YY, c4)); D[2][11] = mul(8.0f * s3c, YZ);
+    D[0][12] = mul(-6.0f * s3d, XZ); D[1][12] = mul(-6.0f * s3d, YZ);
+    D[2][12] = mul(s3d, fma(6.0f, ZZ, mul(-3.0f, sXY)));
+    D[0][13] = mul(s3c, fma(-2.0f, XX, c4)); D[1][13] = mul(-2.0f * s3c, XY); D[2][13] = mul(8.0f * s3c, XZ);
+    D[0][14] = mul(2.0f * s3e, XZ); D[1][14] = mul(-2.0f * s3e, YZ); D[2][14] = mul(s3e, dXY);
+    D[0][15] = mul(3.0f * s3a, dXY); D[1][15] = mul(-6.0f * s3a, XY);
     const float u[3] = {X, Yv, Z};
 #pragma unroll
     for (int q = 0; q < 16; ++q) {
       const float l = q == 0 ? 0.0f : (q < 4 ? 1.0f : (q < 9 ? 2.0f : 3.0f));
-      const float lp = l * Y[q];
-      const float gX = (D[0][q] - lp * u[0]) * inv_r;
-      const float gY = (D[1][q] - lp * u[1]) * inv_r;
-      const float gZ = (D[2][q] - lp * u[2]) * inv_r;
+      const float lp = mul(-l, Y[q]);
+      const float gX = mul(fma(lp, u[0], D[0][q]), inv_r);
+      const float gY = mul(fma(lp, u[1], D[1][q]), inv_r);
+      const float gZ = mul(fma(lp, u[2], D[2][q]), inv_r);
       // back to (x, y, z): d/dx = d/dY', d/dy = d/dZ', d/dz = d/dX'
       G[0 * 16 + q] = gY;
       G[1 * 16 + q] = gZ;
@@ -481,7 +489,7 @@ __device__ __forceinline__ void dens_eval(const DevModel& m, int layer, int ti, 
   const int pr = a * (2 * m.S - a - 1) / 2 + b;
   int iv = static_cast<int>(r * m.dens_inv_h[layer]);
   iv = iv < 0 ? 0 : (iv >= m.dens_nint[layer] ? m.dens_nint[layer] - 1 : iv);
-  const float x = r - static_cast<float>(iv) * m.dens_h[layer];
+  const float x = __fmaf_rn(-static_cast<float>(iv), m.dens_h[layer], r);
   const float4 c = __ldg(m.dens_spl[layer] + static_cast<size_t>(pr) * m.dens_nint[layer] + iv);
   v = spline_val(c, x);
   d = spline_der(c, x);

@@ -6,7 +6,9 @@ every species and channel uses the same monomial set, only the coefficients diff
 (extract_mace_data.py:239-304 folds U tensors and weights into exactly these
 coefficients).  This script writes those sets, in the order symmetrix_gb300.synth
 emits them, as compile-time code: the A-basis values and the gradient live in
-registers and each monomial costs one coalesced coefficient load plus a few FMAs.
+registers, and the nested form sum_a x_a (c_a + sum_b x_b (c_ab + sum_c c_abc x_c)) costs
+one coalesced coefficient load and one FMA per cubic monomial, two with its gradient,
+without products of pairs kept in registers.
 
     python symmetrix_gb300/csrc/gen_poly.py      # rewrites poly_canon.h next to it
 """
@@ -36,59 +38,93 @@ def pack(m):
     return idx[0] | (idx[1] << 8) | (idx[2] << 16)
 
 
-def term(m):
-    return "*".join(f"x[{a}]" for a in m)
+def tree(monos):
+    """{a: (t of x_a, {b: (t of x_a x_b, [(c, t of x_a x_b x_c)])})}, t = None where there is no such
+    monomial: the polynomial as sum_a x_a (c_a + sum_b x_b (c_ab + sum_c c_abc x_c))."""
+    out = {}
+    for t, m in enumerate(monos):
+        node = out.setdefault(m[0], [None, {}])
+        if len(m) == 1:
+            node[0] = t
+            continue
+        leaf = node[1].setdefault(m[1], [None, []])
+        if len(m) == 2:
+            leaf[0] = t
+        else:
+            leaf[1].append((m[2], t))
+    return out
+
+
+def coef(t):
+    return f"ld(cf + {t} * S)"
+
+
+def inner(leaf, grad):
+    """r = c_ab + sum_c c_abc x_c, with the gradient terms of the x_c."""
+    t, cubic = leaf
+    first = t is None
+    out = [] if first else [f"r = {coef(t)};"]
+    for c, u in cubic:
+        if grad:
+            out.append(f"k = {coef(u)}; g[{c}] = fm(wab, k, g[{c}]);")
+        k = "k" if grad else coef(u)
+        out.append(f"r = ml({k}, x[{c}]);" if first else f"r = fm({k}, x[{c}], r);")
+        first = False
+    return out
 
 
 def value_fn(name, monos):
-    # one sum: the layer-0 kernel evaluates several of these side by side (four partial
-    # sums each measured slower there); the node tail's value_grad uses four
-    out = [f"__device__ __forceinline__ float {name}(const float* x, const float* __restrict__ cf, int C) {{",
-           "  float f = 0.0f;"]
-    for t, m in enumerate(monos):
-        out.append(f"  f = fmaf(__ldg(cf + {t} * C), {term(m)}, f);")
+    out = ["template <typename V>", f"__device__ __forceinline__ V {name}(const V* x, const V* __restrict__ cf, int S) {{",
+           "  V f, q, r;"]
+    started = False
+    for a, (t, bs) in tree(monos).items():
+        first = t is None
+        if not first:
+            out.append(f"  q = {coef(t)};")
+        for b, leaf in bs.items():
+            out.append("  " + " ".join(inner(leaf, False) + [f"q = ml(x[{b}], r);" if first else f"q = fm(x[{b}], r, q);"]))
+            first = False
+        out.append(f"  f = fm(x[{a}], q, f);" if started else f"  f = ml(x[{a}], q);")
+        started = True
     out += ["  return f;", "}"]
     return "\n".join(out)
 
 
-def grad_lines(monos, scaled):
-    out = []
-    for t, m in enumerate(monos):
-        q = f"w * __ldg(cf + {t} * C)" if scaled else f"__ldg(cf + {t} * C)"
-        out.append(f"  {{ const float q = {q};")
-        if len(m) == 1:
-            out.append(f"    g[{m[0]}] += q;")
-        else:
-            for i, a in enumerate(m):
-                rest = [b for j, b in enumerate(m) if j != i]
-                out.append(f"    g[{a}] = fmaf(q, {term(rest)}, g[{a}]);")
-        out.append("  }")
+def grad_body(monos, value):
+    """g[v] += w dP/dx_v, and with `value` f = P."""
+    out, started = [], False
+    for a, (t, bs) in tree(monos).items():
+        out.append(f"  wa = ml(w, x[{a}]);")
+        first = t is None
+        if not first:
+            out.append(f"  q = {coef(t)};")
+        for b, leaf in bs.items():
+            line = [f"wab = ml(wa, x[{b}]);"] if leaf[1] else []
+            line += inner(leaf, True)
+            line += [f"q = ml(x[{b}], r);" if first else f"q = fm(x[{b}], r, q);", f"g[{b}] = fm(wa, r, g[{b}]);"]
+            out.append("  " + " ".join(line))
+            first = False
+        out.append(f"  g[{a}] = fm(w, q, g[{a}]);")
+        if value:
+            out.append(f"  f = fm(x[{a}], q, f);" if started else f"  f = ml(x[{a}], q);")
+            started = True
     return out
 
 
 def grad_fn(name, monos):
-    out = [f"__device__ __forceinline__ void {name}(const float* x, float w, const float* __restrict__ cf, int C, "
-           f"float* g) {{"]
-    out += grad_lines(monos, True)
-    out.append("}")
-    return "\n".join(out)
+    out = ["template <typename V>",
+           f"__device__ __forceinline__ void {name}(const V* x, V w, const V* __restrict__ cf, int S, V* g) {{",
+           "  V q, r, k, wa, wab;"]
+    return "\n".join(out + grad_body(monos, False) + ["}"])
 
 
 def value_grad_fn(name, monos):
-    out = [f"__device__ __forceinline__ float {name}(const float* x, const float* __restrict__ cf, int C, "
-           f"float* g) {{", "  float f0 = 0.0f, f1 = 0.0f, f2 = 0.0f, f3 = 0.0f;"]
-    for t, m in enumerate(monos):
-        out.append(f"  {{ const float q = __ldg(cf + {t} * C);")
-        out.append(f"    f{t % 4} = fmaf(q, {term(m)}, f{t % 4});")
-        if len(m) == 1:
-            out.append(f"    g[{m[0]}] += q;")
-        else:
-            for i, a in enumerate(m):
-                rest = [b for j, b in enumerate(m) if j != i]
-                out.append(f"    g[{a}] = fmaf(q, {term(rest)}, g[{a}]);")
-        out.append("  }")
-    out += ["  return (f0 + f1) + (f2 + f3);", "}"]
-    return "\n".join(out)
+    # (the gradient unweighted: w = 1, whose products the compiler drops)
+    out = ["template <typename V>",
+           f"__device__ __forceinline__ V {name}(const V* x, const V* __restrict__ cf, int S, V* g) {{",
+           "  V f, q, r, k, wa, wab;"]
+    body = [l.replace("  wa = ml(w, ", "  wa = (").replace("fm(w, q, g[", "ad(q, g[") for l in grad_body(monos, True)]
+    return "\n".join(out + body + ["  return f;", "}"])
 
 
 def main(out_dir=HERE):
@@ -112,8 +148,17 @@ def main(out_dir=HERE):
     with open(os.path.join(out_dir, "poly_canon_tables.h"), "w") as f:
         f.write("\n".join(t))
     h = ["// Generated by gen_poly.py: canonical symmetric-contraction monomials (l_max 3,",
-         "// degree <= 3) as straight-line code.  Do not edit; rerun the script.",
-         "#pragma once", "", '#include "poly_canon_tables.h"', "", "namespace smx {", "namespace poly {", ""]
+         "// degree <= 3) as straight-line code, for one channel (float) or two (float2, packed FMAs).",
+         "// Do not edit; rerun the script.",
+         "#pragma once", "", '#include "poly_canon_tables.h"', "", "namespace smx {", "namespace poly {", "",
+         "__device__ __forceinline__ float ld(const float* p) { return __ldg(p); }",
+         "__device__ __forceinline__ float2 ld(const float2* p) { return __ldg(p); }",
+         "__device__ __forceinline__ float fm(float a, float b, float c) { return fmaf(a, b, c); }",
+         "__device__ __forceinline__ float2 fm(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }",
+         "__device__ __forceinline__ float ml(float a, float b) { return a * b; }",
+         "__device__ __forceinline__ float2 ml(float2 a, float2 b) { return __fmul2_rn(a, b); }",
+         "__device__ __forceinline__ float ad(float a, float b) { return a + b; }",
+         "__device__ __forceinline__ float2 ad(float2 a, float2 b) { return __fadd2_rn(a, b); }", ""]
     for LM, lst in enumerate(lists):
         h.append(value_fn(f"value_LM{LM}", lst))
         h.append("")

@@ -1,20 +1,25 @@
-// Edge kernels: the neighbour sums of both interaction layers and their adjoints.
-//
-// One thread block per centre node i, one thread per channel k (blockDim = C).
-// Edges of node i are staged kernel-wide in chunks of kEdgeChunk: geometry,
-// spline interval, Y_lm (and dY/dx in the adjoints) are computed once per edge by
-// one thread and shared; every thread then runs the per-channel arithmetic for
-// its k with channel-fastest, coalesced loads of spline coefficients (float4:
-// one cubic per (spline, channel)) and neighbour features.  Sums over neighbours
-// accumulate in registers of the destination node's block, so the forward
-// A-basis and Phi1 sums use no atomics.
+// Layer-0 kernels: the neighbour sum A0 with its symmetric contraction M0, and their adjoints.
 //
 // Reference stages restated here (libsymmetrix/source/mace.cpp):
-//   k_layer0_fwd : compute_Y + compute_R0 + compute_A0 (:66-201) + compute_M0 (:348-370)
-//   k_layer0_rev : reverse_M0 + reverse_A0 (:372-395, :203-271)
+//   k_layer0_fwd    : compute_Y + compute_R0 + compute_A0 (:66-201) + compute_M0 (:348-370)
+//   k_contract0_rev : reverse_M0 (:372-395)
+//   k_layer0_rev    : reverse_A0 (:203-271)
+//
+// The edge kernels run one warp per node (and 64 channels in the forward), a warp being a
+// block: no block barriers, all per-channel arithmetic on channel pairs with the packed FMA,
+// and the next edge's cubics loaded into the registers that this edge's have left.  What
+// bounds them is the L2 gather of the folded spline rows, 8 KB per edge at 128 channels
+// (0.09 ms for 213k edges at the 19.6 TB/s of a plain gather), and of the contraction's
+// coefficients, 0.2 MB per node.  Against a block of two warp groups per node whose sums met
+// in shared memory, five-and-forty scalar FMAs per edge and channel for the force and
+// polynomials with the products of pairs in registers (255 of them): 4096 atoms, 128
+// channels, forward 0.165 -> 0.137 ms, adjoints together 0.262 -> 0.182 ms; L_max = 2, 2197
+// atoms 0.225 -> 0.126 and 0.260 -> 0.186 ms.
 #include <cuda_runtime.h>
 
-#include "device.cuh"
+#include <algorithm>
+
+#include "edge.cuh"
 #include "kernels.h"
 #include "poly_canon.h"
 
@@ -22,489 +27,573 @@ namespace smx {
 
 namespace {
 
-// Sum a per-thread 3-vector over the block's channels for edge t: float32 warp
-// shuffles (float64 arithmetic is slow on this part), then one partial per warp into
-// sF, summed across warps in float64 after the chunk.  The lanes first trade halves of
-// the vector (x, y | z, 0) with their xor-1 and xor-2 partners, so each lane then holds
-// one component summed over its group of four lanes (lane & 3: 0 x, 1 z, 2 y, 3
-// nothing), and three butterfly steps sum the groups: six shuffles where three separate
-// warp sums take fifteen (k_layer0_rev 0.313 -> 0.283 ms on the 4096-atom workload).
-// The order of the additions is fixed, so results are reproducible.
-__device__ __forceinline__ void block_reduce3(float fx, float fy, float fz, float (*sF)[8][3], int t) {
-  constexpr unsigned kFull = 0xffffffffu;
-  const int lane = threadIdx.x & 31;
-  const bool b0 = lane & 1, b1 = lane & 2;
-  float k0 = b0 ? fz : fx, k1 = b0 ? 0.0f : fy;
-  const float s0 = b0 ? fx : fz, s1 = b0 ? fy : 0.0f;
-  k0 += __shfl_xor_sync(kFull, s0, 1);
-  k1 += __shfl_xor_sync(kFull, s1, 1);
-  float v = b1 ? k1 : k0;
-  v += __shfl_xor_sync(kFull, b1 ? k0 : k1, 2);
-  v += __shfl_xor_sync(kFull, v, 4);
-  v += __shfl_xor_sync(kFull, v, 8);
-  v += __shfl_xor_sync(kFull, v, 16);
-  if (lane < 3) sF[t][threadIdx.x >> 5][lane == 1 ? 2 : lane == 2 ? 1 : 0] = v;
-}
-
-}  // namespace
-
-namespace {
-
-// Edge chunk staged for the layer-0 kernels: Y_lm (and, for the adjoint, dY/dx, dY/dy,
-// dY/dz) packed as float4 rows, the ordered-pair spline row of the folded layer-0 table, and the
-// compacted list of active edges (r < r_cut).
-template <bool GRAD>
+// Up to 32 edges of a node staged by one warp, those inside the cut-off packed to the front.
 struct L0Stage {
-  float2 Y2[kEdgeChunk][16];  // (Y_lm, Y_lm): operand of the packed FMAs
-  float4 G[GRAD ? kEdgeChunk : 1][16];  // (dY_lm/dx, dY_lm/dy, dY_lm/dz, Y_lm): one load per lm
-  float4 u[GRAD ? kEdgeChunk : 1];
-  float x[kEdgeChunk];
-  int row[kEdgeChunk];  // (ti * S + tj) * nint + interval, or -1
-  int act[kEdgeChunk];
-  int nact;
+  alignas(16) float2 Y2[kEdgeChunk][16];  // (Y_lm, Y_lm): operands of the packed FMAs
+  int2 meta[kEdgeChunk];      // offset inside the spline interval (float bits), ordered-pair spline row
 };
 
-template <bool GRAD>
-__device__ __forceinline__ void stage_l0(const DevModel& m, const EdgeIn& in, int ti, int eb, int ne,
-                                         L0Stage<GRAD>& st) {
-  if (threadIdx.x >= 32) return;
-  const int t = threadIdx.x;
-  bool active = false;
-  if (t < ne) {
-    const long e = static_cast<long>(eb) + t;
-    const float vx = static_cast<float>(in.xyz[3 * e]);
-    const float vy = static_cast<float>(in.xyz[3 * e + 1]);
-    const float vz = static_cast<float>(in.xyz[3 * e + 2]);
-    const float rr = static_cast<float>(in.r[e]);
-    float Y[16], G[GRAD ? 48 : 1];
-    sph_harm16<GRAD>(vx, vy, vz, Y, G);
-#pragma unroll
-    for (int q = 0; q < 16; ++q) st.Y2[t][q] = make_float2(Y[q], Y[q]);
-    if constexpr (GRAD) {
-#pragma unroll
-      for (int c = 0; c < 16; ++c) st.G[t][c] = make_float4(G[c], G[16 + c], G[32 + c], Y[c]);
-      const float inv = 1.0f / rr;
-      st.u[t] = make_float4(vx * inv, vy * inv, vz * inv, 0.0f);
-    }
-    const int iv = spline_at(m, in.r[e], st.x[t]);
-    active = rr < m.r_cut;
-    st.row[t] = active ? (ti * m.S + in.ntype_e[e]) * m.nint + iv : -1;
-  }
+// rows first, so that the first edge's loads can go out (as stage_rows in layer1.cuh)
+__device__ __forceinline__ int stage_rows0(const DevModel& m, L0Stage& st, const LaneEdge& ed, int ti, bool active,
+                                           int& count) {
   const unsigned ball = __ballot_sync(0xffffffffu, active);
-  if (active) st.act[__popc(ball & ((1u << t) - 1u))] = t;
-  if (t == 0) st.nact = __popc(ball);
+  const int pos = __popc(ball & ((1u << (threadIdx.x & 31)) - 1u));
+  count = __popc(ball);
+  __syncwarp();  // the last chunk has been read
+  if (active) st.meta[pos] = make_int2(__float_as_int(ed.x), (ti * m.S + ed.tj) * m.nint + ed.iv);
+  __syncwarp();
+  return pos;
 }
+__device__ __forceinline__ void stage_Y0(L0Stage& st, const LaneEdge& ed, bool active, int pos) {
+  if (active) {
+    float Y[16];
+    sph_harm16<false>(ed.vx, ed.vy, ed.vz, Y, nullptr);
+#pragma unroll
+    for (int v = 0; v < 8; ++v)
+      *reinterpret_cast<float4*>(&st.Y2[pos][2 * v]) = make_float4(Y[2 * v], Y[2 * v], Y[2 * v + 1], Y[2 * v + 1]);
+  }
+  __syncwarp();
+}
+__device__ __forceinline__ void read_Y2(const float2* Y2, float2* y) {
+#pragma unroll
+  for (int v = 0; v < 8; ++v) {
+    const float4 f = *reinterpret_cast<const float4*>(Y2 + 2 * v);
+    y[2 * v] = make_float2(f.x, f.y);
+    y[2 * v + 1] = make_float2(f.z, f.w);
+  }
+}
+
+// split terms of a channel pair (write_split)
+__device__ __forceinline__ void write_split2(__nv_bfloat16* row, int K, int T, int col, float2 v) {
+  const __nv_bfloat162 hi = __float22bfloat162_rn(v);
+  *reinterpret_cast<__nv_bfloat162*>(row + col) = hi;
+  if (T == 3) {
+    const float2 h = __bfloat1622float2(hi);
+    *reinterpret_cast<__nv_bfloat162*>(row + K + col) = __float22bfloat162_rn(make_float2(v.x - h.x, v.y - h.y));
+  }
+}
+
+// P_LM and its weighted gradient for the generated polynomials, by a compile-time LM
+template <int LM>
+__device__ __forceinline__ float2 contract_value(const float2* x, const float2* cf, int S) {
+  if constexpr (LM == 0) return poly::value_LM0(x, cf, S);
+  if constexpr (LM == 1) return poly::value_LM1(x, cf, S);
+  if constexpr (LM == 2) return poly::value_LM2(x, cf, S);
+  if constexpr (LM == 3) return poly::value_LM3(x, cf, S);
+  if constexpr (LM == 4) return poly::value_LM4(x, cf, S);
+  if constexpr (LM == 5) return poly::value_LM5(x, cf, S);
+  if constexpr (LM == 6) return poly::value_LM6(x, cf, S);
+  if constexpr (LM == 7) return poly::value_LM7(x, cf, S);
+  if constexpr (LM == 8) return poly::value_LM8(x, cf, S);
+}
+template <int LM>
+__device__ __forceinline__ void contract_grad(const float2* x, float2 w, const float2* cf, int S, float2* g) {
+  if constexpr (LM == 0) poly::grad_LM0(x, w, cf, S, g);
+  if constexpr (LM == 1) poly::grad_LM1(x, w, cf, S, g);
+  if constexpr (LM == 2) poly::grad_LM2(x, w, cf, S, g);
+  if constexpr (LM == 3) poly::grad_LM3(x, w, cf, S, g);
+  if constexpr (LM == 4) poly::grad_LM4(x, w, cf, S, g);
+  if constexpr (LM == 5) poly::grad_LM5(x, w, cf, S, g);
+  if constexpr (LM == 6) poly::grad_LM6(x, w, cf, S, g);
+  if constexpr (LM == 7) poly::grad_LM7(x, w, cf, S, g);
+  if constexpr (LM == 8) poly::grad_LM8(x, w, cf, S, g);
+}
+
+constexpr int kDepth0 = 2;  // edges in flight per warp of the forward
 
 }  // namespace
 
 // ---------------------------------------------------------------------------
 // Layer 0 forward: A0[i,lm,k] = sum_j Y_lm(x_ij) R0'_{ti,tj,l}(r_ij)[k] with the
-// folded ordered-pair splines, then M0[i,LM,k] = P_{ti,LM,k}(A0[i,:,k]).
+// folded ordered-pair splines, then M0[i,LM,k] = P_{ti,LM,k}(A0[i,:,k]) for the lane's two
+// channels.  (The contraction as a kernel of its own, a warp per output LM: 0.108 + 0.039 ms
+// against 0.137 ms together.)
 // ---------------------------------------------------------------------------
-template <int NLM>
-__device__ __forceinline__ void layer0_fwd_atom(const DevModel& m, const EdgeIn& in, float* __restrict__ A0,
-                                                float* __restrict__ M0, float* __restrict__ zbl_e, int i) {
-  extern __shared__ float dyn[];  // [17][C]: A0 columns (+ constant one) for the contraction
-  __shared__ L0Stage<false> st;
-  const int C = m.C, C2 = C >> 1, BW = (C2 + 31) & ~31;
-  // two groups of channel-pair threads, each taking every other active edge
-  const int half = static_cast<int>(threadIdx.x) >= BW ? 1 : 0;
-  const int lt = threadIdx.x - half * BW;
-  const bool live = lt < C2;
-  const int cp = live ? lt : 0, kc = 2 * cp;
+template <int NLM, int CT>
+__device__ __forceinline__ void layer0_fwd_item(const DevModel& m, const EdgeIn& in, float* __restrict__ A0,
+                                                float* __restrict__ M0, float* __restrict__ zbl_e, L0Stage& st,
+                                                float* sA, int i, int slice) {
+  const int C = CT > 0 ? CT : m.C, C2 = C >> 1;
+  const int lane = threadIdx.x & 31;
+  const bool live = slice * 32 + lane < C2;
+  const int cp = live ? slice * 32 + lane : slice * 32, kc = 2 * cp;
   const int ti = in.node_type[i];
   const int e0 = in.first[i], e1 = in.end(i);
   float2 acc[16];
 #pragma unroll
   for (int q = 0; q < 16; ++q) acc[q] = make_float2(0.0f, 0.0f);
   for (int eb = e0; eb < e1; eb += kEdgeChunk) {
-    const int ne = min(kEdgeChunk, e1 - eb);
-    __syncthreads();
-    stage_l0<false>(m, in, ti, eb, ne, st);
-    __syncthreads();
-    // this group's active edges; the next one's cubics load while this one accumulates
-    const int na = st.nact;
-    float4 c[8];
-    auto fetch = [&](int a) {
-      const float4* p = m.spl0 + static_cast<size_t>(st.row[st.act[a]]) * 4 * C + cp;
+    LaneEdge ed;
+    ed.load(m, in, min(eb + lane, e1 - 1));
+    int na;
+    const bool active = eb + lane < e1 && ed.r < m.r_cut;
+    const int pos = stage_rows0(m, st, ed, ti, active, na);
+    if (na == 0) continue;
+    float4 c[kDepth0][8];
+    static_for<kDepth0>([&](auto dc) {
+      constexpr int d = decltype(dc)::value;
+      const float4* p = m.spl0 + static_cast<size_t>(st.meta[min(d, na - 1)].y) * 4 * C + cp;
 #pragma unroll
-      for (int q = 0; q < 8; ++q) c[q] = __ldg(p + q * C2);
-    };
-    if (half < na) fetch(half);
-    for (int a = half; a < na; a += 2) {
-      const int t = st.act[a];
-      const float2 x2 = make_float2(st.x[t], st.x[t]);
-      float2 R[4];
+      for (int q = 0; q < 8; ++q) c[d][q] = __ldg(p + q * C2);
+    });
+    stage_Y0(st, ed, active, pos);
+    for (int a0 = 0; a0 < na; a0 += kDepth0) {
+      static_for<kDepth0>([&](auto dc) {
+        constexpr int d = decltype(dc)::value;
+        const int a = a0 + d;
+        if (a >= na) return;
+        const float4* p = m.spl0 + static_cast<size_t>(st.meta[min(a + kDepth0, na - 1)].y) * 4 * C + cp;
+        const float x = __int_as_float(st.meta[a].x);
+        const float2 x2 = make_float2(x, x);
+        float2 y[16];
+        read_Y2(st.Y2[a], y);
+        static_for<4>([&](auto lc) {
+          constexpr int l = decltype(lc)::value;
+          const float2 R = spline2_val(c[d][2 * l], c[d][2 * l + 1], x2);
+          c[d][2 * l] = __ldg(p + 2 * l * C2);
+          c[d][2 * l + 1] = __ldg(p + (2 * l + 1) * C2);
+          if constexpr (l == 0) {
+            acc[0] = __fadd2_rn(R, acc[0]);  // Y_00 = 1 (sph_harm16)
+          } else {
 #pragma unroll
-      for (int l = 0; l < 4; ++l) R[l] = spline2_val(c[2 * l], c[2 * l + 1], x2);
-      if (a + 2 < na) fetch(a + 2);
-      acc[0] = __fadd2_rn(R[0], acc[0]);  // Y_00 = 1 (sph_harm16)
-#pragma unroll
-      for (int q = 1; q < 16; ++q) {
-        const int l = q < 4 ? 1 : (q < 9 ? 2 : 3);
-        acc[q] = fma2(R[l], st.Y2[t][q], acc[q]);
-      }
+            for (int q = l * l; q < (l + 1) * (l + 1); ++q) acc[q] = fma2(R, y[q], acc[q]);
+          }
+        });
+      });
     }
   }
-  if (m.has_zbl) {  // ZBL energy of node i: sum over its directed edges (zbl.cpp:96-125)
+  if (m.has_zbl && slice == 0) {  // ZBL energy of node i: sum over its directed edges (zbl.cpp:96-125)
     float z = 0.0f;
-    for (int e = e0 + threadIdx.x; e < e1; e += blockDim.x) {
+    for (int e = e0 + lane; e < e1; e += 32) {
       float V, dV;
       zbl_edge(m, m.zbl_pair[ti * m.S + in.ntype_e[e]], static_cast<float>(in.r[e]), V, dV);
       z += V;
     }
-    z = block_sum(z);
-    if (threadIdx.x == 0) zbl_e[i] = z;
+    z = warp_sum(z);
+    if (lane == 0) zbl_e[i] = z;
   }
-  float S = 1.0f;
   if (m.dens_spl[0]) {  // density-normalised A0: A0 /= 1 + sum_j s(r_ij)  (mace.cpp:273-297)
-    S = dens_factor(m, 0, in, i, ti);
-    if (threadIdx.x == 0) m.dens_s[0][i] = S;
+    const float S = dens_factor(m, 0, in, i, ti);
+    if (lane == 0 && slice == 0) m.dens_s[0][i] = S;
+#pragma unroll
+    for (int q = 0; q < 16; ++q) acc[q] = make_float2(acc[q].x / S, acc[q].y / S);
   }
-  float* sA = dyn;
-  if (half == 1 && live)
+  if (live)
 #pragma unroll
-    for (int q = 0; q < 16; ++q) *reinterpret_cast<float2*>(sA + q * C + kc) = acc[q];
-  __syncthreads();
-  if (half == 0 && live) {
-#pragma unroll
-    for (int q = 0; q < 16; ++q) {
-      const float2 o = *reinterpret_cast<const float2*>(sA + q * C + kc);
-      float2 v = make_float2(acc[q].x + o.x, acc[q].y + o.y);
-      if (S != 1.0f) v = make_float2(v.x / S, v.y / S);  // (no division sequence without the scaling)
-      *reinterpret_cast<float2*>(sA + q * C + kc) = v;
-      *reinterpret_cast<float2*>(A0 + (static_cast<size_t>(i) * 16 + q) * C + kc) = v;
-    }
+    for (int q = 0; q < 16; ++q)
+      *reinterpret_cast<float2*>(A0 + (static_cast<size_t>(i) * 16 + q) * C + kc) = acc[q];
+  auto put = [&](int LM, float2 v) {  // M0 nullptr: only the split rows are consumed
+    if (!live) return;
+    if (M0) *reinterpret_cast<float2*>(M0 + (static_cast<size_t>(i) * m.nLM + LM) * C + kc) = v;
+    if (m.op_m0)  // BF16 form: the H1 GEMM's split operand
+      write_split2(m.op_m0 + (static_cast<size_t>(i) * m.nLM + LM) * split_xterms(m.tc_terms) * C, C, m.tc_terms, kc, v);
+  };
+  if (m.poly_canon) {  // generated straight-line polynomials, A0 columns in registers
+    const float2* cf = reinterpret_cast<const float2*>(m.coef0 + static_cast<size_t>(ti * m.nLM) * m.T0 * C) + cp;
+    const size_t sst = static_cast<size_t>(m.T0) * C2;
+    static_for<NLM>([&](auto lc) {
+      constexpr int LM = decltype(lc)::value;
+      put(LM, contract_value<LM>(acc, cf + LM * sst, C2));
+    });
+    return;
   }
-  for (int k = threadIdx.x; k < C; k += blockDim.x) sA[16 * C + k] = 1.0f;
-  __syncthreads();
-  // the symmetric contraction, one thread per channel
-  for (int k = threadIdx.x; k < C; k += blockDim.x) {
-    if (m.poly_canon) {  // generated straight-line polynomials, A0 column in registers
-      float x[16];
+  float2* x = reinterpret_cast<float2*>(sA) + lane;  // [17][32]: this lane's columns (+ constant one)
 #pragma unroll
-      for (int q = 0; q < 16; ++q) x[q] = sA[q * C + k];
-      const float* cf = m.coef0 + static_cast<size_t>(ti * m.nLM) * m.T0 * C + k;
-      const size_t sst = static_cast<size_t>(m.T0) * C;
-      float* out = M0 + static_cast<size_t>(i) * m.nLM * C + k;
-      float v[9];
-      v[0] = poly::value_LM0(x, cf, C);
-      v[1] = poly::value_LM1(x, cf + sst, C);
-      v[2] = poly::value_LM2(x, cf + 2 * sst, C);
-      v[3] = poly::value_LM3(x, cf + 3 * sst, C);
-      if constexpr (NLM == 9) {  // L_max = 2: the five l = 2 outputs
-        v[4] = poly::value_LM4(x, cf + 4 * sst, C);
-        v[5] = poly::value_LM5(x, cf + 5 * sst, C);
-        v[6] = poly::value_LM6(x, cf + 6 * sst, C);
-        v[7] = poly::value_LM7(x, cf + 7 * sst, C);
-        v[8] = poly::value_LM8(x, cf + 8 * sst, C);
-      }
-#pragma unroll
-      for (int LM = 0; LM < NLM; ++LM) {
-        if (M0) out[LM * C] = v[LM];  // nullptr: only the split rows are consumed
-        if (m.op_m0)  // BF16 form: the H1 GEMM's split operand
-          write_split(m.op_m0 + (static_cast<size_t>(i) * m.nLM + LM) * split_xterms(m.tc_terms) * C, C, m.tc_terms,
-                      k, v[LM]);
-      }
-      continue;
+  for (int q = 0; q < 16; ++q) x[q * 32] = acc[q];
+  x[16 * 32] = make_float2(1.0f, 1.0f);
+  for (int LM = 0; LM < m.nLM; ++LM) {
+    const int t0 = m.mono0_off[LM], t1 = m.mono0_off[LM + 1];
+    const float2* cf = reinterpret_cast<const float2*>(m.coef0 + (static_cast<size_t>(ti * m.nLM + LM) * m.T0) * C) + cp;
+    float2 f = make_float2(0.0f, 0.0f);
+    for (int t = t0; t < t1; ++t) {
+      const int pk = __ldg(m.mono0 + t);
+      const float2 p = mul2(mul2(x[(pk & 255) * 32], x[((pk >> 8) & 255) * 32]), x[(pk >> 16) * 32]);
+      f = fma2(__ldg(cf + static_cast<size_t>(t - t0) * C2), p, f);
     }
-    for (int LM = 0; LM < m.nLM; ++LM) {
-      const int t0 = m.mono0_off[LM], t1 = m.mono0_off[LM + 1];
-      const float* cf = m.coef0 + (static_cast<size_t>(ti * m.nLM + LM) * m.T0) * C + k;
-      float f = 0.0f;
-      for (int t = t0; t < t1; ++t) {
-        const int pk = __ldg(m.mono0 + t);
-        const float xa = sA[(pk & 255) * C + k], xb = sA[((pk >> 8) & 255) * C + k], xc = sA[(pk >> 16) * C + k];
-        f = fmaf(__ldg(cf + static_cast<size_t>(t - t0) * C), xa * xb * xc, f);
-      }
-      if (M0) M0[(static_cast<size_t>(i) * m.nLM + LM) * C + k] = f;
-      if (m.op_m0)
-        write_split(m.op_m0 + (static_cast<size_t>(i) * m.nLM + LM) * split_xterms(m.tc_terms) * C, C, m.tc_terms, k,
-                    f);
-    }
+    put(LM, f);
   }
 }
 
-template <bool P, int NLM>
-__global__ void __launch_bounds__(256) k_layer0_fwd(DevModel m, EdgeIn in, float* __restrict__ A0,
-                                                    float* __restrict__ M0, float* __restrict__ zbl_e) {
+__host__ __device__ inline int layer0_slices(int C) { return (C + 63) / 64; }
+
+// (this kernel and k_contract0_rev hold the generated polynomials and have no persistent form:
+// their blocks are single warps, which gain nothing from one, and the code would double)
+template <int NLM, int CT>
+__global__ void __launch_bounds__(32, 12) k_layer0_fwd(DevModel m, EdgeIn in, float* __restrict__ A0,
+                                                       float* __restrict__ M0, float* __restrict__ zbl_e) {
   pdl_begin();
-  AtomCursor cur{P ? m.sched : nullptr, in.N, 0};
-  for (int b = cur.first(); b < in.N; b = cur.next())
-    layer0_fwd_atom<NLM>(m, in, A0, M0, zbl_e, in.atom_at(b));
-  cur.done();
+  __shared__ L0Stage st;
+  extern __shared__ float dyn[];
+  const int ns = layer0_slices(CT > 0 ? CT : m.C), b = blockIdx.x;
+  layer0_fwd_item<NLM, CT>(m, in, A0, M0, zbl_e, st, dyn, in.atom_at(b / ns), b % ns);
 }
 
 // ---------------------------------------------------------------------------
 // Layer-0 contraction adjoint (mace.cpp:372-395):
 //   A0_adj[i,:,k] = sum_LM M0_adj[i,LM,k] grad P_{ti,LM,k}(A0[i,:,k]).
-// Its own kernel, so its register-heavy generated code does not limit the occupancy
-// of the layer-0 edge adjoint.
+// A block per node, a lane per channel pair: one warp per 64 channels, or (SPLIT, small
+// systems) a warp per output LM and 64 channels, whose gradients meet in shared memory and
+// are added in the order of LM.
 // ---------------------------------------------------------------------------
-template <int NLM>
-__device__ __forceinline__ void contract0_rev_atom(const DevModel& m, const int* __restrict__ node_type,
-                                                   const float* __restrict__ A0, const float* __restrict__ M0_adj,
-                                                   float* __restrict__ A0_adj, int i) {
+constexpr int contract0_max_warps(int NLM, int CT, bool SPLIT) {
+  return (SPLIT ? NLM : 1) * (CT > 0 ? (CT + 63) / 64 : (NLM == 9 ? 2 : 4));
+}
+// (SPLIT: 20 warps per SM)
+template <int NLM, int CT, bool SPLIT>
+__global__ void __launch_bounds__(32 * contract0_max_warps(NLM, CT, SPLIT),
+                                  !SPLIT || contract0_max_warps(NLM, CT, SPLIT) > 10
+                                      ? 1
+                                      : 20 / contract0_max_warps(NLM, CT, SPLIT))
+    k_contract0_rev(DevModel m, const int* __restrict__ node_type, const int* __restrict__ order, const float* __restrict__ A0,
+                    const float* __restrict__ M0_adj, float* __restrict__ A0_adj) {
+  pdl_begin();
   extern __shared__ float dyn[];
-  const int C = m.C, k = threadIdx.x;
+  const int C = CT > 0 ? CT : m.C, C2 = C >> 1, ns = layer0_slices(C);
+  const int i = order ? order[blockIdx.x] : blockIdx.x;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
+  const int slice = SPLIT ? warp % ns : warp, part = SPLIT ? warp / ns : 0, parts = SPLIT ? m.nLM : 1;
+  const bool live = slice * 32 + lane < C2;
+  const int cp = live ? slice * 32 + lane : slice * 32;
   const int ti = node_type[i];
-  float dA[16];
-  if (m.poly_canon) {  // dA0 = sum_LM dM0[LM] grad P_LM, generated code, registers only
-    float x[16];
+  const float2* xr = reinterpret_cast<const float2*>(A0 + static_cast<size_t>(i) * 16 * C) + cp;
+  const float2* w = reinterpret_cast<const float2*>(M0_adj + static_cast<size_t>(i) * m.nLM * C) + cp;
+  const size_t sst = static_cast<size_t>(m.T0) * C2;
+  const float2* cf = reinterpret_cast<const float2*>(m.coef0 + static_cast<size_t>(ti * m.nLM) * m.T0 * C) + cp;
+  float2 x[16], dA[16];
 #pragma unroll
-    for (int q = 0; q < 16; ++q) {
-      x[q] = A0[(static_cast<size_t>(i) * 16 + q) * C + k];
-      dA[q] = 0.0f;
-    }
-    const float* cf = m.coef0 + static_cast<size_t>(ti * m.nLM) * m.T0 * C + k;
-    const size_t st = static_cast<size_t>(m.T0) * C;
-    const float* w = M0_adj + static_cast<size_t>(i) * m.nLM * C + k;
-    poly::grad_LM0(x, w[0], cf, C, dA);
-    poly::grad_LM1(x, w[C], cf + st, C, dA);
-    poly::grad_LM2(x, w[2 * C], cf + 2 * st, C, dA);
-    poly::grad_LM3(x, w[3 * C], cf + 3 * st, C, dA);
-    if constexpr (NLM == 9) {  // L_max = 2: the five l = 2 outputs
-      poly::grad_LM4(x, w[4 * C], cf + 4 * st, C, dA);
-      poly::grad_LM5(x, w[5 * C], cf + 5 * st, C, dA);
-      poly::grad_LM6(x, w[6 * C], cf + 6 * st, C, dA);
-      poly::grad_LM7(x, w[7 * C], cf + 7 * st, C, dA);
-      poly::grad_LM8(x, w[8 * C], cf + 8 * st, C, dA);
-    }
-  } else {  // data-driven monomial lists, this thread's columns in shared memory
-    float* sA = dyn;            // [17][C] A0 column
-    float* sGd = dyn + 17 * C;  // [17][C] gradient column (row 16 absorbs the constant slot)
+  for (int q = 0; q < 16; ++q) {
+    x[q] = __ldg(xr + q * C2);
+    dA[q] = make_float2(0.0f, 0.0f);
+  }
+  if (m.poly_canon) {  // generated code, registers only
+    static_for<NLM>([&](auto lc) {
+      constexpr int LM = decltype(lc)::value;
+      if (!SPLIT || LM == part) contract_grad<LM>(x, __ldg(w + LM * C2), cf + LM * sst, C2, dA);
+    });
+  } else {  // data-driven monomial lists, this lane's columns in shared memory
+    float2* sA = reinterpret_cast<float2*>(dyn) + warp * 17 * 32 * 2 + lane;  // [17][32]
+    float2* sG = sA + 17 * 32;                                               // (row 16 absorbs the constant slot)
 #pragma unroll
-    for (int q = 0; q < 16; ++q) {
-      sA[q * C + k] = A0[(static_cast<size_t>(i) * 16 + q) * C + k];
-      sGd[q * C + k] = 0.0f;
+    for (int q = 0; q < 17; ++q) {
+      sA[q * 32] = q < 16 ? x[q < 16 ? q : 0] : make_float2(1.0f, 1.0f);
+      sG[q * 32] = make_float2(0.0f, 0.0f);
     }
-    sA[16 * C + k] = 1.0f;
-    sGd[16 * C + k] = 0.0f;
-    for (int LM = 0; LM < m.nLM; ++LM) {
-      const float w = M0_adj[(static_cast<size_t>(i) * m.nLM + LM) * C + k];
+    for (int LM = part; LM < m.nLM; LM += parts) {
+      const float2 wl = __ldg(w + LM * C2);
       const int t0 = m.mono0_off[LM], t1 = m.mono0_off[LM + 1];
-      const float* cf = m.coef0 + (static_cast<size_t>(ti * m.nLM + LM) * m.T0) * C + k;
       for (int t = t0; t < t1; ++t) {
         const int pk = __ldg(m.mono0 + t);
-        const int a = pk & 255, b = (pk >> 8) & 255, c = pk >> 16;
-        const float cw = __ldg(cf + static_cast<size_t>(t - t0) * C) * w;
-        const float xa = sA[a * C + k], xb = sA[b * C + k], xc = sA[c * C + k];
-        sGd[a * C + k] += cw * xb * xc;
-        sGd[b * C + k] += cw * xa * xc;
-        sGd[c * C + k] += cw * xa * xb;
+        const int a = (pk & 255) * 32, b = ((pk >> 8) & 255) * 32, c = (pk >> 16) * 32;
+        const float2 cw = mul2(__ldg(cf + LM * sst + static_cast<size_t>(t - t0) * C2), wl);
+        const float2 xa = sA[a], xb = sA[b], xc = sA[c];
+        sG[a] = fma2(mul2(cw, xb), xc, sG[a]);
+        sG[b] = fma2(mul2(cw, xa), xc, sG[b]);
+        sG[c] = fma2(mul2(cw, xa), xb, sG[c]);
       }
+      if (SPLIT) break;
     }
 #pragma unroll
-    for (int q = 0; q < 16; ++q) dA[q] = sGd[q * C + k];
+    for (int q = 0; q < 16; ++q) dA[q] = sG[q * 32];
   }
-  if (m.dens_spl[0]) {  // reverse_A0_scaled (mace.cpp:299-346): c_i = dA . A0 / s_i, dA /= s_i
-    float dot = 0.0f;
-#pragma unroll
-    for (int q = 0; q < 16; ++q) dot = fmaf(dA[q], A0[(static_cast<size_t>(i) * 16 + q) * C + k], dot);
-    dot = block_sum(dot);
-    const float S = m.dens_s[0][i];
+  float2* out = reinterpret_cast<float2*>(A0_adj + static_cast<size_t>(i) * 16 * C) + cp;
+  float S = 1.0f;  // reverse_A0_scaled (mace.cpp:299-346): c_i = dA . A0 / s_i, dA /= s_i
+  auto density = [&](float2 d2) {
+    const float dot = block_sum(live ? d2.x + d2.y : 0.0f);
+    S = m.dens_s[0][i];
     if (threadIdx.x == 0) m.dens_c[0][i] = dot / S;
+  };
+  auto store = [&](int q, float2 v) {
+    if (m.dens_spl[0]) v = make_float2(v.x / S, v.y / S);
+    if (live) out[q * C2] = v;
+  };
+  float2 d2 = make_float2(0.0f, 0.0f);
+  if constexpr (!SPLIT) {
+    if (m.dens_spl[0]) {
 #pragma unroll
-    for (int q = 0; q < 16; ++q) dA[q] /= S;
+      for (int q = 0; q < 16; ++q) d2 = fma2(dA[q], x[q], d2);
+      density(d2);
+    }
+#pragma unroll
+    for (int q = 0; q < 16; ++q) store(q, dA[q]);
+  } else {
+    // [nwarp][16][32], behind the data-driven columns
+    float2* sum = reinterpret_cast<float2*>(dyn) + (m.poly_canon ? 0 : nwarp * 17 * 32 * 2) + lane;
+#pragma unroll
+    for (int q = 0; q < 16; ++q) sum[(warp * 16 + q) * 32] = dA[q];
+    __syncthreads();
+    auto row = [&](int q) {  // warp (LM, slice) takes the rows q = LM (mod nLM) of its slice
+      float2 s = sum[(slice * 16 + q) * 32];
+      for (int u = 1; u < parts; ++u) s = __fadd2_rn(s, sum[((u * ns + slice) * 16 + q) * 32]);
+      return s;
+    };
+    if (m.dens_spl[0]) {
+      for (int q = part; q < 16; q += parts) d2 = fma2(row(q), __ldg(xr + q * C2), d2);
+      density(d2);
+    }
+    for (int q = part; q < 16; q += parts) store(q, row(q));
   }
-#pragma unroll
-  for (int q = 0; q < 16; ++q) A0_adj[(static_cast<size_t>(i) * 16 + q) * C + k] = dA[q];
 }
-
-template <bool P, int NLM>
-__global__ void __launch_bounds__(256) k_contract0_rev(DevModel m, const int* __restrict__ node_type,
-                                                       const float* __restrict__ A0, const float* __restrict__ M0_adj,
-                                                       float* __restrict__ A0_adj, int N) {
-  pdl_begin();
-  AtomCursor cur{P ? m.sched : nullptr, N, 0};
-  for (int i = cur.first(); i < N; i = cur.next()) contract0_rev_atom<NLM>(m, node_type, A0, M0_adj, A0_adj, i);
-  cur.done();
-}
-
-
 
 // ---------------------------------------------------------------------------
 // Layer-0 edge adjoint (mace.cpp:203-271): dE/dx_ij from A0_adj through the folded
-// radial splines and Y_lm; ZBL and the density factor add their terms; forces =
-// -(layer 0 + layer 1).  The next active edge's four spline cubics are loaded while
-// this edge computes.
+// radial splines and Y_lm; ZBL and the density factors add their terms; forces =
+// -(layer 0 + layer 1).  A warp sums all channels of its node's edges, up to two channel
+// pairs per lane at a time: dE/dY_lm and the radial term over the lanes four edges at a
+// time, and only these sums meet dY_lm/dx.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void layer0_rev_atom(const DevModel& m, const EdgeIn& in, const float* __restrict__ A0_adj,
-                                                const float* __restrict__ f1, double* __restrict__ forces, int i) {
-  __shared__ L0Stage<true> st;
-  __shared__ float sF[kEdgeChunk][8][3];
-  const int C = m.C, C2 = C >> 1;
-  const bool live = static_cast<int>(threadIdx.x) < C2;
-  const int cp = live ? threadIdx.x : 0, kc = 2 * cp;  // this thread's channel pair
-  const int nwarp = blockDim.x >> 5;
+namespace {
+
+struct Rev0Smem {
+  L0Stage st;
+  float S[kEdgeChunk][16];  // (dE/dr term, dE/dY_1 .. dE/dY_15) of the staged edges
+  float2 buf[kSumEdges * 8 * kSumRow];
+};
+
+}  // namespace
+
+template <int CT>
+__device__ __forceinline__ void layer0_rev_item(const DevModel& m, const EdgeIn& in, const float* __restrict__ A0_adj,
+                                                const float* __restrict__ f1, double* __restrict__ forces,
+                                                Rev0Smem& s, int i, int part, int split, int cs) {
+  constexpr int NP = CT > 0 && CT <= 64 ? 1 : 2;  // channel pairs per lane
+  const int C = CT > 0 ? CT : m.C, C2 = C >> 1;
+  const int lane = threadIdx.x & 31;
   const int ti = in.node_type[i];
   const int e0 = in.first[i], e1 = in.end(i);
+  if (e0 + part * cs >= e1) return;
   const bool local = i < in.n_local;  // a halo centre: layer 0 only
-  float2 dA[16];
+  LaneEdge ed;
+  ed.load(m, in, min(e0 + part * cs + lane, e1 - 1));
+  // the lane's pairs cb + lane, cb + lane + 32 of a channel block; zero adjoints past the last
+  float2 dA[NP][16];
+  int cp[NP];
+  auto load_dA = [&](int cb) {
 #pragma unroll
-  for (int q = 0; q < 16; ++q)
-    dA[q] = *reinterpret_cast<const float2*>(A0_adj + (static_cast<size_t>(i) * 16 + q) * C + kc);
-  for (int eb = e0; eb < e1; eb += kEdgeChunk) {
-    const int ne = min(kEdgeChunk, e1 - eb);
-    __syncthreads();
-    stage_l0<true>(m, in, ti, eb, ne, st);
-    __syncthreads();
-    const int na = st.nact;
-    float4 c[8];
-    auto fetch = [&](int a) {
-      const float4* p = m.spl0 + static_cast<size_t>(st.row[st.act[a]]) * 4 * C + cp;
+    for (int p = 0; p < NP; ++p) {
+      const int c = cb + 32 * p + lane;
+      cp[p] = c < C2 ? c : 0;
+      const float2* a = reinterpret_cast<const float2*>(A0_adj + static_cast<size_t>(i) * 16 * C) + cp[p];
 #pragma unroll
-      for (int q = 0; q < 8; ++q) c[q] = __ldg(p + q * C2);
-    };
-    if (na > 0) fetch(0);
-    for (int a = 0; a < na; ++a) {
-      const int t = st.act[a];
-      const float2 x2 = make_float2(st.x[t], st.x[t]);
-      float2 R[4], Rd[4];
-#pragma unroll
-      for (int l = 0; l < 4; ++l) spline2(c[2 * l], c[2 * l + 1], x2, R[l], Rd[l]);
-      if (a + 1 < na) fetch(a + 1);
-      float2 dr = make_float2(0.0f, 0.0f);
-      float fx = 0.0f, fy = 0.0f, fz = 0.0f;
-#pragma unroll
-      for (int l = 0; l < 4; ++l) {
-        float2 dRl = make_float2(0.0f, 0.0f);
-#pragma unroll
-        for (int q = l * l; q < (l + 1) * (l + 1); ++q) {
-          if (q == 0) {  // Y_00 = 1 with a zero gradient (sph_harm16): the R_0' term alone
-            dRl = dA[0];
-            continue;
-          }
-          const float4 g = st.G[t][q];  // (dY/dx, dY/dy, dY/dz, Y)
-          dRl = fma2(dA[q], make_float2(g.w, g.w), dRl);
-          const float2 w = mul2(dA[q], R[l]);
-          const float s = w.x + w.y;
-          fx = fmaf(s, g.x, fx);
-          fy = fmaf(s, g.y, fy);
-          fz = fmaf(s, g.z, fz);
-        }
-        dr = fma2(dRl, Rd[l], dr);
-      }
-      const float d = dr.x + dr.y;
-      const float4 u = st.u[t];
-      fx = fmaf(d, u.x, fx);
-      fy = fmaf(d, u.y, fy);
-      fz = fmaf(d, u.z, fz);
-      if (!live) fx = fy = fz = 0.0f;
-      block_reduce3(fx, fy, fz, sF, t);
+      for (int q = 0; q < 16; ++q) dA[p][q] = c < C2 ? __ldg(a + q * C2) : make_float2(0.0f, 0.0f);
     }
-    __syncthreads();
-    for (int t = threadIdx.x; t < ne; t += blockDim.x) {
-      const long e = static_cast<long>(eb) + t;
-      double s[3] = {0.0, 0.0, 0.0};
-      if (st.row[t] >= 0)
-        for (int w = 0; w < nwarp; ++w)
-          for (int a = 0; a < 3; ++a) s[a] += static_cast<double>(sF[t][w][a]);
+  };
+  load_dA(0);
+  for (int eb = e0 + part * cs; eb < e1; eb += split * cs) {
+    const int ne = min(cs, e1 - eb);
+    const long e = static_cast<long>(eb) + lane;
+    if (eb > e0 + part * cs) ed.load(m, in, min(eb + lane, e1 - 1));
+    const bool active = lane < ne && ed.r < m.r_cut;
+    int na;
+    const int pos = stage_rows0(m, s.st, ed, ti, active, na);
+    bool staged = false;
+    for (int cb = 0; cb < C2 && na > 0; cb += 32 * NP) {
+      if (C2 > 32 * NP) load_dA(cb);
+      float4 c[NP][8];
+      {
+        const float4* r = m.spl0 + static_cast<size_t>(s.st.meta[0].y) * 4 * C;
+#pragma unroll
+        for (int p = 0; p < NP; ++p)
+#pragma unroll
+          for (int q = 0; q < 8; ++q) c[p][q] = __ldg(r + q * C2 + cp[p]);
+      }
+      if (!staged) stage_Y0(s.st, ed, active, pos);
+      staged = true;
+      for (int a = 0; a < na; ++a) {
+        const float4* r = m.spl0 + static_cast<size_t>(s.st.meta[min(a + 1, na - 1)].y) * 4 * C;
+        const float x = __int_as_float(s.st.meta[a].x);
+        const float2 x2 = make_float2(x, x);
+        float2 y[16], dY[16], dr = make_float2(0.0f, 0.0f);
+        read_Y2(s.st.Y2[a], y);
+        static_for<4>([&](auto lc) {
+          constexpr int l = decltype(lc)::value;
+#pragma unroll
+          for (int p = 0; p < NP; ++p) {
+            float2 R, Rd;
+            spline2(c[p][2 * l], c[p][2 * l + 1], x2, R, Rd);
+            c[p][2 * l] = __ldg(r + 2 * l * C2 + cp[p]);
+            c[p][2 * l + 1] = __ldg(r + (2 * l + 1) * C2 + cp[p]);
+            float2 dR;
+            if constexpr (l == 0) {  // Y_00 = 1 with a zero gradient (sph_harm16): the R_0' term alone
+              dR = dA[p][0];
+            } else {
+#pragma unroll
+              for (int q = l * l; q < (l + 1) * (l + 1); ++q) {
+                dR = q == l * l ? mul2(dA[p][q], y[q]) : fma2(dA[p][q], y[q], dR);
+                dY[q] = p == 0 ? mul2(dA[p][q], R) : fma2(dA[p][q], R, dY[q]);
+              }
+            }
+            dr = l == 0 && p == 0 ? mul2(dR, Rd) : fma2(dR, Rd, dr);
+          }
+        });
+        float2* t = s.buf + (a % kSumEdges) * 8 * kSumRow + lane;
+        t[0] = make_float2(dr.x + dr.y, dY[1].x + dY[1].y);
+#pragma unroll
+        for (int v = 1; v < 8; ++v)
+          t[kSumRow * v] = make_float2(dY[2 * v].x + dY[2 * v].y, dY[2 * v + 1].x + dY[2 * v + 1].y);
+        if (a % kSumEdges == kSumEdges - 1 || a == na - 1) {
+          float* out = &s.S[a - a % kSumEdges][0];
+          if (cb == 0)
+            sum_lanes<false>(s.buf, out, a % kSumEdges + 1);
+          else
+            sum_lanes<true>(s.buf, out, a % kSumEdges + 1);
+        }
+      }
+    }
+    if (lane < ne) {  // this lane's edge
+      double f[3] = {0.0, 0.0, 0.0};
+      if (active) {
+        float Y[16], D[48];
+        sph_harm16<true>(ed.vx, ed.vy, ed.vz, Y, D);
+        const float* S = s.S[pos];
+        const float d = __fdiv_rn(S[0], ed.r);
+        float fx = __fmul_rn(d, ed.vx), fy = __fmul_rn(d, ed.vy), fz = __fmul_rn(d, ed.vz);
+#pragma unroll
+        for (int q = 1; q < 16; ++q) {
+          fx = fmaf(S[q], D[q], fx);
+          fy = fmaf(S[q], D[16 + q], fy);
+          fz = fmaf(S[q], D[32 + q], fz);
+        }
+        f[0] = fx;
+        f[1] = fy;
+        f[2] = fz;
+      }
       if (m.has_zbl && local) {  // node_forces -= xyz / r * dV_ZBL/dr (zbl.cpp:118-121)
         float V, dV;
         const double r = in.r[e];
-        zbl_edge(m, m.zbl_pair[ti * m.S + in.ntype_e[e]], static_cast<float>(r), V, dV);
-        for (int a = 0; a < 3; ++a) s[a] += in.xyz[3 * e + a] / r * static_cast<double>(dV);
+        zbl_edge(m, m.zbl_pair[ti * m.S + ed.tj], static_cast<float>(r), V, dV);
+        for (int a = 0; a < 3; ++a) f[a] = fma(in.xyz[3 * e + a] / r, static_cast<double>(dV), f[a]);
       }
-      if (m.dens_spl[0]) {  // dE/dx through the layer-0 density factor (mace.cpp:334-339)
+      for (int layer = 0; layer < 2; ++layer) {  // through the density factors (mace.cpp:334-339, :744-749)
+        if (!m.dens_spl[layer] || (layer == 1 && !local)) continue;
         float v, d;
         const double r = in.r[e];
-        dens_eval(m, 0, ti, in.ntype_e[e], static_cast<float>(r), v, d);
-        const double g = static_cast<double>(m.dens_c[0][i]) * static_cast<double>(d) / r;
-        for (int a = 0; a < 3; ++a) s[a] -= g * in.xyz[3 * e + a];
-      }
-      if (m.dens_spl[1] && local) {  // and through the layer-1 one (mace.cpp:744-749)
-        float v, d;
-        const double r = in.r[e];
-        dens_eval(m, 1, ti, in.ntype_e[e], static_cast<float>(r), v, d);
-        const double g = static_cast<double>(m.dens_c[1][i]) * static_cast<double>(d) / r;
-        for (int a = 0; a < 3; ++a) s[a] -= g * in.xyz[3 * e + a];
+        dens_eval(m, layer, ti, ed.tj, static_cast<float>(r), v, d);
+        const double g = static_cast<double>(m.dens_c[layer][i]) * static_cast<double>(d) / r;
+        for (int a = 0; a < 3; ++a) f[a] = fma(-g, in.xyz[3 * e + a], f[a]);
       }
       for (int a = 0; a < 3; ++a) {
-        double f = 0.0;
-        if (local) {
-          for (int h = 0; h < C >> 5; ++h) f += static_cast<double>(f1[h * m.f1_stride + 3 * e + a]);  // channel slices
-        }
-        forces[3 * e + a] = -(s[a] + f);
+        double w = 0.0;
+        if (local)
+          for (int h = 0; h < C >> 5; ++h) w += static_cast<double>(f1[h * m.f1_stride + 3 * e + a]);  // channel slices
+        forces[3 * e + a] = -(f[a] + w);
       }
     }
   }
 }
 
-template <bool P>
-__global__ void __launch_bounds__(128) k_layer0_rev(DevModel m, EdgeIn in, const float* __restrict__ A0_adj,
-                                                    const float* __restrict__ f1, double* __restrict__ forces) {
+template <int CT, bool P>
+__global__ void __launch_bounds__(32, 12) k_layer0_rev(DevModel m, EdgeIn in, const float* __restrict__ A0_adj,
+                                                       const float* __restrict__ f1, double* __restrict__ forces,
+                                                       int split, int cs) {
   pdl_begin();
-  AtomCursor cur{P ? m.sched : nullptr, in.N, 0};
-  for (int b = cur.first(); b < in.N; b = cur.next())
-    layer0_rev_atom(m, in, A0_adj, f1, forces, in.atom_at(b));
+  __shared__ Rev0Smem s;
+  const int n = in.N * split;
+  AtomCursor cur{P ? m.sched : nullptr, n, 0};
+  for (int b = cur.first(); b < n; b = cur.next())
+    layer0_rev_item<CT>(m, in, A0_adj, f1, forces, s, in.atom_at(b / split), b % split, split, cs);
   cur.done();
 }
 
 // ---------------------------------------------------------------------------
 // launchers
 // ---------------------------------------------------------------------------
-// Dynamic shared memory above 48 KB must be opted into once per kernel (outside
-// any stream capture).
-cudaError_t init_edge_kernels(const DevModel& m) { return init_layer1_kernels(m); }
+namespace {
 
-// layer-0 edge kernels: one thread per channel pair, whole warps
-int layer0_block(int C) { return ((C >> 1) + 31) & ~31; }
+// warps of the contraction adjoint's block
+int contract0_warps(const DevModel& m, bool split) { return (split ? m.nLM : 1) * layer0_slices(m.C); }
+// A warp per output while the (node, 64 channels) warps are fewer than this (us, one : a warp
+// per output: 300 nodes of L_max = 2 and 128 channels 77 : 21, 999 of 64 channels 34 : 16,
+// 2197 of L_max = 2 and 128 channels 65 : 103, 4096 of 128 channels 71 : 76)
+constexpr long kContractWarps = 3000;
+bool contract0_split(const DevModel& m, long n) { return n * layer0_slices(m.C) < kContractWarps; }
 
-// the canonical polynomial outputs compiled into the layer-0 kernels: 9 (L_max = 2) or 4
-// (L_max = 1, and every model on the data-driven polynomial path)
+// f(outputs, C): the kernels with generated polynomials, 9 (L_max = 2) or 4 (L_max = 1) outputs
+// and the channel counts compiled in (0: any)
 template <typename F>
-void dispatch_nlm(const DevModel& m, F&& f) {
-  if (m.poly_canon && m.nLM == 9)
-    f(std::integral_constant<int, 9>{});
-  else
-    f(std::integral_constant<int, 4>{});
+void dispatch_poly(const DevModel& m, F&& f) {
+  if (m.nLM == 9) {
+    constexpr std::integral_constant<int, 9> n{};
+    m.C == 128 ? f(n, std::integral_constant<int, 128>{}) : f(n, std::integral_constant<int, 0>{});
+    return;
+  }
+  constexpr std::integral_constant<int, 4> n{};
+  switch (m.C) {
+    case 64: f(n, std::integral_constant<int, 64>{}); break;
+    case 128: f(n, std::integral_constant<int, 128>{}); break;
+    default: f(n, std::integral_constant<int, 0>{}); break;
+  }
+}
+template <typename F>
+void dispatch_c0(int C, F&& f) {
+  switch (C) {
+    case 32: f(std::integral_constant<int, 32>{}); break;
+    case 64: f(std::integral_constant<int, 64>{}); break;
+    case 128: f(std::integral_constant<int, 128>{}); break;
+    default: f(std::integral_constant<int, 0>{}); break;
+  }
+}
+
+size_t fwd0_smem(const DevModel& m) { return m.poly_canon ? 0 : 17 * 32 * sizeof(float2); }
+size_t contract0_smem(const DevModel& m, bool split) {
+  return contract0_warps(m, split) * ((split ? 16 : 0) + (m.poly_canon ? 0 : 2 * 17)) * 32 * sizeof(float2);
+}
+
+}  // namespace
+
+// Dynamic shared memory above 48 KB must be opted into once per kernel (outside any stream
+// capture).
+cudaError_t init_edge_kernels(const DevModel& m) {
+  cudaError_t e = init_layer1_kernels(m);
+  dispatch_poly(m, [&](auto nc, auto cc) {
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(k_contract0_rev<decltype(nc)::value, decltype(cc)::value, true>,
+                               cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(contract0_smem(m, true)));
+  });
+  return e;
 }
 
 void launch_layer0_fwd(const DevModel& m, const EdgeIn& in, float* A0, float* M0, float* zbl_e, cudaStream_t s) {
   if (in.N <= 0) return;
-  const size_t smem = 17 * sizeof(float) * m.C;
-  DevModel mk;
-  const int grid = atom_grid(m, kAkLayer0Fwd, in.N, mk);
-  dispatch_nlm(m, [&](auto nc) {
-    constexpr int NLM = decltype(nc)::value;
-    if (mk.sched)
-      launch_pdl(k_layer0_fwd<true, NLM>, grid, 2 * layer0_block(m.C), smem, s, mk, in, A0, M0, zbl_e);
-    else
-      launch_pdl(k_layer0_fwd<false, NLM>, grid, 2 * layer0_block(m.C), smem, s, mk, in, A0, M0, zbl_e);
+  dispatch_poly(m, [&](auto nc, auto cc) {
+    launch_pdl(k_layer0_fwd<decltype(nc)::value, decltype(cc)::value>, in.N * layer0_slices(m.C), 32, fwd0_smem(m), s, m,
+               in, A0, M0, zbl_e);
   });
 }
 
 void launch_layer0_rev(const DevModel& m, const EdgeIn& in, const float* A0, const float* M0_adj, const float* f1,
                        float* A0_adj, double* forces, cudaStream_t s) {
   if (in.N <= 0) return;
-  DevModel mk;
-  int grid = atom_grid(m, kAkContract0Rev, in.N, mk);
-  const size_t smem = m.poly_canon ? 0 : 34 * sizeof(float) * m.C;
-  dispatch_nlm(m, [&](auto nc) {
-    constexpr int NLM = decltype(nc)::value;
-    if (mk.sched)
-      launch_pdl(k_contract0_rev<true, NLM>, grid, m.C, smem, s, mk, in.node_type, A0, M0_adj, A0_adj, in.N);
-    else
-      launch_pdl(k_contract0_rev<false, NLM>, grid, m.C, smem, s, mk, in.node_type, A0, M0_adj, A0_adj, in.N);
+  const bool by_lm = contract0_split(m, in.N);
+  dispatch_poly(m, [&](auto nc, auto cc) {
+    auto go = [&](auto sc) {
+      launch_pdl(k_contract0_rev<decltype(nc)::value, decltype(cc)::value, decltype(sc)::value>, in.N,
+                 32 * contract0_warps(m, by_lm), contract0_smem(m, by_lm), s, m, in.node_type, in.order, A0, M0_adj, A0_adj);
+    };
+    by_lm ? go(std::true_type{}) : go(std::false_type{});
   });
-  grid = atom_grid(m, kAkLayer0Rev, in.N, mk);
-  if (mk.sched)
-    launch_pdl(k_layer0_rev<true>, grid, layer0_block(m.C), 0, s, mk, in, A0_adj, f1, forces);
-  else
-    launch_pdl(k_layer0_rev<false>, grid, layer0_block(m.C), 0, s, mk, in, A0_adj, f1, forces);
+  const int split = edge_split(in.N), cs = edge_chunk(split);
+  DevModel mk;
+  const int grid = atom_grid(m, kAkLayer0Rev, in.N * split, mk);
+  dispatch_c0(m.C, [&](auto cc) {
+    constexpr int CT = decltype(cc)::value;
+    if (mk.sched)
+      launch_pdl(k_layer0_rev<CT, true>, grid, 32, 0, s, mk, in, A0_adj, f1, forces, split, cs);
+    else
+      launch_pdl(k_layer0_rev<CT, false>, grid, 32, 0, s, mk, in, A0_adj, f1, forces, split, cs);
+  });
 }
 
-// resident blocks per SM of the persistent layer-0 kernels at this model's launch shapes
+// resident blocks per SM of the layer-0 kernels at this model's launch shapes
 void layer0_residency(const DevModel& m, int* per_sm) {
-  dispatch_nlm(m, [&](auto nc) {
-    constexpr int NLM = decltype(nc)::value;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm[kAkLayer0Fwd], k_layer0_fwd<true, NLM>,
-                                                  2 * layer0_block(m.C), 17 * sizeof(float) * m.C);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm[kAkContract0Rev], k_contract0_rev<true, NLM>, m.C,
-                                                  m.poly_canon ? 0 : 34 * sizeof(float) * m.C);
+  dispatch_poly(m, [&](auto nc, auto cc) {
+    constexpr int NLM = decltype(nc)::value, CT = decltype(cc)::value;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm[kAkLayer0Fwd], k_layer0_fwd<NLM, CT>, 32, fwd0_smem(m));
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm[kAkContract0Rev], k_contract0_rev<NLM, CT, false>,
+                                                  32 * contract0_warps(m, false), contract0_smem(m, false));
   });
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm[kAkLayer0Rev], k_layer0_rev<true>, layer0_block(m.C), 0);
+  dispatch_c0(m.C, [&](auto cc) {
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm[kAkLayer0Rev], k_layer0_rev<decltype(cc)::value, true>, 32, 0);
+  });
 }
 
 }  // namespace smx

@@ -77,9 +77,6 @@ __host__ __device__ constexpr bool row_started(int i, int b) {
   return false;
 }
 
-constexpr int kSumEdges = 4;  // edges summed over the lanes at a time
-constexpr int kSumRow = 33;   // row pitch of their terms: 32 rows read at one column hit all banks
-
 // shared memory of one warp
 struct RevSmem {
   EdgeStage st;   // Y rows: once an edge is done, (dE/dr term, dE/dY_1 .. dE/dY_15) in their place
@@ -137,26 +134,6 @@ __device__ __forceinline__ void rev_edge(const float* g, float4* c, const float4
   t[0] = make_float2(dr, dY[1]);
 #pragma unroll
   for (int v = 1; v < 8; ++v) t[kSumRow * v] = make_float2(dY[2 * v], dY[2 * v + 1]);
-}
-
-// The sums over the lanes of edges [a0, a0 + n) (n <= kSumEdges) into their Y rows: lane
-// 8 e + v adds component pair v of edge e, four partial sums in a fixed order.
-__device__ __forceinline__ void rev_sums(RevSmem& s, int a0, int n) {
-  const int lane = threadIdx.x & 31, e = lane >> 3, v = lane & 7;
-  __syncwarp();
-  if (e < n) {
-    const float2* row = s.buf + lane * kSumRow;
-    float2 p0 = make_float2(0.0f, 0.0f), p1 = p0, p2 = p0, p3 = p0;
-#pragma unroll
-    for (int i = 0; i < 32; i += 4) {
-      p0 = __fadd2_rn(p0, row[i]);
-      p1 = __fadd2_rn(p1, row[i + 1]);
-      p2 = __fadd2_rn(p2, row[i + 2]);
-      p3 = __fadd2_rn(p3, row[i + 3]);
-    }
-    *reinterpret_cast<float2*>(&s.st.Y[a0 + e][2 * v]) = __fadd2_rn(__fadd2_rn(p0, p1), __fadd2_rn(p2, p3));
-  }
-  __syncwarp();
 }
 
 // Group G over the edges of chunks `split` apart; the edge forces of the earlier groups
@@ -252,7 +229,7 @@ __device__ __forceinline__ void rev_group(const DevModel& m, const EdgeIn& in, c
         if constexpr (NR % 2) add_fixed(dst + (NR - 1) * C, hadj[NR - 1]);
         mt = mn;
         if (a % kSumEdges == kSumEdges - 1 || a == na - 1)
-          rev_sums(s, a - a % kSumEdges, a % kSumEdges + 1);
+          sum_lanes<false>(s.buf, &s.st.Y[a - a % kSumEdges][0], a % kSumEdges + 1);
       }
     }
     if (lane < ne) {  // this lane's edge: the sums against u and dY/dx
@@ -261,10 +238,10 @@ __device__ __forceinline__ void rev_group(const DevModel& m, const EdgeIn& in, c
         float Y[16], D[48];
         sph_harm16<true>(ed.vx, ed.vy, ed.vz, Y, D);
         const float* S = s.st.Y[pos];
-        const float d = S[0] / ed.r;
-        fx = d * ed.vx;
-        fy = d * ed.vy;
-        fz = d * ed.vz;
+        const float d = __fdiv_rn(S[0], ed.r);
+        fx = __fmul_rn(d, ed.vx);
+        fy = __fmul_rn(d, ed.vy);
+        fz = __fmul_rn(d, ed.vz);
 #pragma unroll
         for (int q = 1; q < 16; ++q) {
           fx = fmaf(S[q], D[q], fx);
@@ -316,12 +293,6 @@ __global__ void __launch_bounds__(32, 12) k_layer1_rev(DevModel m, EdgeIn in, co
 
 namespace {
 
-// Warps the chip holds at once (12 per SM).  A node's edges are split over `split` warps
-// while all parts still fit at once, each part paying the g prologue again, and over two
-// when the items would run as one full and one nearly empty wave (us, whole : split:
-// 64 items 24.6 : 12.3 (16 parts), 1000 items 55.3 : 59.4 (3), 1998 items 105.5 : 98.3 (2)).
-constexpr long kSlots = 12 * 152;
-
 size_t rev_smem(const DevModel& m) {
   const size_t rows = m.cg_val ? 0 : m.n_lme + m.n_p;
   return offsetof(RevSmem, buf) + std::max<size_t>(sizeof(float2) * kSumEdges * 8 * kSumRow, sizeof(float) * 32 * rows);
@@ -333,9 +304,9 @@ void launch_layer1_rev(const DevModel& m, const EdgeIn& in, const float* H1, con
                        float* f1, cudaStream_t s) {
   if (in.N <= 0) return;
   const long items = static_cast<long>(in.N) * (m.C >> 5);
-  const int split =
-      items > 2 * kSlots ? 1 : (items > kSlots ? 2 : static_cast<int>(std::min<long>(16, kSlots / items)));
-  const int cs = split == 1 ? kEdgeChunk : (split <= 2 ? 16 : (split <= 8 ? 8 : 4));
+  // parts pay the g prologue again (us, whole : split: 64 items 24.6 : 12.3 (16 parts), 1000
+  // items 55.3 : 59.4 (3), 1998 items, one full wave and a nearly empty one, 105.5 : 98.3 (2))
+  const int split = edge_split(items), cs = edge_chunk(split);
   DevModel mk;
   const int grid = atom_grid(m, kAkLayer1Rev, static_cast<int>(items * split), mk);
   dispatch_layer1(m, [&](auto lc, auto cc, auto nc) {

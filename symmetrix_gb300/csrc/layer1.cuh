@@ -3,7 +3,7 @@
 #pragma once
 
 #include "cg_canon.h"
-#include "device.cuh"
+#include "edge.cuh"
 
 namespace smx {
 
@@ -92,22 +92,6 @@ __device__ __forceinline__ void for_paths(F&& f) {
 struct EdgeStage {
   float Y[kEdgeChunk][16];  // Y_lm
   int4 meta[kEdgeChunk];    // offset inside the spline interval (float bits), spline row, neighbour
-};
-
-// This lane's edge of a chunk, loaded ahead of its staging.
-struct LaneEdge {
-  float vx, vy, vz, r, x;  // x: offset inside spline interval iv
-  int tj, j, iv;
-  __device__ __forceinline__ void load(const DevModel& m, const EdgeIn& in, long e) {
-    vx = static_cast<float>(in.xyz[3 * e]);
-    vy = static_cast<float>(in.xyz[3 * e + 1]);
-    vz = static_cast<float>(in.xyz[3 * e + 2]);
-    const double rd = in.r[e];
-    r = static_cast<float>(rd);
-    iv = spline_at(m, rd, x);
-    tj = in.ntype_e[e];
-    j = in.nidx[e];
-  }
 };
 
 // Stage the warp's edges (lanes with `active`): first where their spline rows and neighbours

@@ -1,8 +1,9 @@
-"""The layer-1 forward and adjoint (k_layer1.cu, k_layer1_rev.cu): edge counts around the
-adjoint's sum batches (4 edges) and the staging chunks (4 to 32 edges), nodes of one and of
-several warps, every instruction group, and the Clebsch-Gordan tables: the canonical zero
-pattern, its general form and a table outside the pattern; the pattern's generated source
-and the fixed-point conversion of the H1_adj terms (CPU)."""
+"""The edge kernels of both layers (k_edge.cu, k_layer1.cu, k_layer1_rev.cu): edge counts around
+the adjoints' sum batches (4 edges) and the staging chunks (4 to 32 edges), nodes of one and
+of several warps, channel counts that leave lanes idle or need several channel blocks, every
+instruction group, the Clebsch-Gordan tables (the canonical zero pattern, its general form, a
+table outside the pattern) and contraction polynomials outside the canonical set; the
+pattern's generated source and the fixed-point conversion of the H1_adj terms (CPU)."""
 import importlib.util
 import os
 import sys
@@ -30,7 +31,8 @@ def clusters(sizes, seed, S):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("C,L_max,table", [(32, 1, "canonical"), (96, 1, "rows"), (128, 1, "canonical"),
-                                           (64, 2, "canonical"), (32, 2, "rows"), (64, 1, "other"), (96, 2, "other")])
+                                           (64, 2, "canonical"), (32, 2, "rows"), (64, 1, "other"), (96, 2, "other"),
+                                           (192, 1, "canonical"), (32, 1, "poly"), (64, 2, "poly")])
 def test_edge_counts_and_splits(engine_lib, tmp_path, C, L_max, table):
     from oracle.pyoracle import Evaluator
     from symmetrix_gb300 import MACE
@@ -43,6 +45,11 @@ def test_edge_counts_and_splits(engine_lib, tmp_path, C, L_max, table):
         model["Phi1_lme"].append(0)
         model["Phi1_lelm1lm2"].append(unused)
         model["Phi1_clebsch_gordan"].append(0.3)
+    if table == "poly":  # one monomial more than the canonical set of output 0
+        model["M0_monomials"]["0"].append([0, 1])
+        for w in model["M0_weights"].values():
+            for k in w["0"]:
+                w["0"][k].append(0.1)
     path = write_model(model, str(tmp_path / "m.json"))
     pos, species = clusters([1, 2, 4, 5, 6, 9, 10, 17, 18, 33, 34], 3, 3)
     nl = neighbor_list(pos, 5.0)
@@ -50,19 +57,20 @@ def test_edge_counts_and_splits(engine_lib, tmp_path, C, L_max, table):
     m = MACE(path)
     m.set_option("cg_padded", 0 if table == "rows" else 1)
     m.compute_node_energies_forces(*a)
-    e, f, h, phi = m.node_energies, m.node_forces, m.H1_adj, m.Phi1
+    stages = ("A0", "M0", "Phi1", "H1_adj", "A0_adj")
     ref = Evaluator(path, "port")
     ref.compute_node_energies_forces(*a)
     # float32 sums of a few hundred terms against float64: 1e-5 of the largest component
-    for got, want in ((e, ref.node_energies), (f, ref.node_forces), (h, ref.get("H1_adj")), (phi, ref.get("Phi1"))):
+    for got, want in [(m.node_energies, ref.node_energies), (m.node_forces, ref.node_forces)] + [
+            (m.stage(s), ref.get(s)) for s in stages]:
         assert np.abs(got - want).max() <= 1e-5 * max(1.0, np.abs(want).max())
     # many copies: the edges of a node stay with one warp
     n, E = len(species), len(nl["r"])
-    copies = 1 + 2 * 12 * 152 // (n * C // 32)
+    copies = 1 + 4 * 12 * 152 // (n * max(C // 64, 1))
     rep = np.tile(nl["neigh_indices"], copies) + np.repeat(np.arange(copies) * n, E)
     m.compute_node_energies_forces(n * copies, np.tile(species, copies), np.tile(nl["num_neigh"], copies), rep,
                                    np.tile(a[4], copies), np.tile(nl["xyz"], (copies, 1)), np.tile(nl["r"], copies))
-    for got, want in ((m.node_forces, ref.node_forces), (m.Phi1, ref.get("Phi1")), (m.H1_adj, ref.get("H1_adj"))):
+    for got, want in [(m.node_forces, ref.node_forces)] + [(m.stage(s), ref.get(s)) for s in stages]:
         assert np.abs(got.reshape(copies, -1) - want).max() <= 1e-5 * max(1.0, np.abs(want).max())
 
 
