@@ -224,6 +224,27 @@ __global__ void k_reverse_edges(int N, const int* __restrict__ first, const int*
   }
 }
 
+// rev[e] for lists in ascending neighbour order without images (non-periodic): a binary search
+// of i in j's list, one thread per edge (1.04 M edges of molecules: 78 us by scanning -> 13 us).
+__global__ void k_reverse_edges_sorted(long cap, int N, const int* __restrict__ first, const int* __restrict__ nidx,
+                                       const int* __restrict__ edge_i, int* __restrict__ rev) {
+  const long E = first[N];
+  for (long e = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x; e < E && e < cap;
+       e += static_cast<long>(gridDim.x) * blockDim.x) {
+    const int i = edge_i[e], j = nidx[e];
+    int lo = first[j], hi = first[j + 1];
+    const int end = hi;
+    while (lo < hi) {  // first entry of j's list that is not below i
+      const int mid = (lo + hi) >> 1;
+      if (nidx[mid] < i)
+        lo = mid + 1;
+      else
+        hi = mid;
+    }
+    rev[e] = lo < end && nidx[lo] == i ? lo : -1;
+  }
+}
+
 // rev[e] for a cell-list build: the reverse of e = (i -> j, shift) lies in j's segment for
 // the neighbour cell at the negated cell offset (cellseg), a few entries, scanned in order
 // (the first match, as k_reverse_edges finds).  One thread per edge.
@@ -257,6 +278,14 @@ __global__ void k_reverse_edges_cells(long cap, int N, const int* __restrict__ f
   }
 }
 
+// sqrt(r2) to ~1e-15: the float32 root and one Newton step on the float64 r2, without the
+// float64 root (its arithmetic runs on this part's slow pipe)
+__device__ __forceinline__ double length_of(double r2) {
+  const float rf = sqrtf(static_cast<float>(r2));
+  const double rd = rf;
+  return rf > 0.0f ? rd + static_cast<double>(__fdividef(static_cast<float>(fma(-rd, rd, r2)), rf + rf)) : 0.0;
+}
+
 // xyz_e = x_j + shift_e * box - x_i, r_e = |xyz_e|
 __global__ void k_edge_geometry(long cap, int N, const int* __restrict__ first, const double* __restrict__ pos,
                                 double3 box, const int* __restrict__ nidx, const int* __restrict__ edge_i,
@@ -273,7 +302,7 @@ __global__ void k_edge_geometry(long cap, int N, const int* __restrict__ first, 
   xyz[3 * e] = dx;
   xyz[3 * e + 1] = dy;
   xyz[3 * e + 2] = dz;
-  r[e] = sqrt(dx * dx + dy * dy + dz * dz);
+  r[e] = length_of(fma(dx, dx, fma(dy, dy, dz * dz)));
 }
 
 // velocity Verlet units: positions A, velocities A/fs, forces eV/A, masses amu, dt fs
@@ -309,13 +338,8 @@ __global__ void k_edge_geometry_packed(int N, const int* __restrict__ first, con
       dx = pos[3 * j] + sh.x * box.x - px;
       dy = pos[3 * j + 1] + sh.y * box.y - py;
       dz = pos[3 * j + 2] + sh.z * box.z - pz;
-      // the float32 root and one Newton step on the float64 r^2: the float64 length to
-      // ~1e-15, without the float64 root (its arithmetic runs on this part's slow pipe)
-      const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
-      const float rf = sqrtf(static_cast<float>(r2));
-      const double rd = rf;
-      re = rf > 0.0f ? rd + static_cast<double>(__fdividef(static_cast<float>(fma(-rd, rd, r2)), rf + rf)) : 0.0;
-      active = rf < r_cut_f;
+      re = length_of(fma(dx, dx, fma(dy, dy, dz * dz)));
+      active = static_cast<float>(re) < r_cut_f;  // as the evaluator compares
     }
     const unsigned ball = __ballot_sync(0xffffffffu, active);
     const int q = e0 + count + __popc(ball & ((1u << lane) - 1u));
@@ -424,12 +448,17 @@ __global__ void k_reduce_partials(int N, const int* __restrict__ first, const do
   if (threadIdx.x < 10) partial[blockIdx.x * 10 + threadIdx.x] = sh[threadIdx.x][0];
 }
 
-__global__ void k_reduce_final(int nblocks, const double* __restrict__ partial, double* __restrict__ out) {
-  if (threadIdx.x < 10) {
-    CompSum s;
-    for (int b = 0; b < nblocks; ++b) s.add(partial[b * 10 + threadIdx.x]);
-    out[threadIdx.x] = s.value();
-  }
+// one warp per quantity: compensated sums of every 32nd block, then a pairwise tree in a fixed
+// order (one thread per quantity over 64 blocks took 20 us, a chain of float64 sums)
+__global__ void __launch_bounds__(320) k_reduce_final(int nblocks, const double* __restrict__ partial,
+                                                      double* __restrict__ out) {
+  const int q = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  CompSum s;
+  for (int b = lane; b < nblocks; b += 32) s.add(partial[b * 10 + q]);
+  double v = s.value();
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+  if (lane == 0) out[q] = v;
 }
 
 // velocity Verlet halves
@@ -533,6 +562,13 @@ void launch_reverse_edges(long cap, int N, const int* first, const int* nidx, co
   if (cap > 0 && N > 0) k_reverse_edges<<<N, 128, 0, s>>>(N, first, nidx, shift, rev);  // block per atom
 }
 
+void launch_reverse_edges_sorted(long cap, int N, const int* first, const int* nidx, const int* edge_i, int* rev,
+                                 cudaStream_t s) {
+  if (cap > 0 && N > 0)
+    k_reverse_edges_sorted<<<static_cast<int>(std::min<long>(ceil_div(cap, 256), 152L * 16)), 256, 0, s>>>(
+        cap, N, first, nidx, edge_i, rev);
+}
+
 void launch_reverse_edges_cells(long cap, int N, const int* first, const int* nidx, const int* edge_i,
                                 const char4* shift, const int* cell, int3 nc, const int* cellseg, int* rev,
                                 cudaStream_t s) {
@@ -575,7 +611,7 @@ void launch_atom_forces(int N, const int* first, const int* rev, const double* f
 void launch_reduce(int N, const int* first, const double* energies, const double* xyz, const double* f,
                    double* partial, int nblocks, double* out, cudaStream_t s) {
   k_reduce_partials<<<nblocks, 256, 0, s>>>(N, first, energies, xyz, f, partial);
-  k_reduce_final<<<1, 32, 0, s>>>(nblocks, partial, out);
+  k_reduce_final<<<1, 320, 0, s>>>(nblocks, partial, out);
 }
 
 void launch_vv_first(int N, double dt, const double* F, const double* inv_m, double* v, double* x, cudaStream_t s) {

