@@ -96,6 +96,7 @@ void smx_destroy(smx_engine* eng) {
   if (!eng) return;
   cudaSetDevice(eng->device);
   if (eng->stream) cudaStreamSynchronize(eng->stream);
+  eng->atoms_ws.reset();
   eng->free_workspace();
   for (void* p : eng->model_mem) cudaFree(p);
   if (eng->stream) cudaStreamDestroy(eng->stream);

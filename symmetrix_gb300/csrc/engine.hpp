@@ -7,6 +7,7 @@
 #include <algorithm>
 #include <cstdint>
 #include <cstring>
+#include <memory>
 #include <stdexcept>
 #include <string>
 #include <vector>
@@ -99,6 +100,12 @@ struct smx_engine {
   long lastE = 0;                  // edges of the last host- or device-pointer call or stage call
   bool evaluated = false;          // the workspace holds the stages of an evaluation
   bool M0_kept = false, Phi1_kept = false, A1adj_kept = false;  // float32 rows written by it
+
+  // Buffers of the atom-level calls (neighbour list, atom arrays; md.cu), kept between calls
+  // like the workspace above: a call allocated and freed some thirty of them, 0.3 ms of a
+  // 0.5 ms evaluation of 500 atoms.  Given back with the engine, or after a call that leaves
+  // more than AtomsWorkspace::kKeepBytes in them.
+  std::shared_ptr<void> atoms_ws;
 
   // B operand of a tensor-core GEMM from a row-major float [nrows][K] matrix: row n
   // holds (W_hi) for 1 split product, (W_hi | W_lo) for 2 or 3, W_lo = bf16(W - W_hi)

@@ -200,6 +200,7 @@ struct smx_md {
   int3 periodic{};
   double dt = 0.5, skin = 1.0;
   int rebuild_every = 10;
+  bool single = false;  // one evaluation of the current list, no dynamics
   long step = 0;
   double *pos = nullptr, *vel = nullptr, *F = nullptr, *inv_m = nullptr, *energies = nullptr, *partial = nullptr,
          *reduced = nullptr;
@@ -220,7 +221,7 @@ struct smx_md {
   NeighList nl;
   cudaGraphExec_t graph = nullptr;
   int graph_steps = 0;
-  static constexpr int kReduceBlocks = 304;  // two per SM (64: 82 against 17 us for 200k edges)
+  static constexpr int kReduceBlocks = 304;  // two per SM (64: 82 against 42 us for 200k edges)
 
   ~smx_md() {
     if (graph) cudaGraphExecDestroy(graph);
@@ -250,7 +251,9 @@ struct smx_md {
                                      inv_m, vel, s);
       return;
     }
-    smx::launch_edge_geometry(nl.capE, N, nl.first, pos, box, nl.nidx, nl.edge_i, nl.shift, nl.xyz, nl.r, s);
+    // (a captured graph outlives its list: the capacity; a single evaluation: the edges)
+    smx::launch_edge_geometry(single ? nl.E : nl.capE, N, nl.first, pos, box, nl.nidx, nl.edge_i, nl.shift, nl.xyz, nl.r,
+                              s);
     eng->run(edges(), energies, nl.forces, s);
     smx::launch_atom_forces(N, nl.first, nl.rev, nl.forces, F, s);
     if (kick) smx::launch_vv_second(N, dt, F, inv_m, vel, s);
@@ -349,11 +352,50 @@ struct smx_md {
   }
 };
 
-extern "C" {
-
-}  // extern "C"
-
 namespace {
+
+// The buffers of compute_atoms_impl: an MD object without dynamics whose arrays grow and stay.
+struct AtomsWorkspace {
+  static constexpr long kKeepBytes = 1L << 30;
+  smx_md md;
+  int cap_atoms = 0, cap_mol = 0;
+  int *seg_of = nullptr, *seg_first = nullptr;  // lent to md by a call with molecules
+
+  ~AtomsWorkspace() {
+    md.seg_of = md.seg_first = nullptr;
+    if (seg_of) cudaFree(seg_of);
+    if (seg_first) cudaFree(seg_first);
+  }
+  void reserve(int n) {
+    if (n <= cap_atoms) return;
+    cap_atoms = 0;
+    for (double** p : {&md.pos, &md.F, &md.energies}) {
+      if (*p) cudaFree(*p);
+      *p = nullptr;
+    }
+    if (md.species) cudaFree(md.species);
+    if (seg_of) cudaFree(seg_of);
+    md.species = seg_of = nullptr;
+    md.pos = dalloc<double>(3L * n);
+    md.F = dalloc<double>(3L * n);
+    md.energies = dalloc<double>(n);
+    md.species = dalloc<int>(n);
+    seg_of = dalloc<int>(n);
+    if (!md.partial) md.partial = dalloc<double>(10 * smx_md::kReduceBlocks);
+    if (!md.reduced) md.reduced = dalloc<double>(10);
+    cap_atoms = n;
+  }
+  void reserve_molecules(int n_mol) {
+    if (n_mol <= cap_mol) return;
+    cap_mol = 0;
+    if (seg_first) cudaFree(seg_first);
+    seg_first = nullptr;
+    seg_first = dalloc<int>(n_mol + 1);
+    cap_mol = n_mol;
+  }
+  // about: per edge 8 indices, maps and types and 14 float64 values; per atom 12 float64 and the cells
+  long bytes() const { return md.nl.capE * 152 + static_cast<long>(md.nl.capN) * 256 + cap_atoms * 80L; }
+};
 
 int compute_atoms_impl(smx_engine* eng, int n_atoms, const double* positions, const int* species,
                        const double* box_lengths, int n_mol, const int* mol_first, double* energy,
@@ -363,38 +405,56 @@ int compute_atoms_impl(smx_engine* eng, int n_atoms, const double* positions, co
     return fail(SMX_ERR_INVALID, "bad atom arrays");
   for (int a = 0; a < n_atoms; ++a)
     if (species[a] < 0 || species[a] >= eng->hm.S) return fail(SMX_ERR_INVALID, "species out of range");
+  struct DropOnError {  // a call that fails leaves no half-grown workspace behind
+    smx_engine* eng;
+    bool done = false;
+    ~DropOnError() {
+      if (!done) eng->atoms_ws.reset();
+    }
+  } drop{eng};
   try {
     check(cudaSetDevice(eng->device), "cudaSetDevice");
     double3 box;
     int3 periodic;
     box_args(box_lengths, box, periodic);
-    smx_md md;  // borrowed as a workspace: no dynamics
-    md.eng = eng;
-    md.N = n_atoms;
-    md.box = box;
-    md.periodic = periodic;
-    md.skin = 0.0;
     cudaStream_t s = eng->stream;
     if (n_atoms == 0) {
       if (energy) *energy = 0.0;
       if (virial) std::memset(virial, 0, 9 * sizeof(double));
+      drop.done = true;
       return SMX_OK;
     }
-    md.pos = dalloc<double>(3 * n_atoms);
-    md.F = dalloc<double>(3 * n_atoms);
-    md.energies = dalloc<double>(n_atoms);
-    md.species = dalloc<int>(n_atoms);
-    md.partial = dalloc<double>(10 * smx_md::kReduceBlocks);
-    md.reduced = dalloc<double>(10);
+    if (!eng->atoms_ws) eng->atoms_ws = std::make_shared<AtomsWorkspace>();
+    AtomsWorkspace& ws = *static_cast<AtomsWorkspace*>(eng->atoms_ws.get());
+    smx_md& md = ws.md;
+    ws.reserve(n_atoms);
+    md.eng = eng;
+    md.device = eng->device;
+    md.N = n_atoms;
+    md.box = box;
+    md.periodic = periodic;
+    md.skin = 0.0;
+    md.single = true;
+    md.seg_of = md.seg_first = nullptr;
     check(cudaMemcpyAsync(md.pos, positions, sizeof(double) * 3 * n_atoms, cudaMemcpyHostToDevice, s), "H2D");
     check(cudaMemcpyAsync(md.species, species, sizeof(int) * n_atoms, cudaMemcpyHostToDevice, s), "H2D");
-    if (mol_first) md.set_molecules(n_mol, mol_first, s);
-    md.rebuild(s);
+    std::vector<int> of;
+    if (mol_first) {
+      of = molecule_of(n_mol, mol_first, n_atoms);
+      ws.reserve_molecules(n_mol);
+      md.seg_of = ws.seg_of;
+      md.seg_first = ws.seg_first;
+      check(cudaMemcpyAsync(md.seg_of, of.data(), sizeof(int) * n_atoms, cudaMemcpyHostToDevice, s), "H2D");
+      check(cudaMemcpyAsync(md.seg_first, mol_first, sizeof(int) * (n_mol + 1), cudaMemcpyHostToDevice, s), "H2D");
+    }
+    md.rebuild(s);  // (waits for the stream: `of` has been copied)
     md.forces(s);
-    smx::launch_reduce(n_atoms, md.nl.first, md.energies, md.nl.xyz, md.nl.forces, md.partial, smx_md::kReduceBlocks,
-                       md.reduced, s);
-    double red[10];
-    check(cudaMemcpyAsync(red, md.reduced, sizeof(red), cudaMemcpyDeviceToHost, s), "D2H");
+    double red[10] = {};
+    if (energy || virial) {
+      smx::launch_reduce(n_atoms, md.nl.first, md.energies, md.nl.xyz, md.nl.forces, md.partial, smx_md::kReduceBlocks,
+                         md.reduced, s);
+      check(cudaMemcpyAsync(red, md.reduced, sizeof(red), cudaMemcpyDeviceToHost, s), "D2H");
+    }
     check(cudaMemcpyAsync(forces, md.F, sizeof(double) * 3 * n_atoms, cudaMemcpyDeviceToHost, s), "D2H");
     if (node_energies)
       check(cudaMemcpyAsync(node_energies, md.energies, sizeof(double) * n_atoms, cudaMemcpyDeviceToHost, s), "D2H");
@@ -402,6 +462,7 @@ int compute_atoms_impl(smx_engine* eng, int n_atoms, const double* positions, co
     if (energy) *energy = red[0];
     if (virial)
       for (int q = 0; q < 9; ++q) virial[q] = red[1 + q];
+    drop.done = ws.bytes() <= AtomsWorkspace::kKeepBytes;
   } catch (const CudaError& e) {
     return fail(SMX_ERR_CUDA, e.what());
   } catch (const std::exception& e) {
