@@ -99,6 +99,13 @@ void launch_gemm(const GemmBatch& b, cudaStream_t s) {
 //   dE/dH2 (MLP gradient), H1_adj[i,0,:] = w1 + W_H1[ti] dE/dH2 (other rows 0; fixed point),
 //   M1_adj = W_M1 dE/dH2, A1_adj[i,lm,k] = dM1/dA1[lm] * M1_adj[k].
 // ---------------------------------------------------------------------------
+__device__ __forceinline__ void axpy4(float4& y, float a, float4 x) {
+  y.x = fmaf(a, x.x, y.x);
+  y.y = fmaf(a, x.y, y.y);
+  y.z = fmaf(a, x.z, y.z);
+  y.w = fmaf(a, x.w, y.w);
+}
+
 __device__ __forceinline__ void node_tail_atom(const DevModel& m, const int* __restrict__ ntype, float* __restrict__ A1,
                                                const float* __restrict__ H1, float* __restrict__ M1o,
                                                float* __restrict__ H2o, float* __restrict__ A1_adj,
@@ -117,7 +124,8 @@ __device__ __forceinline__ void node_tail_atom(const DevModel& m, const int* __r
   float* sH2 = sH10 + C;        // [C]
   float* sdH2 = sH2 + C;        // [C]
   float* sRed = sdH2 + C;       // [33][8]
-  float* sS = sRed + 33 * 8;    // [33]
+  float* sS = sRed + 33 * 8;    // [33] readout-MLP gradient factors
+  float* sE = sS + 33;          // [33] energy terms
   float f = 0.0f;
   const float* cf = m.coef1 + static_cast<size_t>(ti) * m.T1 * C + k;
   const bool dens = m.dens_spl[1] != nullptr;
@@ -159,19 +167,24 @@ __device__ __forceinline__ void node_tail_atom(const DevModel& m, const int* __r
   const float h10 = H1[static_cast<size_t>(i) * m.nLM * C + k];
   sH10[k] = h10;
   __syncthreads();
-  // H2 = W_H1[ti]^T H1[i,0,:] + W_M1^T M1: four partial sums, eight rows' loads in flight
-  const float* W = m.H2W_H1 + static_cast<size_t>(ti) * C * C + k;
-  const float* WM = m.H2W_M1 + k;
-  float hp0 = 0.0f, hp1 = 0.0f, hp2 = 0.0f, hp3 = 0.0f;  // C is a multiple of 32
-#pragma unroll 4
-  for (int r = 0; r < C; r += 4) {
-    const size_t o = static_cast<size_t>(r) * C;
-    hp0 = fmaf(sM1[r], __ldg(WM + o), fmaf(sH10[r], __ldg(W + o), hp0));
-    hp1 = fmaf(sM1[r + 1], __ldg(WM + o + C), fmaf(sH10[r + 1], __ldg(W + o + C), hp1));
-    hp2 = fmaf(sM1[r + 2], __ldg(WM + o + 2 * C), fmaf(sH10[r + 2], __ldg(W + o + 2 * C), hp2));
-    hp3 = fmaf(sM1[r + 3], __ldg(WM + o + 3 * C), fmaf(sH10[r + 3], __ldg(W + o + 3 * C), hp3));
+  // H2 = W_H1[ti]^T H1[i,0,:] + W_M1^T M1.  A thread has four output channels and a quarter
+  // of the rows, so that a weight row is read in 16-byte loads, C / 2 of them in all and
+  // independent; the quarters meet in shared memory (sX is free: the polynomial is done)
+  const int C4 = C >> 2, quarter = k / C4, c4 = k - quarter * C4, r0 = quarter * C4;
+  float4* sP = reinterpret_cast<float4*>(sX);  // [2][4 quarters][C / 4]
+  {
+    const float4* W = reinterpret_cast<const float4*>(m.H2W_H1 + static_cast<size_t>(ti) * C * C) + r0 * C4 + c4;
+    const float4* WM = reinterpret_cast<const float4*>(m.H2W_M1) + r0 * C4 + c4;
+    float4 p = make_float4(0.f, 0.f, 0.f, 0.f), q = p;
+#pragma unroll 8
+    for (int r = r0; r < r0 + C4; ++r, W += C4, WM += C4) {
+      axpy4(p, sH10[r], __ldg(W));
+      axpy4(q, sM1[r], __ldg(WM));
+    }
+    sP[k] = make_float4(p.x + q.x, p.y + q.y, p.z + q.z, p.w + q.w);
   }
-  const float h2 = (hp0 + hp1) + (hp2 + hp3);
+  __syncthreads();
+  const float h2 = (sX[k] + sX[C + k]) + (sX[2 * C + k] + sX[3 * C + k]);
   sH2[k] = h2;
   // hidden pre-activations s_u = W1[u,:] . H2 and the linear readout w1 . H1[i,0,:] (slot nh)
 #pragma unroll 4
@@ -181,46 +194,46 @@ __device__ __forceinline__ void node_tail_atom(const DevModel& m, const int* __r
     if (lane == 0) sRed[u * 8 + warp] = v;
   }
   __syncthreads();
-  for (int u = k; u <= nh; u += C) {
+  for (int u = k; u <= nh; u += C) {  // one thread per hidden unit
     float s = 0.0f;
     for (int w = 0; w < nwarp; ++w) s += sRed[u * 8 + w];
-    sS[u] = s;
+    if (u < nh) {
+      const float w2 = __ldg(m.ro2_w2 + u), sg = 1.0f / (1.0f + expf(-s));
+      sS[u] = w2 * (m.ro2_scale * sg + m.ro2_scale * s * sg * (1.0f - sg));
+      sE[u] = w2 * (m.ro2_scale * s * sg);
+    } else {
+      sE[u] = s;
+    }
   }
   __syncthreads();
   float dh2 = 0.0f;
-  for (int u = 0; u < nh; ++u) {
-    const float s = sS[u];
-    const float sg = 1.0f / (1.0f + expf(-s));
-    const float dact = m.ro2_scale * sg + m.ro2_scale * s * sg * (1.0f - sg);
-    dh2 = fmaf(__ldg(m.ro2_w2 + u) * dact, __ldg(m.ro2_w1 + static_cast<size_t>(u) * C + k), dh2);
-  }
+  for (int u = 0; u < nh; ++u) dh2 = fmaf(sS[u], __ldg(m.ro2_w1 + static_cast<size_t>(u) * C + k), dh2);
   sdH2[k] = dh2;
   if (k == 0) {
-    double e = static_cast<double>(__ldg(m.e0 + ti)) + static_cast<double>(sS[nh]);
-    for (int u = 0; u < nh; ++u) {
-      const float s = sS[u];
-      const float sg = 1.0f / (1.0f + expf(-s));
-      e += static_cast<double>(__ldg(m.ro2_w2 + u) * (m.ro2_scale * s * sg));
-    }
+    double e = static_cast<double>(__ldg(m.e0 + ti)) + static_cast<double>(sE[nh]);
+    for (int u = 0; u < nh; ++u) e += static_cast<double>(sE[u]);
     if (zbl_e) e += static_cast<double>(zbl_e[i]);
     energies[i] = e;
   }
   __syncthreads();
   // H1_adj[i,0,:] = w1 + W_H1[ti] dE/dH2 and M1_adj = W_M1 dE/dH2: as above
-  const float* WT = m.H2W_H1_T + static_cast<size_t>(ti) * C * C + k;
-  const float* WMT = m.H2W_M1_T + k;
-  float ha0 = 0.0f, ha1 = 0.0f, ma0 = 0.0f, ma1 = 0.0f;
+  {
+    const float4* WT = reinterpret_cast<const float4*>(m.H2W_H1_T + static_cast<size_t>(ti) * C * C) + r0 * C4 + c4;
+    const float4* WMT = reinterpret_cast<const float4*>(m.H2W_M1_T) + r0 * C4 + c4;
+    float4 p = make_float4(0.f, 0.f, 0.f, 0.f), q = p;
 #pragma unroll 8
-  for (int c = 0; c < C; c += 2) {
-    const size_t o = static_cast<size_t>(c) * C;
-    const float d0 = sdH2[c], d1 = sdH2[c + 1];
-    ha0 = fmaf(__ldg(WT + o), d0, ha0);
-    ma0 = fmaf(__ldg(WMT + o), d0, ma0);
-    ha1 = fmaf(__ldg(WT + o + C), d1, ha1);
-    ma1 = fmaf(__ldg(WMT + o + C), d1, ma1);
+    for (int r = r0; r < r0 + C4; ++r, WT += C4, WMT += C4) {
+      const float d = sdH2[r];
+      axpy4(p, d, __ldg(WT));
+      axpy4(q, d, __ldg(WMT));
+    }
+    sP[k] = p;
+    sP[C + k] = q;
   }
-  const float ha = __ldg(m.ro1 + k) + (ha0 + ha1);
-  const float m1a = ma0 + ma1;
+  __syncthreads();
+  const float* sQ = sX + 4 * C;
+  const float ha = __ldg(m.ro1 + k) + ((sX[k] + sX[C + k]) + (sX[2 * C + k] + sX[3 * C + k]));
+  const float m1a = (sQ[k] + sQ[C + k]) + (sQ[2 * C + k] + sQ[3 * C + k]);
   if (dens) {  // reverse_A1_scaled (mace.cpp:707-757): c_i = dA1 . A1 / s_i, dA1 /= s_i
     float dot = 0.0f;
 #pragma unroll
@@ -251,12 +264,13 @@ __device__ __forceinline__ void node_tail_atom(const DevModel& m, const int* __r
   H2_adj_o[static_cast<size_t>(i) * C + k] = dh2;
 }
 
-// at most 64 registers: eight 128-thread blocks per SM instead of six at 80 (0.129 -> 0.124 ms
-// on the 4096-atom workload; 12 bytes of spills).  At this cap the register allocation of
-// the whole kernel is sensitive to the split-row block: its row pointer is bumped row by
-// row (computing each row's address afresh took 16/24 bytes of spills and 0.010 ms).
+// What bounds it: the chain of dependent phases of a node and the 0.26 MB of weights that each
+// node reads through L2 (4 C^2 + the species' polynomial).  One output channel per thread and
+// 4-byte loads of the weights, every thread evaluating the readout's activations: 0.115 ms
+// (FP32) / 0.119 ms (BF16) for 4096 nodes of 128 channels, now 0.095 / 0.097; 300 nodes 33 ->
+// 24 us, 64 of 32 channels 17 -> 13.  80 registers: at 64 the large system gains 0.002 ms and the small ones lose 2 to 4 us.
 template <bool P>
-__global__ void __launch_bounds__(256, 4) k_node_tail(DevModel m, const int* __restrict__ ntype, float* __restrict__ A1,
+__global__ void __launch_bounds__(256, 3) k_node_tail(DevModel m, const int* __restrict__ ntype, float* __restrict__ A1,
                                                    const float* __restrict__ H1, float* __restrict__ M1o,
                                                    float* __restrict__ H2o, float* __restrict__ A1_adj,
                                                    fix64* __restrict__ H1_adj, float* __restrict__ M1_adj_o,
@@ -269,7 +283,7 @@ __global__ void __launch_bounds__(256, 4) k_node_tail(DevModel m, const int* __r
   cur.done();
 }
 
-size_t node_tail_smem(const DevModel& m) { return sizeof(float) * (34 * m.C + 4 * m.C + 33 * 8 + 33); }
+size_t node_tail_smem(const DevModel& m) { return sizeof(float) * (34 * m.C + 4 * m.C + 33 * 8 + 2 * 33); }
 
 void launch_node_tail(const DevModel& m, const int* node_type, int N, float* A1, const float* H1, float* M1,
                       float* H2, float* A1_adj, fix64* H1_adj, float* M1_adj, float* H2_adj, const float* zbl_e,
