@@ -215,9 +215,9 @@ int smx_set_option(smx_engine* eng, const char* key, long value);
  * per-atom kernel k (layer0_fwd, contract0_rev, layer0_rev, layer1_fwd, layer1_rev,
  * node_tail) runs as a persistent grid; "species_order": 1 when the sorted order is in
  * effect; "poly_canon": 1 when the model's symmetric-contraction monomials are the
- * canonical sets and run as generated code, 0 for the data-driven path; "l2_split": channel
- * slices per node of the L_max = 2 layer-1 kernels, 1 or 2, picked by the autotuner); -1 if
- * unknown. */
+ * canonical sets and run as generated code, 0 for the data-driven path; "l2_split": always 1,
+ * the layer-1 kernels cut the channels in slices of 32 themselves); -1 if unknown.  Bits of
+ * "persistent" whose kernel has one form only (layer0_fwd, contract0_rev) have no effect. */
 long smx_get_option(const smx_engine* eng, const char* key);
 
 /* The engine's own CUDA stream (a cudaStream_t): host-pointer calls and the MD driver

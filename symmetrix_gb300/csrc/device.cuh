@@ -19,7 +19,10 @@ struct DevModel {
   float h, inv_h, r_cut, ro2_scale;
   double hd;  // knot spacing of the radial splines in float64 (spline_at)
   const float4* spl0;  // [S*S][nint][4][2][C/2]: channel-pair planes
-  const float4* spl1_fwd;  // [npairs][nint][n_instr][C]: per-channel cubics
+  // [npairs][nint][n_instr][C], the instructions in the order of their groups (layer1.cuh) and
+  // two by two: (c0, c0', c1, c1'), (c2, c2', c3, c3'), ' the second one; a group's odd last
+  // one is a plain cubic
+  const float4* spl1;
   const int* mono0;
   int mono0_off[10];
   const float* coef0;  // [S][nLM][T0][C]

@@ -189,7 +189,10 @@ struct smx_engine {
     m.r_cut = pm.r_cut;
     m.ro2_scale = pm.ro2_scale;
     m.spl0 = reinterpret_cast<const float4*>(upload(pm.spl0));
-    m.spl1_fwd = reinterpret_cast<const float4*>(upload(pm.spl1_fwd));
+    m.spl1 = reinterpret_cast<const float4*>(upload(pm.spl1_fwd));
+    smx::launch_pair_splines(const_cast<float4*>(m.spl1), static_cast<long>(pm.npairs) * pm.nint, pm.C, pm.L_max);
+    check(cudaGetLastError(), "k_pair_splines");
+    check(cudaStreamSynchronize(nullptr), "k_pair_splines");
     m.mono0 = upload(pm.mono0);
     for (int q = 0; q < 10; ++q) m.mono0_off[q] = q < static_cast<int>(pm.mono0_off.size()) ? pm.mono0_off[q] : pm.mono0_off.back();
     m.coef0 = upload(pm.coef0);

@@ -13,8 +13,8 @@
 // What bounds it: the L2 gather of the spline rows, 20 KB per edge at L_max = 1 and 128
 // channels, which a plain gather kernel of the same rows runs at 19.6 TB/s (0.22 ms for 213k
 // edges).  One block of C threads per node, no prefetch, all paths and a table walk for the
-// Clebsch-Gordan rows took 0.373 ms on the 4096-atom box (213k edges), this form 0.250 ms;
-// L_max = 2, 2197 atoms, 178k edges 0.816 -> 0.437 ms; 64 atoms of 32 channels 37 -> 14.5 us.
+// Clebsch-Gordan rows took 0.373 ms on the 4096-atom box (213k edges), this form 0.251 ms;
+// L_max = 2, 2197 atoms, 178k edges 0.816 -> 0.440 ms; 64 atoms of 32 channels 37 -> 14.5 us.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -122,11 +122,9 @@ __device__ __forceinline__ void fwd_sums(const DevModel& m, const EdgeIn& in, co
     static_for<DEPTH>([&](auto dc) {
       constexpr int d = decltype(dc)::value;
       const int4 mt = st.meta[min(d, na - 1)];
-      const float4* cp = m.spl1_fwd + static_cast<size_t>(mt.y) * NI * C + k;
-      static_for<NQ>([&](auto ic) {
-        constexpr int w = decltype(ic)::value;
-        c[d][w] = __ldg(cp + grp_ins(LMAX, G, w) * C);
-      });
+      const float4* cp = m.spl1 + (static_cast<size_t>(mt.y) * NI + grp_slot(G)) * C + k;
+#pragma unroll
+      for (int w = 0; w < NQ; ++w) c[d][w] = __ldg(cp + w * C);
       const float* hp = H1 + (static_cast<size_t>(mt.z) * NL2 + r0) * C + k;
 #pragma unroll
       for (int b = 0; b < NR; ++b) h[d][b] = __ldg(hp + b * C);
@@ -138,7 +136,7 @@ __device__ __forceinline__ void fwd_sums(const DevModel& m, const EdgeIn& in, co
         const int a = a0 + d;
         if (a >= na) return;
         const int4 mn = st.meta[min(a + DEPTH, na - 1)];
-        const float4* cn = m.spl1_fwd + static_cast<size_t>(mn.y) * NI * C + k;
+        const float4* cn = m.spl1 + (static_cast<size_t>(mn.y) * NI + grp_slot(G)) * C + k;
         const float* hp = H1 + (static_cast<size_t>(mn.z) * NL2 + r0) * C + k;
         const float x = __int_as_float(st.meta[a].x);
         float hv[NR], y[16];
@@ -148,12 +146,23 @@ __device__ __forceinline__ void fwd_sums(const DevModel& m, const EdgeIn& in, co
           h[d][b] = __ldg(hp + b * C);
         }
         read_Y(st.Y[a], y);
+        float2 R2 = make_float2(0.0f, 0.0f);
         static_for<NQ>([&](auto ic) {
           constexpr int w = decltype(ic)::value;
           constexpr int q = grp_ins(LMAX, G, w);
           constexpr int l1 = ins_l1(LMAX, q), l2 = ins_l2(LMAX, q), nb = 2 * l2 + 1;
-          const float R = spline_val(c[d][w], x);
-          c[d][w] = __ldg(cn + q * C);
+          float R;
+          if constexpr (w % 2 == 0 && w + 1 < NQ) {  // the pair's values at once
+            R2 = spline2_val(c[d][w], c[d][w + 1], make_float2(x, x));
+            c[d][w] = __ldg(cn + w * C);
+            c[d][w + 1] = __ldg(cn + (w + 1) * C);
+            R = R2.x;
+          } else if constexpr (w % 2 == 1) {
+            R = R2.y;
+          } else {
+            R = spline_val(c[d][w], x);
+            c[d][w] = __ldg(cn + w * C);
+          }
           float rh[nb];
 #pragma unroll
           for (int b = 0; b < nb; ++b) rh[b] = R * hv[l2 * l2 - r0 + b];
@@ -290,12 +299,50 @@ size_t fwd_smem(int lmax, bool canon) {
   return canon ? sizeof(EdgeStage) : l1_groups(lmax) * sizeof(EdgeStage) + sizeof(float) * ins_np(lmax) * 32;
 }
 
-// Canonical items up to which two edges are kept in flight: as many as fit at once at DEPTH
-// 2's 8 warps per SM (us, one : two edges: 64 items 16.5 : 14.4, 1000 items 27.6 : 25.6, 3600
-// items of L_max = 2 71 : 82).
-constexpr long kDeepItems = 8 * 152;
+// Canonical items up to which two edges are kept in flight: DEPTH 2 has 8 warps per SM, so past
+// two rounds of them (one, for the longer edges of L_max 2) the warps hide the loads themselves
+// (us, one : two edges: 64 items 16.5 : 14.4, 2000 items 57.4 : 47.1, 16400 items 252 : 266;
+// 3600 items of L_max 2 73 : 82).
+constexpr long deep_items(int lmax) { return (lmax == 1 ? 16 : 8) * 152; }
 
 }  // namespace
+
+// Once per model, after its upload.  One thread per (row, channel): its cubics gathered, then
+// written back in pairs
+template <int LMAX>
+__global__ void k_pair_splines(float4* __restrict__ spl, long rows, int C) {
+  constexpr int NI = ins_count(LMAX);
+  const long n = rows * C;
+  for (long t = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x; t < n;
+       t += static_cast<long>(gridDim.x) * blockDim.x) {
+    float4* p = spl + t / C * NI * C + t % C;
+    float4 c[NI];
+#pragma unroll
+    for (int q = 0; q < NI; ++q) c[q] = p[q * C];
+    static_for<l1_groups(LMAX)>([&](auto gc) {
+      constexpr int G = decltype(gc)::value;
+      static_for<grp_count(G)>([&](auto ic) {
+        constexpr int w = decltype(ic)::value, slot = grp_slot(G) + w, q = grp_ins(LMAX, G, w);
+        if constexpr (w % 2 == 0 && w + 1 < grp_count(G)) {
+          constexpr int q2 = grp_ins(LMAX, G, w + 1 < grp_count(G) ? w + 1 : w);
+          p[slot * C] = make_float4(c[q].x, c[q2].x, c[q].y, c[q2].y);
+          p[(slot + 1) * C] = make_float4(c[q].z, c[q2].z, c[q].w, c[q2].w);
+        } else if constexpr (w % 2 == 0) {
+          p[slot * C] = c[q];
+        }
+      });
+    });
+  }
+}
+
+void launch_pair_splines(float4* spl, long rows, int C, int L_max) {
+  if (rows <= 0) return;
+  const int blocks = static_cast<int>(std::min<long>((rows * C + 127) / 128, 152L * 32));
+  if (L_max == 2)
+    k_pair_splines<2><<<blocks, 128>>>(spl, rows, C);
+  else
+    k_pair_splines<1><<<blocks, 128>>>(spl, rows, C);
+}
 
 bool canonical_cg(int L_max, const std::vector<int>& off, const std::vector<int>& lme, const std::vector<float>& v,
                   const int* lme_off, const int* num_e, std::vector<float>& val) {
@@ -324,7 +371,7 @@ void launch_layer1_fwd(const DevModel& m, const EdgeIn& in, const float* H1, flo
   const bool canon = m.cg_val != nullptr;
   const int nb = fwd_groups_in_block(m.L_max, canon);
   const long items = static_cast<long>(in.N) * (m.C >> 5) * (l1_groups(m.L_max) / nb);
-  const bool deep = canon && items <= kDeepItems;
+  const bool deep = canon && items <= deep_items(m.L_max);
   DevModel mk;
   const int grid = atom_grid(m, kAkLayer1Fwd, static_cast<int>(items), mk);
   const size_t smem = fwd_smem(m.L_max, canon);

@@ -18,8 +18,9 @@
 // registers; 255 registers, 8 warps: 0.55 -> 0.58 ms).  Against one block per node with two
 // instruction halves of channel pairs, which met at a barrier for every edge (8 warps per SM,
 // 47% of the cycles issuing, four FMAs on each of the 88 paths): 4096 atoms, 128 channels,
-// 213k edges 0.733 -> 0.533 ms, and without the paths that reach no output 0.47 ms; L_max = 2,
-// 2197 atoms, 178k edges 2.12 -> 1.15 -> 0.97 ms.
+// 213k edges 0.733 -> 0.533 ms; L_max = 2, 2197 atoms, 178k edges 2.12 -> 1.15 ms.  Without the
+// paths that reach no output 0.475 and 0.975 ms; with the cubics of two instructions side by
+// side in the table, so that a packed FMA takes both, 0.453 and 0.960 ms.
 //
 // L_max = 2 (17 instructions): three instruction groups in turn (layer1.cuh), so that a
 // group's g fits the registers; the H1_adj rows of l = 0, 1 are added once, those of l = 2
@@ -92,17 +93,29 @@ __device__ __forceinline__ void rev_edge(const float* g, float4* c, const float4
   read_Y(Y, y);
   constexpr int r0 = grp_row0(G);
   float dY[16], dr = 0.0f;
+  float2 R2 = make_float2(0.0f, 0.0f), Rd2 = R2;
   static_for<grp_count(G)>([&](auto ic) {
     constexpr int i = decltype(ic)::value;
     constexpr int q = grp_ins(LMAX, G, i);
     constexpr int l1 = ins_l1(LMAX, q), l2 = ins_l2(LMAX, q), nb = 2 * l2 + 1;
-    // value and derivative by the two-row Horner scheme
-    float R = fmaf(c[i].w, x, c[i].z);
-    float Rd = fmaf(c[i].w, x, R);
-    R = fmaf(R, x, c[i].y);
-    Rd = fmaf(Rd, x, R);
-    R = fmaf(R, x, c[i].x);
-    c[i] = __ldg(cn + q * C);
+    float R, Rd;
+    if constexpr (i % 2 == 0 && i + 1 < grp_count(G)) {  // the pair's values and derivatives at once
+      spline2(c[i], c[i + 1], make_float2(x, x), R2, Rd2);
+      c[i] = __ldg(cn + i * C);
+      c[i + 1] = __ldg(cn + (i + 1) * C);
+      R = R2.x;
+      Rd = Rd2.x;
+    } else if constexpr (i % 2 == 1) {
+      R = R2.y;
+      Rd = Rd2.y;
+    } else {  // by the two-row Horner scheme
+      R = fmaf(c[i].w, x, c[i].z);
+      Rd = fmaf(c[i].w, x, R);
+      R = fmaf(R, x, c[i].y);
+      Rd = fmaf(Rd, x, R);
+      R = fmaf(R, x, c[i].x);
+      c[i] = __ldg(cn + i * C);
+    }
     float us[nb], rh[nb];
 #pragma unroll
     for (int b = 0; b < nb; ++b) rh[b] = R * h[l2 * l2 - r0 + b];
@@ -201,11 +214,9 @@ __device__ __forceinline__ void rev_group(const DevModel& m, const EdgeIn& in, c
       float h[NR];
       int4 mt = s.st.meta[0];
       {
-        const float4* cp = m.spl1_fwd + static_cast<size_t>(mt.y) * NI * C + k;
-        static_for<NQ>([&](auto ic) {
-          constexpr int w = decltype(ic)::value;
-          c[w] = __ldg(cp + grp_ins(LMAX, G, w) * C);
-        });
+        const float4* cp = m.spl1 + (static_cast<size_t>(mt.y) * NI + grp_slot(G)) * C + k;
+#pragma unroll
+        for (int w = 0; w < NQ; ++w) c[w] = __ldg(cp + w * C);
         const float* hp = H1 + (static_cast<size_t>(mt.z) * NL2 + r0) * C + k;
 #pragma unroll
         for (int b = 0; b < NR; ++b) h[b] = __ldg(hp + b * C);
@@ -213,7 +224,7 @@ __device__ __forceinline__ void rev_group(const DevModel& m, const EdgeIn& in, c
       stage_Y(s.st, ed, active, pos);
       for (int a = 0; a < na; ++a) {
         const int4 mn = s.st.meta[min(a + 1, na - 1)];
-        const float4* cn = m.spl1_fwd + static_cast<size_t>(mn.y) * NI * C + k;
+        const float4* cn = m.spl1 + (static_cast<size_t>(mn.y) * NI + grp_slot(G)) * C + k;
         float hv[NR], hadj[NR];
         const float* hp = H1 + (static_cast<size_t>(mn.z) * NL2 + r0) * C + k;
 #pragma unroll

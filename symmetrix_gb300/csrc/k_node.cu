@@ -268,7 +268,8 @@ __device__ __forceinline__ void node_tail_atom(const DevModel& m, const int* __r
 // node reads through L2 (4 C^2 + the species' polynomial).  One output channel per thread and
 // 4-byte loads of the weights, every thread evaluating the readout's activations: 0.115 ms
 // (FP32) / 0.119 ms (BF16) for 4096 nodes of 128 channels, now 0.095 / 0.097; 300 nodes 33 ->
-// 24 us, 64 of 32 channels 17 -> 13.  80 registers: at 64 the large system gains 0.002 ms and the small ones lose 2 to 4 us.
+// 24 us, 64 of 32 channels 17 -> 13.  80 registers: at 64 the large system gains 0.002 ms and
+// the small ones lose 2 to 4 us.
 template <bool P>
 __global__ void __launch_bounds__(256, 3) k_node_tail(DevModel m, const int* __restrict__ ntype, float* __restrict__ A1,
                                                    const float* __restrict__ H1, float* __restrict__ M1o,

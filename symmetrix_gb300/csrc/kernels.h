@@ -27,6 +27,8 @@ void launch_layer0_rev(const DevModel& m, const EdgeIn& in, const float* A0, con
 bool canonical_cg(int L_max, const std::vector<int>& off, const std::vector<int>& lme, const std::vector<float>& v,
                   const int* lme_off, const int* num_e, std::vector<float>& val);
 cudaError_t init_layer1_kernels(const DevModel& m);
+// per-channel cubics [rows][n_instr][C] into the paired layout of DevModel::spl1, in place
+void launch_pair_splines(float4* spl, long rows, int C, int L_max);
 void launch_layer1_fwd(const DevModel& m, const EdgeIn& in, const float* H1, float* Phi1, cudaStream_t s);
 // H1_adj: fixed-point accumulator (see to_fixed), seeded by launch_node_tail
 // k_layer1_rev.cu: f1 receives the edge forces' sums over each 32-channel slice, f1_stride apart

@@ -17,6 +17,12 @@ __host__ __device__ constexpr int grp_ins(int LMAX, int G, int i) {
   constexpr int b[10] = {0, 4, 3, 1, 9, 8, 5, 14, 13, 10}, b1[4] = {11, 15, 2, 16}, b2[3] = {6, 12, 7};
   return LMAX == 1 ? a[i] : (G == 0 ? b[i] : (G == 1 ? b1[i] : b2[i]));
 }
+// first slot of group G in a spline row (DevModel::spl1)
+__host__ __device__ constexpr int grp_slot(int G) {
+  int s = 0;
+  for (int w = 0; w < G; ++w) s += grp_count(w);
+  return s;
+}
 // the H1 rows [row0, row0 + rows) that group G reads
 __host__ __device__ constexpr int grp_row0(int G) { return G == 0 ? 0 : 4; }
 __host__ __device__ constexpr int grp_rows(int G) { return G == 0 ? 4 : 5; }
