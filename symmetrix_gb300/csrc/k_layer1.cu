@@ -13,8 +13,8 @@
 // What bounds it: the L2 gather of the spline rows, 20 KB per edge at L_max = 1 and 128
 // channels, which a plain gather kernel of the same rows runs at 19.6 TB/s (0.22 ms for 213k
 // edges).  One block of C threads per node, no prefetch, all paths and a table walk for the
-// Clebsch-Gordan rows took 0.373 ms on the 4096-atom box (213k edges), this form 0.251 ms;
-// L_max = 2, 2197 atoms, 178k edges 0.816 -> 0.440 ms; 64 atoms of 32 channels 37 -> 14.5 us.
+// Clebsch-Gordan rows took 0.373 ms on the 4096-atom box (213k edges), this form 0.250 ms;
+// L_max = 2, 2197 atoms, 178k edges 0.816 -> 0.435 ms; 64 atoms of 32 channels 37 -> 14.5 us.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -266,11 +266,13 @@ __device__ __forceinline__ void fwd_general(const DevModel& m, const EdgeIn& in,
 
 // Blocks: general tables, one per (node, slice) with the groups' warps in it; canonical ones,
 // one warp per (node, slice, group).  DEPTH 1: 168 registers, 12 warps per SM; DEPTH 2: 8.
+// (Asked for 11, DEPTH 1 keeps the 12 and its loads are ordered better, ms, 11 : 12: 213k edges
+// 0.250 : 0.252, L_max 2, 178k edges 0.435 : 0.440; for 13, 0.352 and 0.497.)
 __host__ __device__ constexpr int fwd_groups_in_block(int LMAX, bool CANON) { return CANON ? 1 : l1_groups(LMAX); }
 
 template <int LMAX, int CT, bool CANON, int DEPTH, bool P>
 __global__ void __launch_bounds__(32 * fwd_groups_in_block(LMAX, CANON),
-                                  (DEPTH == 1 ? 12 : 8) / fwd_groups_in_block(LMAX, CANON))
+                                  (DEPTH == 1 ? (CANON ? 11 : 12) : 8) / fwd_groups_in_block(LMAX, CANON))
     k_layer1_fwd(DevModel m, EdgeIn in, const float* __restrict__ H1, float* __restrict__ Phi1) {
   pdl_begin();
   extern __shared__ __align__(16) unsigned char dyn[];

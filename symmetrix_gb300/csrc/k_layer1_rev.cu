@@ -14,13 +14,13 @@
 // the radial term are summed over the lanes four edges at a time through shared memory, and
 // only these sums meet dY_a/dx.
 //
-// What bounds it: issue slots (64 to 70% of the cycles issue, at 12 warps per SM and 168
+// What bounds it: issue slots (63% of the cycles issue, at 12 warps per SM and 168
 // registers; 255 registers, 8 warps: 0.55 -> 0.58 ms).  Against one block per node with two
 // instruction halves of channel pairs, which met at a barrier for every edge (8 warps per SM,
 // 47% of the cycles issuing, four FMAs on each of the 88 paths): 4096 atoms, 128 channels,
 // 213k edges 0.733 -> 0.533 ms; L_max = 2, 2197 atoms, 178k edges 2.12 -> 1.15 ms.  Without the
 // paths that reach no output 0.475 and 0.975 ms; with the cubics of two instructions side by
-// side in the table, so that a packed FMA takes both, 0.453 and 0.960 ms.
+// side in the table, so that a packed FMA takes both, 0.444 and 0.960 ms.
 //
 // L_max = 2 (17 instructions): three instruction groups in turn (layer1.cuh), so that a
 // group's g fits the registers; the H1_adj rows of l = 0, 1 are added once, those of l = 2
@@ -288,8 +288,11 @@ __device__ __forceinline__ void rev_item(const DevModel& m, const EdgeIn& in, co
 
 }  // namespace
 
+// 12 warps per SM either way (168 registers, three warps per scheduler); asked for 11, the
+// compiler orders the L_max = 1 kernel's loads better (ms, 11 : 12, 213k edges of 128 channels
+// 0.444 : 0.453; L_max = 2, 178k edges 0.962 : 0.959).
 template <int LMAX, int CT, bool CANON, bool P>
-__global__ void __launch_bounds__(32, 12) k_layer1_rev(DevModel m, EdgeIn in, const float* __restrict__ H1,
+__global__ void __launch_bounds__(32, LMAX == 1 ? 11 : 12) k_layer1_rev(DevModel m, EdgeIn in, const float* __restrict__ H1,
                                                       const float* __restrict__ dPhi1, fix64* __restrict__ H1_adj,
                                                       float* __restrict__ f1, int split, int cs) {
   pdl_begin();
