@@ -728,7 +728,7 @@ struct smx_engine {
       smx::launch_rows_to_fixed(nullptr, H1_adj_fx + static_cast<size_t>(N1) * dm.nLM * C,
                                 static_cast<long>(N - N1) * dm.nLM * C, true, s);
     // The BF16 form's GEMMs read the producers' split bf16 rows; the float32 copies of
-    // M0, Phi1 and A1_adj are then written only for inspection or a SIMT fallback.
+    // M0, Phi1 and A1_adj are then written only for inspection or a float32 GEMM.
     bool all_A1 = true, all_Phi1adj = true;
     for (int l = 0; l < 4; ++l)
       if (dm.num_e[l] > 0) {

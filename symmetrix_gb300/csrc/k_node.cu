@@ -304,7 +304,7 @@ void node_tail_residency(const DevModel& m, int* per_sm) {
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm[kAkNodeTail], k_node_tail<true>, m.C, node_tail_smem(m));
 }
 
-// H1_adj from its fixed-point accumulator: float rows for the SIMT GEMM and the stage
+// H1_adj from its fixed-point accumulator: float rows for the float32 GEMM and the stage
 // reads, and in the BF16 form the M0_adj GEMM's split operand rows (write_split with
 // `terms` products: row pitch split_xterms(terms) * C; rows grouped by L, lgroup_row).
 __global__ void k_fixed_rows(const fix64* __restrict__ src, float* __restrict__ dst, __nv_bfloat16* __restrict__ bf,

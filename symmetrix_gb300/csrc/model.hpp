@@ -82,7 +82,8 @@ struct PackedModel {
   // plane 0 = (c0, c0', c1, c1'), plane 1 = (c2, c2', c3, c3')
   std::vector<float> spl0;
   // [npairs][nint][n_instr][2][C/2][4], canonical instruction order; channel pairs
-  // (2c, 2c+1): plane 0 = (c0, c0', c1, c1'), plane 1 = (c2, c2', c3, c3')
+  // (2c, 2c+1): plane 0 = (c0, c0', c1, c1'), plane 1 = (c2, c2', c3, c3').  Part of the
+  // binary model file's format; the kernels read spl1_fwd's values
   std::vector<float> spl1;
   std::vector<float> spl1_fwd;  // [npairs][nint][n_instr][C][4]: one float4 cubic per channel
   std::vector<int> mono0;      // packed a | b<<8 | c<<16 (16 = constant one), per LM contiguous
