@@ -534,20 +534,27 @@ void dispatch_c0(int C, F&& f) {
 }
 
 size_t fwd0_smem(const DevModel& m) { return m.poly_canon ? 0 : 17 * 32 * sizeof(float2); }
+size_t contract0_smem(int warps, bool split, bool canon) {
+  return warps * ((split ? 16 : 0) + (canon ? 0 : 2 * 17)) * 32 * sizeof(float2);
+}
 size_t contract0_smem(const DevModel& m, bool split) {
-  return contract0_warps(m, split) * ((split ? 16 : 0) + (m.poly_canon ? 0 : 2 * 17)) * 32 * sizeof(float2);
+  return contract0_smem(contract0_warps(m, split), split, m.poly_canon != 0);
 }
 
 }  // namespace
 
 // Dynamic shared memory above 48 KB must be opted into once per kernel (outside any stream
-// capture).
+// capture).  The limit belongs to the function, which serves every engine of the process, so
+// it is the most that any model of the instantiation needs (data-driven polynomials of its
+// widest block: 204,800 bytes for 4 outputs of 256 channels, 230,400 for 9 of 128): set by
+// each engine's own need, a later engine's would narrow an earlier one's.
 cudaError_t init_edge_kernels(const DevModel& m) {
   cudaError_t e = init_layer1_kernels(m);
   dispatch_poly(m, [&](auto nc, auto cc) {
+    constexpr int NLM = decltype(nc)::value, CT = decltype(cc)::value;
     if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(k_contract0_rev<decltype(nc)::value, decltype(cc)::value, true>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(contract0_smem(m, true)));
+      e = cudaFuncSetAttribute(k_contract0_rev<NLM, CT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               static_cast<int>(contract0_smem(contract0_max_warps(NLM, CT, true), true, false)));
   });
   return e;
 }
