@@ -233,7 +233,9 @@ __global__ void __launch_bounds__(32, 12) k_layer0_fwd(DevModel m, EdgeIn in, fl
 //   A0_adj[i,:,k] = sum_LM M0_adj[i,LM,k] grad P_{ti,LM,k}(A0[i,:,k]).
 // A block per node, a lane per channel pair: one warp per 64 channels, or (SPLIT, small
 // systems) a warp per output LM and 64 channels, whose gradients meet in shared memory and
-// are added in the order of LM.
+// are added in the order of LM.  The one warp adds whole gradients of the outputs in that order
+// too: a node's bits do not depend on the form, which follows from the number of nodes, so a
+// molecule gives the same forces alone and in a batch.
 // ---------------------------------------------------------------------------
 constexpr int contract0_max_warps(int NLM, int CT, bool SPLIT) {
   return (SPLIT ? NLM : 1) * (CT > 0 ? (CT + 63) / 64 : (NLM == 9 ? 2 : 4));
@@ -268,17 +270,25 @@ __global__ void __launch_bounds__(32 * contract0_max_warps(NLM, CT, SPLIT),
   if (m.poly_canon) {  // generated code, registers only
     static_for<NLM>([&](auto lc) {
       constexpr int LM = decltype(lc)::value;
-      if (!SPLIT || LM == part) contract_grad<LM>(x, __ldg(w + LM * C2), cf + LM * sst, C2, dA);
+      if constexpr (SPLIT) {
+        if (LM == part) contract_grad<LM>(x, __ldg(w + LM * C2), cf + LM * sst, C2, dA);
+      } else {
+        float2 g[16];
+#pragma unroll
+        for (int q = 0; q < 16; ++q) g[q] = make_float2(0.0f, 0.0f);
+        contract_grad<LM>(x, __ldg(w + LM * C2), cf + LM * sst, C2, g);
+#pragma unroll
+        for (int q = 0; q < 16; ++q) dA[q] = LM == 0 ? g[q] : __fadd2_rn(dA[q], g[q]);
+      }
     });
   } else {  // data-driven monomial lists, this lane's columns in shared memory
     float2* sA = reinterpret_cast<float2*>(dyn) + warp * 17 * 32 * 2 + lane;  // [17][32]
     float2* sG = sA + 17 * 32;                                               // (row 16 absorbs the constant slot)
 #pragma unroll
-    for (int q = 0; q < 17; ++q) {
-      sA[q * 32] = q < 16 ? x[q < 16 ? q : 0] : make_float2(1.0f, 1.0f);
-      sG[q * 32] = make_float2(0.0f, 0.0f);
-    }
+    for (int q = 0; q < 17; ++q) sA[q * 32] = q < 16 ? x[q < 16 ? q : 0] : make_float2(1.0f, 1.0f);
     for (int LM = part; LM < m.nLM; LM += parts) {
+#pragma unroll
+      for (int q = 0; q < 17; ++q) sG[q * 32] = make_float2(0.0f, 0.0f);
       const float2 wl = __ldg(w + LM * C2);
       const int t0 = m.mono0_off[LM], t1 = m.mono0_off[LM + 1];
       for (int t = t0; t < t1; ++t) {
@@ -290,10 +300,9 @@ __global__ void __launch_bounds__(32 * contract0_max_warps(NLM, CT, SPLIT),
         sG[b] = fma2(mul2(cw, xa), xc, sG[b]);
         sG[c] = fma2(mul2(cw, xa), xb, sG[c]);
       }
-      if (SPLIT) break;
-    }
 #pragma unroll
-    for (int q = 0; q < 16; ++q) dA[q] = sG[q * 32];
+      for (int q = 0; q < 16; ++q) dA[q] = LM == part ? sG[q * 32] : __fadd2_rn(dA[q], sG[q * 32]);
+    }
   }
   float2* out = reinterpret_cast<float2*>(A0_adj + static_cast<size_t>(i) * 16 * C) + cp;
   float S = 1.0f;  // reverse_A0_scaled (mace.cpp:299-346): c_i = dA . A0 / s_i, dA /= s_i
@@ -326,8 +335,10 @@ __global__ void __launch_bounds__(32 * contract0_max_warps(NLM, CT, SPLIT),
       for (int u = 1; u < parts; ++u) s = __fadd2_rn(s, sum[((u * ns + slice) * 16 + q) * 32]);
       return s;
     };
-    if (m.dens_spl[0]) {
-      for (int q = part; q < 16; q += parts) d2 = fma2(row(q), __ldg(xr + q * C2), d2);
+    if (m.dens_spl[0]) {  // by the warps of output 0, in the order of the other form
+      if (part == 0)
+#pragma unroll
+        for (int q = 0; q < 16; ++q) d2 = fma2(row(q), x[q], d2);
       density(d2);
     }
     for (int q = part; q < 16; q += parts) store(q, row(q));
