@@ -448,17 +448,22 @@ __global__ void k_reduce_partials(int N, const int* __restrict__ first, const do
   if (threadIdx.x < 10) partial[blockIdx.x * 10 + threadIdx.x] = sh[threadIdx.x][0];
 }
 
-// one warp per quantity: compensated sums of every 32nd block, then a pairwise tree in a fixed
-// order (one thread per quantity over 64 blocks took 20 us, a chain of float64 sums; 10 us)
+// one warp per quantity: compensated sums of every 32nd block, then a tree of compensated sums
+// in a fixed order (one thread per quantity over 64 blocks took 20 us, a chain of float64
+// sums; 10 us)
 __global__ void __launch_bounds__(320) k_reduce_final(int nblocks, const double* __restrict__ partial,
                                                       double* __restrict__ out) {
   const int q = threadIdx.x >> 5, lane = threadIdx.x & 31;
   CompSum s;
   for (int b = lane; b < nblocks; b += 32) s.add(partial[b * 10 + q]);
-  double v = s.value();
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-  if (lane == 0) out[q] = v;
+  for (int o = 16; o > 0; o >>= 1) {
+    CompSum t;
+    t.s = __shfl_down_sync(0xffffffffu, s.s, o);
+    t.c = __shfl_down_sync(0xffffffffu, s.c, o);
+    s.add(t);
+  }
+  if (lane == 0) out[q] = s.value();
 }
 
 // velocity Verlet halves
