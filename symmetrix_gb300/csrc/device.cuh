@@ -81,8 +81,11 @@ struct DevModel {
   // sched[0..1]; 0 launches one block per atom.  pgrid is read on the host only.
   int* sched;
   int pgrid[8];
-  // layer-1 adjoint: the offset between the partial edge forces of its 32-channel slices
+  // layer-1 adjoint: its partial edge forces, one plane of f1_stride components per 32-channel
+  // slice.  A component is f1_width floats: 1, or at L_max = 2, where a slice's three instruction
+  // groups are added, (sum, what its rounding dropped), which hold the sum as float64 would
   long f1_stride;
+  int f1_width;
   // the engine's status word (mapped host memory): a bounded wait that gave up sets bit 0
   unsigned* status;
 };
@@ -441,6 +444,22 @@ __device__ __forceinline__ void sph_harm16(float vx, float vy, float vz, float* 
       G[2 * 16 + q] = gX;
     }
   }
+}
+
+// Component t of the layer-1 edge forces: the float64 sum of its planes (DevModel::f1_stride)
+__device__ __forceinline__ double f1_sum(const float* __restrict__ f1, long stride, int planes, int width, long t) {
+  double f = 0.0;
+  if (width == 1) {
+    for (int h = 0; h < planes; ++h) f += static_cast<double>(f1[h * stride + t]);
+    return f;
+  }
+  float low = 0.0f;  // below 2^-24 of the sums
+  for (int h = 0; h < planes; ++h) {
+    const float2 v = reinterpret_cast<const float2*>(f1)[h * stride + t];
+    f += static_cast<double>(v.x);
+    low += v.y;
+  }
+  return f + static_cast<double>(low);
 }
 
 __device__ __forceinline__ float warp_sum(float v) {

@@ -84,7 +84,7 @@ struct smx_engine {
   float *A0 = nullptr, *M0 = nullptr, *H1 = nullptr, *Phi1 = nullptr, *A1 = nullptr, *M1 = nullptr, *H2 = nullptr;
   float *A0_adj = nullptr, *M0_adj = nullptr, *H1_adj = nullptr, *Phi1_adj = nullptr, *A1_adj = nullptr;
   float *M1_adj = nullptr, *H2_adj = nullptr;
-  float* f1 = nullptr;  // layer-1 edge forces, one partial sum per 32-channel slice
+  float* f1 = nullptr;  // layer-1 edge forces, partial sums (DevModel::f1_stride)
   smx::fix64* H1_adj_fx = nullptr;  // H1_adj accumulator (fixed point: order-independent sums)
   // precision form: bf16 GEMM operands (M0 and H1_adj as [N*nLM][C]; Phi1 and A1_adj
   // regrouped per l as [N*(2l+1)][n_eta*C] and [N*(2l+1)][C])
@@ -253,6 +253,7 @@ struct smx_engine {
     m.op_m0 = m.op_phi1 = m.op_a1adj = nullptr;
     m.tc_terms = tc_terms;
     m.f1_stride = 0;
+    m.f1_width = pm.L_max == 2 ? 2 : 1;
     m.zbl_p = pm.zbl_p;
     for (int q = 0; q < 4; ++q) m.zbl_c[q] = pm.zbl_c[q];
     m.zbl_pair = pm.has_zbl ? reinterpret_cast<const float4*>(upload(pm.zbl_pair)) : nullptr;
@@ -367,7 +368,7 @@ struct smx_engine {
     M1_adj = dalloc<float>(nN * C);
     H2_adj = dalloc<float>(nN * C);
     dm.f1_stride = 3 * nE;
-    f1 = dalloc<float>(3 * nE * (C >> 5));
+    f1 = dalloc<float>(3 * nE * (C >> 5) * dm.f1_width);
     zbl_e = dalloc<float>(nN);
     first = dalloc<int>(nN + 1);
     ntype = dalloc<int>(nN);
@@ -676,7 +677,7 @@ struct smx_engine {
     smx::launch_rows_to_fixed(H1_adj, H1_adj_fx, nh, zero_h1adj, s);
     smx::launch_layer1_rev(m, in, H1, Phi1_adj, H1_adj_fx, f1, s);
     smx::launch_fixed_rows(H1_adj_fx, H1_adj, nullptr, in.N * static_cast<long>(dm.nLM), dm.C, 1, dm.nLM, s);
-    smx::launch_forces_from_f1(forces, f1, dm.f1_stride, dm.C >> 5, 3 * E, zero_dxyz, s);
+    smx::launch_forces_from_f1(forces, f1, dm.f1_stride, dm.C >> 5, dm.f1_width, 3 * E, zero_dxyz, s);
   }
 
   // The full forward + adjoint pass on device-resident inputs (tuning the atom schedule

@@ -483,9 +483,7 @@ __device__ __forceinline__ void layer0_rev_item(const DevModel& m, const EdgeIn&
         for (int a = 0; a < 3; ++a) f[a] = fma(-g, in.xyz[3 * e + a], f[a]);
       }
       for (int a = 0; a < 3; ++a) {
-        double w = 0.0;
-        if (local)
-          for (int h = 0; h < C >> 5; ++h) w += static_cast<double>(f1[h * m.f1_stride + 3 * e + a]);  // channel slices
+        const double w = local ? f1_sum(f1, m.f1_stride, C >> 5, m.f1_width, 3 * e + a) : 0.0;
         forces[3 * e + a] = -(f[a] + w);
       }
     }

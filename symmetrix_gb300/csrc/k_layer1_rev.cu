@@ -149,8 +149,14 @@ __device__ __forceinline__ void rev_edge(const float* g, float4* c, const float4
   for (int v = 1; v < 8; ++v) t[kSumRow * v] = make_float2(dY[2 * v], dY[2 * v + 1]);
 }
 
+// a + b as its rounding and what that drops (Knuth, The Art of Computer Programming 2, 4.2.2)
+__device__ __forceinline__ float2 two_sum(float a, float b) {
+  const float s = __fadd_rn(a, b), t = __fsub_rn(s, a);
+  return make_float2(s, __fadd_rn(__fsub_rn(a, __fsub_rn(s, t)), __fsub_rn(b, t)));
+}
+
 // Group G over the edges of chunks `split` apart; the edge forces of the earlier groups
-// of the same warp are in f1 already.
+// of the same warp are in f1 already (DevModel::f1_stride).
 template <int LMAX, int G, int CT, bool CANON>
 __device__ __forceinline__ void rev_group(const DevModel& m, const EdgeIn& in, const float* __restrict__ H1,
                                           const float* __restrict__ dPhi1, fix64* __restrict__ H1_adj,
@@ -260,10 +266,21 @@ __device__ __forceinline__ void rev_group(const DevModel& m, const EdgeIn& in, c
           fz = fmaf(S[q], D[32 + q], fz);
         }
       }
-      float* o = f1 + 3 * e;
-      o[0] = G > 0 ? o[0] + fx : fx;
-      o[1] = G > 0 ? o[1] + fy : fy;
-      o[2] = G > 0 ? o[2] + fz : fz;
+      const float f[3] = {fx, fy, fz};
+#pragma unroll
+      for (int v = 0; v < 3; ++v) {
+        if constexpr (LMAX == 1) {
+          f1[3 * e + v] = f[v];
+        } else {
+          float2* o = reinterpret_cast<float2*>(f1) + 3 * e + v;
+          if constexpr (G == 0) {
+            *o = make_float2(f[v], 0.0f);
+          } else {
+            const float2 a = *o, s = two_sum(a.x, f[v]);
+            *o = make_float2(s.x, a.y + s.y);
+          }
+        }
+      }
     }
   }
 }
@@ -278,7 +295,7 @@ __device__ __forceinline__ void rev_item(const DevModel& m, const EdgeIn& in, co
   const int i = in.atom_at(w / ns), slice = w % ns;
   if (in.first[i] + part * cs >= in.end(i)) return;
   const int k = slice * 32 + (threadIdx.x & 31);
-  float* f1s = f1 + slice * m.f1_stride;
+  float* f1s = f1 + slice * m.f1_stride * (LMAX == 2 ? 2 : 1);
   rev_group<LMAX, 0, CT, CANON>(m, in, H1, dPhi1, H1_adj, f1s, s, i, k, part, split, cs);
   if constexpr (LMAX == 2) {
     rev_group<LMAX, 1, CT, CANON>(m, in, H1, dPhi1, H1_adj, f1s, s, i, k, part, split, cs);

@@ -341,13 +341,11 @@ __global__ void k_rows_to_fixed(const float* __restrict__ src, fix64* __restrict
     dst[t] = zero ? 0ull : to_fixed(src[t]);
 }
 
-__global__ void k_forces_from_f1(double* __restrict__ forces, const float* __restrict__ f1, long stride, int nslices,
-                                 long n, int zero) {
+__global__ void k_forces_from_f1(double* __restrict__ forces, const float* __restrict__ f1, long stride, int planes,
+                                 int width, long n, int zero) {
   for (long t = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x; t < n;
        t += static_cast<long>(gridDim.x) * blockDim.x) {
-    double f = 0.0;
-    for (int h = 0; h < nslices; ++h) f += static_cast<double>(f1[h * stride + t]);
-    forces[t] = (zero ? 0.0 : forces[t]) - f;
+    forces[t] = (zero ? 0.0 : forces[t]) - f1_sum(f1, stride, planes, width, t);
   }
 }
 
@@ -356,11 +354,11 @@ void launch_rows_to_fixed(const float* src, fix64* dst, long n, bool zero, cudaS
   k_rows_to_fixed<<<static_cast<int>(std::min<long>((n + 255) / 256, 152L * 16)), 256, 0, s>>>(src, dst, n, zero);
 }
 
-void launch_forces_from_f1(double* forces, const float* f1, long stride, int nslices, long n, bool zero,
-                           cudaStream_t s) {
+void launch_forces_from_f1(double* forces, const float* f1, long stride, int planes, int width, long n,
+                           bool zero, cudaStream_t s) {
   if (n <= 0) return;
   k_forces_from_f1<<<static_cast<int>(std::min<long>((n + 255) / 256, 152L * 16)), 256, 0, s>>>(forces, f1, stride,
-                                                                                               nslices, n, zero);
+                                                                                               planes, width, n, zero);
 }
 
 // Centre atoms sorted by species (a counting sort; the order inside a species is

@@ -31,7 +31,7 @@ cudaError_t init_layer1_kernels(const DevModel& m);
 void launch_pair_splines(float4* spl, long rows, int C, int L_max);
 void launch_layer1_fwd(const DevModel& m, const EdgeIn& in, const float* H1, float* Phi1, cudaStream_t s);
 // H1_adj: fixed-point accumulator (see to_fixed), seeded by launch_node_tail
-// k_layer1_rev.cu: f1 receives the edge forces' sums over each 32-channel slice, f1_stride apart
+// k_layer1_rev.cu: f1 receives the edge forces' partial sums (DevModel::f1_stride)
 int layer1_rev_residency(const DevModel& m);
 void launch_layer1_rev(const DevModel& m, const EdgeIn& in, const float* H1, const float* dPhi1, fix64* H1_adj,
                        float* f1, cudaStream_t s);
@@ -66,10 +66,10 @@ void launch_node_tail(const DevModel& m, const int* node_type, int N, float* A1,
 void launch_fixed_rows(const fix64* src, float* dst, __nv_bfloat16* bf, long rows, int C, int terms, int nLM,
                        cudaStream_t s);
 // single-stage calls: dst = fixed-point copy of src (zero: dst = 0); forces = (zero ? 0 :
-// forces) - the sum of the nslices f1 slices (stride apart), n = 3 * edges
+// forces) - the sum of the f1 planes (stride components of width floats apart), n = 3 * edges
 void launch_rows_to_fixed(const float* src, fix64* dst, long n, bool zero, cudaStream_t s);
-void launch_forces_from_f1(double* forces, const float* f1, long stride, int nslices, long n, bool zero,
-                           cudaStream_t s);
+void launch_forces_from_f1(double* forces, const float* f1, long stride, int planes, int width, long n,
+                           bool zero, cudaStream_t s);
 void launch_scan_first(const int* num_neigh, int N, int* first, cudaStream_t s);
 // input check of the host API (bits of the flags word)
 constexpr unsigned kBadNodeType = 1, kBadNumNeigh = 2, kBadEdgeCount = 4, kBadNeighIndex = 8, kBadNeighType = 16,

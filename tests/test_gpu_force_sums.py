@@ -1,0 +1,49 @@
+"""Per-edge forces are summed in float64 above the float32 sums over lanes: the layer-1 adjoint's three
+instruction groups at L_max = 2."""
+import numpy as np
+import pytest
+
+from helpers import edge_args
+from symmetrix_gb300.synth.model import make_model, write_model
+from symmetrix_gb300.synth.structures import neighbor_list, random_box
+
+pytestmark = pytest.mark.gpu
+
+# (l1, l2, l) of the groups of l2 = 2; the first group has the instructions of l2 = 0, 1
+GROUPS = [{(0, 2, 2), (1, 2, 3), (2, 2, 0), (3, 2, 3)}, {(1, 2, 1), (2, 2, 2), (3, 2, 1)}]
+
+
+def test_instruction_groups_of_l_max_2(engine_lib, tmp_path):
+    """The edge forces of dPhi1 are the float64 sum of those of its rows of each group."""
+    from symmetrix_gb300 import MACE
+    C = 32  # one slice
+    model = make_model(num_channels=C, species=("H", "C", "O"), r_cut=4.0, L_max=2, num_knots=40, seed=4)
+    m = MACE(write_model(model, str(tmp_path / "m.json")))
+    pos, L, species = random_box(40, 0.08, 0.9, 3, seed=6)
+    nl = neighbor_list(pos, 4.0, L)
+    a = edge_args(species, nl)
+    n = len(species)
+    m.compute_node_energies_forces(*a)
+    ins = list(zip(model["Phi1_l1"], model["Phi1_l2"], model["Phi1_l"]))
+    group, at = np.zeros(m.stage("Phi1_adj").size // (n * C), int), 0
+    for l in range(4):
+        of_l = [q for q in ins if q[2] == l]
+        for k in range((2 * l + 1) * len(of_l)):
+            q = of_l[k % len(of_l)]
+            group[at + k] = 1 if q in GROUPS[0] else (2 if q in GROUPS[1] else 0)
+        at += (2 * l + 1) * len(of_l)
+    assert at == len(group)
+    dPhi1 = np.random.default_rng(1).normal(size=(n, len(group), C)).astype(np.float32)
+    m.compute_R1(n, species, a[2], a[4], a[6])
+    m.compute_Y(a[5])
+
+    def forces(mask):
+        m.set_stage("Phi1_adj", dPhi1 * mask[None, :, None])
+        m.reverse_Phi1(n, a[2], a[3], a[5], a[6], True, True)
+        return np.array(m.node_forces)
+
+    parts = [forces(group == g) for g in range(3)]
+    for p in parts:  # float32 sums, one slice
+        assert np.abs(p).max() > 1e-3 and np.array_equal(p, p.astype(np.float32))
+    err = np.abs(forces(group >= 0) - (parts[0] + parts[1] + parts[2])).max()
+    assert err <= 1e-13 * max(np.abs(p).max() for p in parts)
