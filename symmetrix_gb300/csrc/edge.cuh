@@ -24,26 +24,29 @@ struct LaneEdge {
 constexpr int kSumEdges = 4;  // edges summed over the lanes at a time
 constexpr int kSumRow = 33;   // row pitch of their terms: 32 rows read at one column hit all banks
 
-
 // Sums over the lanes of the terms of n edges (n <= kSumEdges): lane 8 e + v adds component
-// pair v of edge e, four partial sums in a fixed order, into out[e][16] (ADD: onto it).
-template <bool ADD>
+// pair v of edge e, four partial sums in a fixed order, into the 16 floats at out + e PITCH, or
+// with HALVES the sums of lanes 0-15 and 16-31 into the 32 there.
+template <bool HALVES, int PITCH>
 __device__ __forceinline__ void sum_lanes(const float2* buf, float* out, int n) {
   const int lane = threadIdx.x & 31, e = lane >> 3, v = lane & 7;
   __syncwarp();
   if (e < n) {
     const float2* row = buf + lane * kSumRow;
     float2 p0 = make_float2(0.0f, 0.0f), p1 = p0, p2 = p0, p3 = p0;
+    constexpr int step = HALVES ? 2 : 4, third = HALVES ? 16 : 2;
 #pragma unroll
-    for (int i = 0; i < 32; i += 4) {
+    for (int i = 0; i < 8 * step; i += step) {
       p0 = __fadd2_rn(p0, row[i]);
       p1 = __fadd2_rn(p1, row[i + 1]);
-      p2 = __fadd2_rn(p2, row[i + 2]);
-      p3 = __fadd2_rn(p3, row[i + 3]);
+      p2 = __fadd2_rn(p2, row[i + third]);
+      p3 = __fadd2_rn(p3, row[i + third + 1]);
     }
-    float2* o = reinterpret_cast<float2*>(out + 16 * e + 2 * v);
-    const float2 s = __fadd2_rn(__fadd2_rn(p0, p1), __fadd2_rn(p2, p3));
-    *o = ADD ? __fadd2_rn(*o, s) : s;
+    float2* o = reinterpret_cast<float2*>(out + PITCH * e + 2 * v);
+    p0 = __fadd2_rn(p0, p1);
+    p2 = __fadd2_rn(p2, p3);
+    *o = HALVES ? p0 : __fadd2_rn(p0, p2);
+    if (HALVES) o[8] = p2;
   }
   __syncwarp();
 }

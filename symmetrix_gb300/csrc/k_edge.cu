@@ -13,8 +13,8 @@
 // coefficients, 0.2 MB per node.  Against a block of two warp groups per node whose sums met
 // in shared memory, five-and-forty scalar FMAs per edge and channel for the force and
 // polynomials with the products of pairs in registers (255 of them): 4096 atoms, 128
-// channels, forward 0.165 -> 0.137 ms, adjoints together 0.262 -> 0.182 ms; L_max = 2, 2197
-// atoms 0.225 -> 0.126 and 0.260 -> 0.186 ms.
+// channels, forward 0.165 -> 0.130 ms, adjoints together 0.262 -> 0.181 ms; L_max = 2, 2197
+// atoms 0.225 -> 0.122 and 0.260 -> 0.188 ms.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -27,9 +27,13 @@ namespace smx {
 
 namespace {
 
+constexpr int kRow0 = 18;
+
 // Up to 32 edges of a node staged by one warp, those inside the cut-off packed to the front.
 struct L0Stage {
-  alignas(16) float2 Y2[kEdgeChunk][16];  // (Y_lm, Y_lm): operands of the packed FMAs
+  // (Y_lm, Y_lm): operands of the packed FMAs.  In the adjoint, once an edge is done: its sums in
+  // their place (the row pitch: 16-byte reads of the lanes' own rows hit all banks)
+  alignas(16) float2 Y2[kEdgeChunk][kRow0];
   int2 meta[kEdgeChunk];      // offset inside the spline interval (float bits), ordered-pair spline row
 };
 
@@ -107,7 +111,7 @@ constexpr int kDepth0 = 2;  // edges in flight per warp of the forward
 // Layer 0 forward: A0[i,lm,k] = sum_j Y_lm(x_ij) R0'_{ti,tj,l}(r_ij)[k] with the
 // folded ordered-pair splines, then M0[i,LM,k] = P_{ti,LM,k}(A0[i,:,k]) for the lane's two
 // channels.  (The contraction as a kernel of its own, a warp per output LM: 0.108 + 0.039 ms
-// against 0.137 ms together.)
+// against 0.137 ms together, before the row pitch of the staged Y.)
 // ---------------------------------------------------------------------------
 template <int NLM, int CT>
 __device__ __forceinline__ void layer0_fwd_item(const DevModel& m, const EdgeIn& in, float* __restrict__ A0,
@@ -350,13 +354,13 @@ __global__ void __launch_bounds__(32 * contract0_max_warps(NLM, CT, SPLIT),
 // radial splines and Y_lm; ZBL and the density factors add their terms; forces =
 // -(layer 0 + layer 1).  A warp sums all channels of its node's edges, up to two channel
 // pairs per lane at a time: dE/dY_lm and the radial term over the lanes four edges at a
-// time, and only these sums meet dY_lm/dx.
+// time, and only these sums meet dY_lm/dx.  Lanes sum in float32 up to 64 channels (with two
+// pairs per lane, each half of the warp has 64), whose forces are added in float64.
 // ---------------------------------------------------------------------------
 namespace {
 
 struct Rev0Smem {
   L0Stage st;
-  float S[kEdgeChunk][16];  // (dE/dr term, dE/dY_1 .. dE/dY_15) of the staged edges
   float2 buf[kSumEdges * 8 * kSumRow];
 };
 
@@ -375,13 +379,14 @@ __device__ __forceinline__ void layer0_rev_item(const DevModel& m, const EdgeIn&
   const bool local = i < in.n_local;  // a halo centre: layer 0 only
   LaneEdge ed;
   ed.load(m, in, min(e0 + part * cs + lane, e1 - 1));
-  // the lane's pairs cb + lane, cb + lane + 32 of a channel block; zero adjoints past the last
+  // the lane's pairs of a channel block: cb + lane, or cb + l, cb + l + 16 (l = lane in the first half
+  // of the warp, lane + 16 in the second); zero adjoints past the last
   float2 dA[NP][16];
   int cp[NP];
   auto load_dA = [&](int cb) {
 #pragma unroll
     for (int p = 0; p < NP; ++p) {
-      const int c = cb + 32 * p + lane;
+      const int c = cb + lane + (NP == 2 ? (lane & 16) + 16 * p : 0);
       cp[p] = c < C2 ? c : 0;
       const float2* a = reinterpret_cast<const float2*>(A0_adj + static_cast<size_t>(i) * 16 * C) + cp[p];
 #pragma unroll
@@ -396,7 +401,7 @@ __device__ __forceinline__ void layer0_rev_item(const DevModel& m, const EdgeIn&
     const bool active = lane < ne && ed.r < m.r_cut;
     int na;
     const int pos = stage_rows0(m, s.st, ed, ti, active, na);
-    bool staged = false;
+    double f[3] = {0.0, 0.0, 0.0};  // of this lane's edge
     for (int cb = 0; cb < C2 && na > 0; cb += 32 * NP) {
       if (C2 > 32 * NP) load_dA(cb);
       float4 c[NP][8];
@@ -407,8 +412,8 @@ __device__ __forceinline__ void layer0_rev_item(const DevModel& m, const EdgeIn&
 #pragma unroll
           for (int q = 0; q < 8; ++q) c[p][q] = __ldg(r + q * C2 + cp[p]);
       }
-      if (!staged) stage_Y0(s.st, ed, active, pos);
-      staged = true;
+      if (cb > 0) __syncwarp();  // (the last block's sums have been read)
+      stage_Y0(s.st, ed, active, pos);
       for (int a = 0; a < na; ++a) {
         const float4* r = m.spl0 + static_cast<size_t>(s.st.meta[min(a + 1, na - 1)].y) * 4 * C;
         const float x = __int_as_float(s.st.meta[a].x);
@@ -441,33 +446,38 @@ __device__ __forceinline__ void layer0_rev_item(const DevModel& m, const EdgeIn&
 #pragma unroll
         for (int v = 1; v < 8; ++v)
           t[kSumRow * v] = make_float2(dY[2 * v].x + dY[2 * v].y, dY[2 * v + 1].x + dY[2 * v + 1].y);
-        if (a % kSumEdges == kSumEdges - 1 || a == na - 1) {
-          float* out = &s.S[a - a % kSumEdges][0];
-          if (cb == 0)
-            sum_lanes<false>(s.buf, out, a % kSumEdges + 1);
-          else
-            sum_lanes<true>(s.buf, out, a % kSumEdges + 1);
+        if (a % kSumEdges == kSumEdges - 1 || a == na - 1)
+          sum_lanes<NP == 2, 2 * kRow0>(s.buf, &s.st.Y2[a - a % kSumEdges][0].x, a % kSumEdges + 1);
+      }
+      if (active) {
+        float Y[16], D[48];
+        sph_harm16<true>(ed.vx, ed.vy, ed.vz, Y, D);
+#pragma unroll
+        for (int p = 0; p < NP; ++p) {
+          float S[16];  // (dE/dr term, dE/dY_1 .. dE/dY_15)
+#pragma unroll
+          for (int v = 0; v < 4; ++v) {
+            const float4 w = *reinterpret_cast<const float4*>(&s.st.Y2[pos][8 * p + 2 * v]);
+            S[4 * v] = w.x;
+            S[4 * v + 1] = w.y;
+            S[4 * v + 2] = w.z;
+            S[4 * v + 3] = w.w;
+          }
+          const float d = __fdiv_rn(S[0], ed.r);
+          float fx = __fmul_rn(d, ed.vx), fy = __fmul_rn(d, ed.vy), fz = __fmul_rn(d, ed.vz);
+#pragma unroll
+          for (int q = 1; q < 16; ++q) {
+            fx = fmaf(S[q], D[q], fx);
+            fy = fmaf(S[q], D[16 + q], fy);
+            fz = fmaf(S[q], D[32 + q], fz);
+          }
+          f[0] += fx;
+          f[1] += fy;
+          f[2] += fz;
         }
       }
     }
     if (lane < ne) {  // this lane's edge
-      double f[3] = {0.0, 0.0, 0.0};
-      if (active) {
-        float Y[16], D[48];
-        sph_harm16<true>(ed.vx, ed.vy, ed.vz, Y, D);
-        const float* S = s.S[pos];
-        const float d = __fdiv_rn(S[0], ed.r);
-        float fx = __fmul_rn(d, ed.vx), fy = __fmul_rn(d, ed.vy), fz = __fmul_rn(d, ed.vz);
-#pragma unroll
-        for (int q = 1; q < 16; ++q) {
-          fx = fmaf(S[q], D[q], fx);
-          fy = fmaf(S[q], D[16 + q], fy);
-          fz = fmaf(S[q], D[32 + q], fz);
-        }
-        f[0] = fx;
-        f[1] = fy;
-        f[2] = fz;
-      }
       if (m.has_zbl && local) {  // node_forces -= xyz / r * dV_ZBL/dr (zbl.cpp:118-121)
         float V, dV;
         const double r = in.r[e];

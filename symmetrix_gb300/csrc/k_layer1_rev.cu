@@ -246,7 +246,7 @@ __device__ __forceinline__ void rev_group(const DevModel& m, const EdgeIn& in, c
         if constexpr (NR % 2) add_fixed(dst + (NR - 1) * C, hadj[NR - 1]);
         mt = mn;
         if (a % kSumEdges == kSumEdges - 1 || a == na - 1)
-          sum_lanes<false>(s.buf, &s.st.Y[a - a % kSumEdges][0], a % kSumEdges + 1);
+          sum_lanes<false, 16>(s.buf, &s.st.Y[a - a % kSumEdges][0], a % kSumEdges + 1);
       }
     }
     if (lane < ne) {  // this lane's edge: the sums against u and dY/dx

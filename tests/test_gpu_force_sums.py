@@ -1,5 +1,5 @@
 """Per-edge forces are summed in float64 above the float32 sums over lanes: the layer-1 adjoint's three
-instruction groups at L_max = 2."""
+instruction groups at L_max = 2, the layer-0 adjoint's 64-channel sums."""
 import numpy as np
 import pytest
 
@@ -47,3 +47,27 @@ def test_instruction_groups_of_l_max_2(engine_lib, tmp_path):
         assert np.abs(p).max() > 1e-3 and np.array_equal(p, p.astype(np.float32))
     err = np.abs(forces(group >= 0) - (parts[0] + parts[1] + parts[2])).max()
     assert err <= 1e-13 * max(np.abs(p).max() for p in parts)
+
+
+@pytest.mark.parametrize("C", [64, 96, 128, 256])
+def test_channels_of_layer_0(engine_lib, tmp_path, C):
+    """With the readout of the first layer alone the energy is linear in the layer-0 contraction's
+    channels: the edge forces are the float64 sum of those of each 64 channels by themselves."""
+    from symmetrix_gb300 import MACE
+    model = make_model(num_channels=C, species=("H", "C"), r_cut=4.0, L_max=1, num_knots=40, seed=4)
+    model["readout_2_weights_2"] = [0.0] * len(model["readout_2_weights_2"])
+    pos, L, species = random_box(40, 0.08, 0.9, 2, seed=6)
+    nl = neighbor_list(pos, 4.0, L)
+
+    def forces(channels):
+        d = dict(model)
+        d["M0_weights"] = {z: {LM: {k: c if int(k) in channels else [0.0] * len(c) for k, c in by_k.items()}
+                               for LM, by_k in w.items()} for z, w in model["M0_weights"].items()}
+        m = MACE(write_model(d, str(tmp_path / "m.json")))
+        m.compute_node_energies_forces(*edge_args(species, nl))
+        return np.array(m.node_forces)
+
+    parts = [forces(range(k, min(k + 64, C))) for k in range(0, C, 64)]
+    for p in parts:  # float32 sums
+        assert np.abs(p).max() > 1e-3 and np.array_equal(p, p.astype(np.float32))
+    assert np.abs(forces(range(C)) - sum(parts)).max() <= 1e-14 * max(np.abs(p).max() for p in parts)
