@@ -227,7 +227,7 @@ __global__ void __launch_bounds__(32, 12) k_layer0_fwd(DevModel m, EdgeIn in, fl
                                                        float* __restrict__ M0, float* __restrict__ zbl_e) {
   pdl_begin();
   __shared__ L0Stage st;
-  extern __shared__ float dyn[];
+  extern __shared__ __align__(16) float dyn[];
   const int ns = layer0_slices(CT > 0 ? CT : m.C), b = blockIdx.x;
   layer0_fwd_item<NLM, CT>(m, in, A0, M0, zbl_e, st, dyn, in.atom_at(b / ns), b % ns);
 }
@@ -253,7 +253,7 @@ __global__ void __launch_bounds__(32 * contract0_max_warps(NLM, CT, SPLIT),
     k_contract0_rev(DevModel m, const int* __restrict__ node_type, const int* __restrict__ order, const float* __restrict__ A0,
                     const float* __restrict__ M0_adj, float* __restrict__ A0_adj) {
   pdl_begin();
-  extern __shared__ float dyn[];
+  extern __shared__ __align__(16) float dyn[];
   const int C = CT > 0 ? CT : m.C, C2 = C >> 1, ns = layer0_slices(C);
   const int i = order ? order[blockIdx.x] : blockIdx.x;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;

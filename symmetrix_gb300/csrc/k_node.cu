@@ -112,7 +112,7 @@ __device__ __forceinline__ void node_tail_atom(const DevModel& m, const int* __r
                                                fix64* __restrict__ H1_adj, float* __restrict__ M1_adj_o,
                                                float* __restrict__ H2_adj_o, const float* __restrict__ zbl_e,
                                                double* __restrict__ energies, int N, int i) {
-  extern __shared__ float dyn[];
+  extern __shared__ __align__(16) float dyn[];
   const int C = m.C, k = threadIdx.x;
   const int nwarp = C >> 5, lane = k & 31, warp = k >> 5;
   const int ti = ntype[i];
