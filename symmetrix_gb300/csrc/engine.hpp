@@ -37,7 +37,9 @@ template <typename T>
 T* dalloc(size_t n) {
   void* p = nullptr;
   if (n == 0) n = 1;
-  check(cudaMalloc(&p, n * sizeof(T)), "cudaMalloc");
+  const cudaError_t e = cudaMalloc(&p, n * sizeof(T));
+  if (e != cudaSuccess) (void)cudaGetLastError();  // reported here, not by the next launch check
+  check(e, "cudaMalloc");
   return static_cast<T*>(p);
 }
 }  // namespace smx

@@ -52,12 +52,15 @@ struct NeighList {
     capN = ncell_cap = cell_atoms_cap = 0;
     capE = 0;
   }
+  // give the buffers back and forget them: growing may fail in between
+  template <typename... T>
+  static void drop(T*&... p) {
+    ((cudaFree(p), p = nullptr), ...);
+  }
   void reserve_nodes(int N, int ncell) {
     if (N > capN) {
-      for (int** p : {&cell, &num_neigh, &first, &last})
-        if (*p) cudaFree(*p);
-      if (posf) cudaFree(posf);
-      if (cellseg) cudaFree(cellseg);
+      capN = 0;
+      drop(cell, num_neigh, first, last, posf, cellseg);
       cell = dalloc<int>(N);
       num_neigh = dalloc<int>(N);
       first = dalloc<int>(N + 1);
@@ -68,16 +71,16 @@ struct NeighList {
       realloc_happened = true;
     }
     if (ncell + 1 > ncell_cap) {
-      for (int** p : {&cell_count, &cell_start, &cell_fill})
-        if (*p) cudaFree(*p);
+      ncell_cap = 0;
+      drop(cell_count, cell_start, cell_fill);
       cell_count = dalloc<int>(ncell + 1);
       cell_start = dalloc<int>(ncell + 2);
       cell_fill = dalloc<int>(ncell + 1);
       ncell_cap = ncell + 1;
     }
     if (N > cell_atoms_cap) {
-      for (int** p : {&cell_atoms, &cell_tmp})
-        if (*p) cudaFree(*p);
+      cell_atoms_cap = 0;
+      drop(cell_atoms, cell_tmp);
       cell_atoms = dalloc<int>(N);
       cell_tmp = dalloc<int>(N);
       cell_atoms_cap = N;
@@ -86,10 +89,8 @@ struct NeighList {
   void reserve_edges(long E_) {
     if (E_ <= capE) return;
     const long nE = static_cast<long>(E_ * 1.25) + 1024;
-    void* ps[] = {nidx, ntype_e, edge_i, rev, shift, xyz, r, forces, emap, pinv, nidx_p, ntype_p, xyz_p, r_p,
-                  forces_p};
-    for (void* p : ps)
-      if (p) cudaFree(p);
+    capE = 0;
+    drop(nidx, ntype_e, edge_i, rev, shift, xyz, r, forces, emap, pinv, nidx_p, ntype_p, xyz_p, r_p, forces_p);
     nidx = dalloc<int>(nE);
     ntype_e = dalloc<int>(nE);
     edge_i = dalloc<int>(nE);
