@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstdint>
 #include <cstring>
 #include <memory>
@@ -126,6 +127,13 @@ struct smx_engine {
         for (int t = 0; t < WT; ++t) b[(static_cast<size_t>(n) * WT + t) * K + k] = t == 0 ? hi : lo;
       }
     return reinterpret_cast<const __nv_bfloat16*>(upload(b));
+  }
+
+  // does every weight have a split: finite, and its bf16 rounding finite too?
+  static bool splittable(const std::vector<float>& W) {
+    for (float w : W)
+      if (!(std::fabs(w) <= 3.3895313892515355e38f)) return false;  // bf16's largest
+    return true;
   }
 
   // B operand of a float32 tensor-core GEMM from a row-major float [nrows][K] matrix: row n
@@ -289,7 +297,8 @@ struct smx_engine {
     // Float32 GEMMs on the tensor cores from 64 channels (two k-blocks or more in A1); at 32
     // the SIMT kernel is as fast or faster (5000 x 96 x 96: 12.2 us each).  A rule on the
     // model alone, so that a molecule gives the same bits in a batch and by itself.
-    tc32 = pm.C >= 64 && smx::umma_f32_supported(pm.C, pm.C);
+    tc32 = pm.C >= 64 && smx::umma_f32_supported(pm.C, pm.C) && splittable(pm.H1W);
+    for (int l = 0; l < 4; ++l) tc32 = tc32 && splittable(pm.A1W[l]);
     if (tc32) {
       const int C = pm.C;
       for (int L = 0; L <= pm.L_max; ++L) {

@@ -214,6 +214,8 @@ __global__ void __launch_bounds__(128, 1) k_umma_gemm(const __grid_constant__ Um
 // the mean loss back.  Error against float64 (2-norm; this kernel : the SIMT one, random
 // terms): K = 128 0.7e-7 : 2.0e-7, K = 384 1.0e-7 : 3.5e-7, K = 640 1.6e-7 : 4.5e-7; terms of
 // one sign: 0.8e-7 : 1.6e-7, 1.2e-7 : 2.9e-7, 2.2e-7 : 3.5e-7.
+// Rows with values that have no split (infinities, NaN, values above bf16's largest) give what
+// chains of FMAs give: see plain_tile.  The weights all have one (checked where they are laid out).
 // Eight warps read the float32 rows where the producers left them (the row map of the SIMT
 // GEMM) and split them into the swizzled operand layout, a k-block ahead in registers; one
 // thread of a ninth brings the weights' terms by TMA and issues the MMAs.
@@ -237,10 +239,18 @@ __device__ __forceinline__ uint32_t bf16_pair(float a, float b) {
   const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
   return *reinterpret_cast<const uint32_t*>(&v);
 }
-// the remainder of v after its leading term; an infinite v has none (v - v is NaN)
-__device__ __forceinline__ float rest(float v, float lead) {
-  const float d = v - lead;
-  return d == d ? d : 0.0f;
+// A tile with a value that has no split (an infinity, a NaN, or a finite value above bf16's
+// largest, whose leading term is infinite): its sums as the SIMT kernel forms them, chains of
+// FMAs over k on the float32 weights.
+__device__ __forceinline__ void plain_tile(const GemmSeg& g, const long* x_row, int m0, int n0, int NT, int tid) {
+  for (int t = tid; t < kTileM * NT; t += kF32Split) {
+    const int row = t / NT, n = n0 + t - row * NT, r = m0 + row;
+    if (x_row[row] < 0) continue;
+    const float *x = g.X + x_row[row], *w = g.B + n;
+    float s = 0.0f;
+    for (int k = 0; k < g.K; ++k) s = fmaf(__ldg(x + k), __ldg(w + static_cast<size_t>(k) * g.ncols), s);
+    g.Y[static_cast<long>(r / g.rpn) * g.y_ns + g.y_off + static_cast<long>(r % g.rpn) * g.y_rs + n] = s;
+  }
 }
 
 // Up to K = 128 two CTAs per SM with one stage each (96 KB, 256 TMEM columns) overlap one's
@@ -301,6 +311,7 @@ __global__ void __launch_bounds__(kF32Threads, 2) k_umma_f32(const __grid_consta
   };
   bool ok = true, issued = false;
   int loads = 0;
+  float low = 0.0f;  // sum of this thread's smallest terms
   if (tid < kF32Split) {
     load(0);
     for (int kb = 0; kb < KB; ++kb) {
@@ -321,9 +332,9 @@ __global__ void __launch_bounds__(kF32Threads, 2) k_umma_f32(const __grid_consta
           const uint2 w = make_uint2(bf16_pair(x.x, x.y), bf16_pair(x.z, x.w));
           *reinterpret_cast<uint2*>(a + t * kATerm) = w;
           if (t < 2)
-            x = make_float4(rest(x.x, bf16_lo(w.x)), rest(x.y, bf16_hi(w.x)), rest(x.z, bf16_lo(w.y)),
-                            rest(x.w, bf16_hi(w.y)));
+            x = make_float4(x.x - bf16_lo(w.x), x.y - bf16_hi(w.x), x.z - bf16_lo(w.y), x.w - bf16_hi(w.y));
         }
+        low += (x.x + x.y) + (x.z + x.w);  // a value without a split: NaN from here on
       }
       sm100::fence_async_shared();
       sm100::mbar_arrive(&split[s]);
@@ -379,8 +390,11 @@ __global__ void __launch_bounds__(kF32Threads, 2) k_umma_f32(const __grid_consta
   bool done = false;
   if (any_mma) done = sm100::mbar_wait(&bar_mma, 0);
   const int all_done = __syncthreads_and((done && all_ok) ? 1 : 0);
+  const int plain = __syncthreads_or(low == low ? 0 : 1);
   sm100::tc_fence_after();
-  if (all_done && tid < kF32Split) {
+  if (all_done && plain) {
+    if (tid < kF32Split) plain_tile(g, x_row, m0, n0, NT, tid);
+  } else if (all_done && tid < kF32Split) {
     // warp w reads the accumulator lanes 32 (w mod 4) and every other 32-column chunk; rows
     // leave through a swizzled 4 KB tile per warp, as in k_umma_gemm
     const int quarter = warp & 3, r = m0 + quarter * 32 + lane;

@@ -115,7 +115,7 @@ struct UmmaGemm {
 void launch_umma_gemms(const UmmaGemm* g, int n, unsigned* status, cudaStream_t s, bool test_timeout = false);
 
 // The batch's GEMMs in float32 on the tensor cores; B[q]: segment q's weights as three bf16
-// terms, [ncols][3][umma_f32_kp(K)], zero behind K (GemmSeg::B is not read).
+// terms, [ncols][3][umma_f32_kp(K)], zero behind K (GemmSeg::B serves rows that have no such split).
 bool umma_f32_supported(int K, int ncols);
 int umma_f32_kp(int K);
 void launch_umma_f32(const GemmBatch& b, const __nv_bfloat16* const* B, unsigned* status, cudaStream_t s);
