@@ -205,15 +205,21 @@ __global__ void __launch_bounds__(128, 1) k_umma_gemm(const __grid_constant__ Um
 // Float32 GEMMs:  Y[rows, N] = X[rows, K] . B[N, K]^T with float32 X, split in the kernel.
 //
 // x = x0 + x1 + x2 and w = w0 + w1 + w2 in bf16 (24 bits: what float32 holds), six products:
-// x0 w0 into one accumulator, x0 w1, x1 w0, x1 w1, x0 w2, x2 w0 into another that the
-// epilogue adds, so that the small products are not rounded at the size of the large one.
-// The tensor core's running sum is cut towards zero at every step, measured as a shrinking of
-// the result by 1.2e-8 per 16-wide step for terms of random sign (2e-8 for terms of one
-// sign), where a chain of FMAs errs either way and grows with the root of K.  So above
-// K = 128 the k-blocks alternate between two accumulators of x0 w0, and the epilogue gives
-// the mean loss back.  Error against float64 (2-norm; this kernel : the SIMT one, random
-// terms): K = 128 0.7e-7 : 2.0e-7, K = 384 1.0e-7 : 3.5e-7, K = 640 1.6e-7 : 4.5e-7; terms of
-// one sign: 0.8e-7 : 1.6e-7, 1.2e-7 : 2.9e-7, 2.2e-7 : 3.5e-7.
+// x0 w0 into accumulators of its own, x0 w1, x1 w0, x1 w1, x0 w2, x2 w0 into another that the
+// epilogue adds, so that the small products are not rounded at the size of the large one (the
+// products left out are 2^-27 of x w, root mean square, and below 2^-23; with x1 w2 and x2 w1,
+// 4096 x 5 x 384 x 128 35 -> 42 us).  The tensor core's running sum is cut towards zero at every
+// 16-wide step, where a chain of FMAs errs either way and grows with the root of K, so the steps
+// go round three accumulators of x0 w0.  (One, for two CTAs per SM up to K = 128: the 4096-atom
+// evaluation 1.9% shorter, its forces' error 3.3e-7 -> 4.1e-7.  Giving back the mean loss,
+// 1.2e-8 per step, makes exact sums and rows of few terms wrong by up to 4 ulp.)  Error against
+// float64, 2-norm, this kernel : the SIMT one, in 1e-8 (rows of random sign; of one sign; with
+// one nonzero; with elements over 12 orders of magnitude; sums of integers are exact in both):
+//   K =  64, N =  64    4.8 : 14.4    4.8 : 12.1   2.6 : 2.6    7.1 :  9.2
+//   K = 128, N = 128    6.1 : 20.3    6.4 : 16.0   2.6 : 2.6    8.8 : 12.3
+//   K = 384, N = 128   12.6 : 35.2   16.4 : 29.0   2.6 : 2.5   18.6 : 21.0
+//   K = 640, N = 128   19.5 : 45.3   30.7 : 34.7   2.6 : 2.6   29.1 : 27.7
+//   K = 768, N = 256   23.3 : 49.3   37.3 : 40.7   2.6 : 2.5   34.2 : 30.1
 // Rows with values that have no split (infinities, NaN, values above bf16's largest) give what
 // chains of FMAs give: see plain_tile.  The weights all have one (checked where they are laid out).
 // Eight warps read the float32 rows where the producers left them (the row map of the SIMT
@@ -230,7 +236,7 @@ struct F32GroupDev {
 };
 constexpr int kF32Split = 256;                // threads that split X and store Y
 constexpr int kF32Threads = kF32Split + 32;   // and a warp whose first lane issues TMA and MMAs
-constexpr float kStepLoss = 1.2e-8f;  // mean relative loss of an accumulator per MMA step
+constexpr int kF32Mains = 3;          // accumulators of x0 w0
 constexpr uint32_t kATerm = kTileM * kBoxK * 2;  // bytes of one X term of a k-block
 
 __device__ __forceinline__ float bf16_lo(uint32_t p) { return __uint_as_float(p << 16); }
@@ -253,8 +259,8 @@ __device__ __forceinline__ void plain_tile(const GemmSeg& g, const long* x_row, 
   }
 }
 
-// Up to K = 128 two CTAs per SM with one stage each (96 KB, 256 TMEM columns) overlap one's
-// splitting and stores with the other's MMAs; above, one CTA with two stages and 512 columns.
+// Tiles of 64 columns up to K = 128: two CTAs per SM with one stage each (72 KB, 256 TMEM columns)
+// overlap one's splitting and stores with the other's MMAs; otherwise one CTA with two stages.
 __global__ void __launch_bounds__(kF32Threads, 2) k_umma_f32(const __grid_constant__ F32GroupDev grp,
                                                              unsigned* status) {
   pdl_begin();
@@ -368,7 +374,8 @@ __global__ void __launch_bounds__(kF32Threads, 2) k_umma_f32(const __grid_consta
                            sm100::sdesc_sw128(w0 + wt * b_bytes + k * 32), idesc, acc);
         };
         const uint32_t corr = tmem + seg.mains * NT;
-        mma(tmem + (kb % seg.mains) * NT, 0, 0, kb >= seg.mains || k != 0 ? 1u : 0u);
+        const int step = kb * (kBoxK / 16) + k;
+        mma(tmem + (step % seg.mains) * NT, 0, 0, step >= seg.mains ? 1u : 0u);
         mma(corr, 0, 2, (kb | k) != 0 ? 1u : 0u);
         mma(corr, 2, 0, 1u);
         mma(corr, 1, 1, 1u);
@@ -404,15 +411,13 @@ __global__ void __launch_bounds__(kF32Threads, 2) k_umma_f32(const __grid_consta
     float* stg = reinterpret_cast<float*>(smem) + warp * 32 * 32;
     const int sub = lane >> 3, c4 = lane & 7;
     const uint32_t t0 = tmem + (static_cast<uint32_t>(quarter * 32) << 16);
-    const float loss = kStepLoss * static_cast<float>((KB + seg.mains - 1) / seg.mains * (kBoxK / 16));
     for (int c0 = (warp >> 2) * 32; c0 < NT; c0 += 64) {
-      // mains + (corrections + loss mains)
       float a[32], b[32];
       sm100::tmem_ld32(t0 + static_cast<uint32_t>(seg.mains * NT + c0), a);
       for (int w = seg.mains - 1; w >= 0; --w) {
         sm100::tmem_ld32(t0 + static_cast<uint32_t>(w * NT + c0), b);
 #pragma unroll
-        for (int q = 0; q < 32; ++q) a[q] = b[q] + fmaf(loss, b[q], a[q]);
+        for (int q = 0; q < 32; ++q) a[q] += b[q];
       }
 #pragma unroll
       for (int q = 0; q < 8; ++q)
@@ -491,8 +496,8 @@ bool umma_supported(int K, int NT, int terms) {
 
 namespace {
 
-// x0 w0 accumulators, and ring stages (see k_umma_f32)
-int f32_mains(int K) { return K > 2 * kBoxK ? 2 : 1; }
+// ring stages (see k_umma_f32; two also where one CTA's TMEM columns are more than half)
+int f32_stages(int K, int NT) { return K > 2 * kBoxK || (kF32Mains + 1) * NT > 256 ? 2 : 1; }
 // N-tile: the widest of 128, 96, 64, 32 that divides the columns
 int f32_tile_n(int ncols) {
   for (int nt : {128, 96, 64})
@@ -521,7 +526,8 @@ void launch_umma_f32(const GemmBatch& b, const __nv_bfloat16* const* B, unsigned
     F32SegDev& d = grp.s[used++];
     d.g = g;
     d.NT = f32_tile_n(g.ncols);
-    d.mains = d.stages = f32_mains(g.K);
+    d.mains = kF32Mains;
+    d.stages = f32_stages(g.K, d.NT);
     d.tb = make_map(B[q], g.ncols, 3 * umma_f32_kp(g.K), d.NT);
     d.tiles_m = (g.rows + kTileM - 1) / kTileM;
     d.tiles_n = g.ncols / d.NT;

@@ -71,3 +71,66 @@ def test_weights_beyond_bf16(engine_lib, tmp_path):
                                              for LM, by_k in by.items()} for z, by in model["M0_weights"].items()}}
         m = MACE(write_model(model, str(tmp_path / "m.json")))
         compare(m, a)
+
+
+@pytest.mark.parametrize("channels,L_max", [(64, 1), (128, 1), (160, 1), (128, 2)])
+def test_single_products_and_one_sign(engine_lib, tmp_path, channels, L_max):
+    """Columns with one nonzero weight, a power of two: the product is exact in float32, and so are its
+    split terms and their sums.  Then rows of one sign."""
+    from symmetrix_gb300 import MACE
+    a = system()
+    n, N = channels, a[0]
+    model = make_model(num_channels=n, species=("H", "C"), r_cut=4.0, L_max=L_max, num_knots=40, seed=4)
+    rng = np.random.default_rng(3)
+    ne = [model["Phi1_l"].count(l) for l in range(4)]
+
+    def one_per_column(K):
+        W = np.zeros((K, n))
+        W[rng.permutation(K)[:n], np.arange(n)] = rng.choice([-1, 1], n) * 2.0 ** rng.integers(-3, 4, n)
+        return W.astype(np.float32)
+
+    H1W = [one_per_column(n) for _ in range(L_max + 1)]
+    A1W = [one_per_column(k * n) for k in ne]
+    d = {**model, "H1_weights": np.concatenate([w.ravel() for w in H1W]).tolist(),
+         "A1_weights": [w.ravel().tolist() for w in A1W]}
+    m = MACE(write_model(d, str(tmp_path / "m.json")))
+    m.compute_node_energies_forces(*a)
+    get = {s: m.stage(s).reshape(N, -1, n) for s in ("M0", "H1", "H1_adj", "M0_adj", "Phi1", "A1", "A1_adj", "Phi1_adj")}
+
+    def products(got, x, W):
+        want = x @ W.astype(np.float64)
+        assert np.abs(want).max() > 0 and np.array_equal(got, want)
+
+    for L in range(L_max + 1):
+        r = slice(L * L, (L + 1) ** 2)
+        products(get["H1"][:, r], get["M0"][:, r], H1W[L])
+        products(get["M0_adj"][:, r], get["H1_adj"][:, r], H1W[L].T)
+    at = 0
+    for l in range(4):
+        rows, r = slice(at, at + (2 * l + 1) * ne[l]), slice(l * l, (l + 1) ** 2)
+        at += (2 * l + 1) * ne[l]
+        products(get["A1"][:, r], get["Phi1"][:, rows].reshape(N, 2 * l + 1, ne[l] * n), A1W[l])
+        products(get["Phi1_adj"][:, rows].reshape(N, 2 * l + 1, ne[l] * n), get["A1_adj"][:, r], A1W[l].T)
+
+    # one sign: weights that follow the signs of one node's rows, column by column
+    node = 17
+    sign = np.sign(get["Phi1"][node])
+    at, W1 = 0, []
+    for l in range(4):
+        x = sign[at:at + (2 * l + 1) * ne[l]].reshape(2 * l + 1, ne[l] * n)[0]
+        W1.append((np.abs(rng.normal(size=(ne[l] * n, n))) * x[:, None]).astype(np.float32))
+        at += (2 * l + 1) * ne[l]
+    m = MACE(write_model({**d, "A1_weights": [w.ravel().tolist() for w in W1]}, str(tmp_path / "m.json")))
+    m.compute_node_energies_forces(*a)
+    A1, Phi1 = m.stage("A1").reshape(N, 16, n), m.stage("Phi1").reshape(N, -1, n)
+    at = 0
+    for l in range(4):
+        K = ne[l] * n
+        x = Phi1[node, at:at + (2 * l + 1) * ne[l]].reshape(2 * l + 1, K)[0]
+        at += (2 * l + 1) * ne[l]
+        want = x @ W1[l].astype(np.float64)
+        assert (np.sign(x) * x @ np.abs(W1[l].astype(np.float64)) == np.abs(want)).all()
+        # an accumulator is cut by at most one unit of 2^-23 per 16-wide step, three share the steps
+        # (and one k-block is 4 steps)
+        steps = -(-4 * -(-K // 64) // 3)
+        assert (np.abs(A1[node, l * l] - want) <= (steps + 2) * 2.0 ** -23 * np.abs(want)).all()
