@@ -450,6 +450,11 @@ struct smx_engine {
   // test of the timeout path: this many of the next tensor-core GEMM launches issue no
   // load, so their bounded wait gives up (option "test_gemm_timeout")
   int test_gemm_timeout = 0;
+  bool test_timeout_due() {
+    if (test_gemm_timeout == 0) return false;
+    --test_gemm_timeout;
+    return true;
+  }
 
   void tc_apply(const TcCfg& c, smx::UmmaGemm* g, int ng, bool tile_n) const {
     for (int q = 0; q < ng; ++q) {
@@ -509,7 +514,7 @@ struct smx_engine {
   void gemm32(const smx::GemmBatch& b, const __nv_bfloat16* const* B, cudaStream_t s) {
     if (b.n == 0) return;
     if (tc32)
-      smx::launch_umma_f32(b, B, status_dev, s);
+      smx::launch_umma_f32(b, B, status_dev, s, test_timeout_due());
     else
       smx::launch_gemm(b, s);
   }
@@ -533,9 +538,7 @@ struct smx_engine {
       if (cs == cudaStreamCaptureStatusNone) tc_tune(gid, g, ng, tile_n, s);
     }
     tc_apply(tc_cfg[gid], g, ng, tile_n);
-    const bool test = test_gemm_timeout > 0;
-    if (test) --test_gemm_timeout;
-    smx::launch_umma_gemms(g, ng, status_dev, s, test);
+    smx::launch_umma_gemms(g, ng, status_dev, s, test_timeout_due());
   }
 
   // canonical and padded Clebsch-Gordan tables (option "cg_padded" 0 switches the kernels to

@@ -233,6 +233,8 @@ struct F32SegDev {
 };
 struct F32GroupDev {
   F32SegDev s[4];
+  int skip_loads;  // test of the error path, as in UmmaGroupDev
+  uint64_t wait_ns;
 };
 constexpr int kF32Split = 256;                // threads that split X and store Y
 constexpr int kF32Threads = kF32Split + 32;   // and a warp whose first lane issues TMA and MMAs
@@ -322,7 +324,7 @@ __global__ void __launch_bounds__(kF32Threads, 2) k_umma_f32(const __grid_consta
     load(0);
     for (int kb = 0; kb < KB; ++kb) {
       const int s = kb % S;
-      if (kb >= S && !sm100::mbar_wait(&empty[s], ((kb / S) - 1) & 1)) {  // the stage's last MMAs are done
+      if (kb >= S && !sm100::mbar_wait(&empty[s], ((kb / S) - 1) & 1, grp.wait_ns)) {  // the stage's last MMAs are done
         ok = false;
         break;
       }
@@ -355,15 +357,16 @@ __global__ void __launch_bounds__(kF32Threads, 2) k_umma_f32(const __grid_consta
         sm100::tma_load_2d(st + u * b_bytes, &seg.tb, u * Kp + kb * kBoxK, n0, &full[kb % S]);
       ++loads;
     };
-    for (int kb = 0; kb < KB && kb < S; ++kb) weights(kb);
+    for (int kb = 0; kb < KB && kb < S && !grp.skip_loads; ++kb) weights(kb);
     for (int kb = 0; kb < KB; ++kb) {
       const int s = kb % S;
       // (with one stage: this k-block's weights, once the last one's MMAs are done)
       if (S == 1 && kb > 0) {
-        if (!(ok = sm100::mbar_wait(&empty[0], (kb - 1) & 1))) break;
+        if (!(ok = sm100::mbar_wait(&empty[0], (kb - 1) & 1, grp.wait_ns))) break;
         weights(kb);
       }
-      ok = sm100::mbar_wait(&full[s], (kb / S) & 1) && sm100::mbar_wait(&split[s], (kb / S) & 1);
+      ok = sm100::mbar_wait(&full[s], (kb / S) & 1, grp.wait_ns) &&
+           sm100::mbar_wait(&split[s], (kb / S) & 1, grp.wait_ns);
       if (!ok) break;
       sm100::tc_fence_after();
       const uint32_t x0 = sm100::smem_u32(smem + static_cast<size_t>(s) * stage_bytes), w0 = x0 + 3 * kATerm;
@@ -386,7 +389,7 @@ __global__ void __launch_bounds__(kF32Threads, 2) k_umma_f32(const __grid_consta
       issued = true;
       // while these run: the weights that follow those of the k-block before
       if (S > 1 && kb > 0 && kb - 1 + S < KB) {
-        if (!(ok = sm100::mbar_wait(&empty[(kb - 1) % S], ((kb - 1) / S) & 1))) break;
+        if (!(ok = sm100::mbar_wait(&empty[(kb - 1) % S], ((kb - 1) / S) & 1, grp.wait_ns))) break;
         weights(kb - 1 + S);
       }
     }
@@ -513,9 +516,12 @@ bool umma_f32_supported(int K, int ncols) { return K > 0 && K % 32 == 0 && ncols
 
 int umma_f32_kp(int K) { return (K + kBoxK - 1) / kBoxK * kBoxK; }
 
-void launch_umma_f32(const GemmBatch& b, const __nv_bfloat16* const* B, unsigned* status, cudaStream_t s) {
+void launch_umma_f32(const GemmBatch& b, const __nv_bfloat16* const* B, unsigned* status, cudaStream_t s,
+                     bool test_timeout) {
   F32GroupDev grp;
   std::memset(&grp, 0, sizeof(grp));
+  grp.skip_loads = test_timeout ? 1 : 0;
+  grp.wait_ns = test_timeout ? 2000000ull : sm100::kWaitLimitNs;  // 2 ms when testing
   long gx = 0;
   size_t smem = 0;
   int used = 0;

@@ -118,7 +118,8 @@ void launch_umma_gemms(const UmmaGemm* g, int n, unsigned* status, cudaStream_t 
 // terms, [ncols][3][umma_f32_kp(K)], zero behind K (GemmSeg::B serves rows that have no such split).
 bool umma_f32_supported(int K, int ncols);
 int umma_f32_kp(int K);
-void launch_umma_f32(const GemmBatch& b, const __nv_bfloat16* const* B, unsigned* status, cudaStream_t s);
+void launch_umma_f32(const GemmBatch& b, const __nv_bfloat16* const* B, unsigned* status, cudaStream_t s,
+                     bool test_timeout = false);
 
 // k_md.cu
 void launch_wrap(int N, double3 box, int3 periodic, double* pos, cudaStream_t s);
