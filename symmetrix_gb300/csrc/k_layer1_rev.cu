@@ -277,7 +277,8 @@ __device__ __forceinline__ void rev_group(const DevModel& m, const EdgeIn& in, c
             *o = make_float2(f[v], 0.0f);
           } else {
             const float2 a = *o, s = two_sum(a.x, f[v]);
-            *o = make_float2(s.x, a.y + s.y);
+            const float low = a.y + s.y;  // (undefined beside an infinity)
+            *o = make_float2(s.x, low == low ? low : 0.0f);
           }
         }
       }

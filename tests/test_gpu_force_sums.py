@@ -1,5 +1,5 @@
 """Per-edge forces are summed in float64 above the float32 sums over lanes: the layer-1 adjoint's three
-instruction groups at L_max = 2, the layer-0 adjoint's 64-channel sums."""
+instruction groups at L_max = 2 (an infinite force stays one), the layer-0 adjoint's 64-channel sums."""
 import numpy as np
 import pytest
 
@@ -47,6 +47,37 @@ def test_instruction_groups_of_l_max_2(engine_lib, tmp_path):
         assert np.abs(p).max() > 1e-3 and np.array_equal(p, p.astype(np.float32))
     err = np.abs(forces(group >= 0) - (parts[0] + parts[1] + parts[2])).max()
     assert err <= 1e-13 * max(np.abs(p).max() for p in parts)
+
+
+@pytest.mark.parametrize("L_max", [1, 2])
+def test_infinite_layer_1_forces(engine_lib, tmp_path, L_max):
+    """One channel's scalar row whose product with H1 is beyond float32: the edge forces are infinite,
+    with the signs of a finite row's, at L_max = 2 through the sum of the three groups too."""
+    from symmetrix_gb300 import MACE
+    C, c = 32, 5
+    model = make_model(num_channels=C, species=("H", "C", "O"), r_cut=4.0, L_max=L_max, num_knots=40, seed=4)
+    assert (model["Phi1_l1"][0], model["Phi1_l2"][0], model["Phi1_l"][0]) == (0, 0, 0)  # row 0
+    m = MACE(write_model(model, str(tmp_path / "m.json")))
+    pos, L, species = random_box(40, 0.08, 0.9, 3, seed=6)
+    a = edge_args(species, neighbor_list(pos, 4.0, L))
+    n = len(species)
+    m.compute_node_energies_forces(*a)
+    H1, dPhi1 = np.zeros(m.stage("H1").shape, np.float32), np.zeros(m.stage("Phi1_adj").shape, np.float32)
+    H1.reshape(n, -1, C)[:, 0, c] = 1.0
+    dPhi1.reshape(n, -1, C)[:, 0, c] = 1.0
+    m.compute_R1(n, species, a[2], a[4], a[6])
+    m.compute_Y(a[5])
+
+    def forces(scale):
+        m.set_stage("H1", H1 * np.float32(scale))
+        m.set_stage("Phi1_adj", dPhi1 * np.float32(scale))
+        m.reverse_Phi1(n, a[2], a[3], a[5], a[6], True, True)
+        return np.array(m.node_forces)
+
+    want = forces(1.0)
+    big = np.abs(want) > 1e-12
+    assert big.any()
+    assert np.array_equal(forces(1e30)[big], np.sign(want[big]) * np.inf)
 
 
 @pytest.mark.parametrize("C", [64, 96, 128, 256])
