@@ -106,8 +106,8 @@ struct smx_engine {
 
   // Buffers of the atom-level calls (neighbour list, atom arrays; md.cu), kept between calls
   // like the workspace above: a call allocated and freed some thirty of them, 0.3 ms of a
-  // 0.5 ms evaluation of 500 atoms.  Given back with the engine, or after a call that leaves
-  // more than AtomsWorkspace::kKeepBytes in them.
+  // 0.5 ms evaluation of 500 atoms.  Given back with the engine, after a call that leaves more
+  // than AtomsWorkspace::kKeepBytes in them, or when the workspace above does not fit beside them.
   std::shared_ptr<void> atoms_ws;
 
   // B operand of a tensor-core GEMM from a row-major float [nrows][K] matrix: row n
@@ -361,6 +361,17 @@ struct smx_engine {
   void reserve(long N, long E) {
     if (first && N <= capN && E <= capE) return;
     const long nN = std::max(N, capN), nE = std::max(E, capE);
+    try {
+      allocate(nN, nE);
+    } catch (const CudaError&) {  // once more without the atom-level calls' buffers, unless one is running
+      if (atoms_ws.use_count() != 1) throw;
+      free_workspace();
+      atoms_ws.reset();
+      allocate(nN, nE);
+    }
+  }
+
+  void allocate(long nN, long nE) {
     free_workspace();
     const long C = dm.C;
     A0 = dalloc<float>(nN * 16 * C);

@@ -426,7 +426,8 @@ int compute_atoms_impl(smx_engine* eng, int n_atoms, const double* positions, co
       return SMX_OK;
     }
     if (!eng->atoms_ws) eng->atoms_ws = std::make_shared<AtomsWorkspace>();
-    AtomsWorkspace& ws = *static_cast<AtomsWorkspace*>(eng->atoms_ws.get());
+    const std::shared_ptr<void> held = eng->atoms_ws;  // in use: the engine's workspace grows beside it
+    AtomsWorkspace& ws = *static_cast<AtomsWorkspace*>(held.get());
     smx_md& md = ws.md;
     ws.reserve(n_atoms);
     md.eng = eng;
