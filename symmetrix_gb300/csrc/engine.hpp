@@ -68,7 +68,7 @@ struct smx_engine {
   const __nv_bfloat16 *W_H1 = nullptr, *W_M0adj = nullptr, *W_A1[4] = {}, *W_Phi1adj[4] = {};
   bool tc_H1 = false, tc_A1[4] = {}, tc_Phi1adj[4] = {};
   // float32 tensor-core GEMMs: three bf16 terms per weight (see f32_operand)
-  const __nv_bfloat16 *W32_H1[3] = {}, *W32_M0adj[3] = {}, *W32_A1[4] = {}, *W32_Phi1adj[4] = {};
+  smx::F32Weights W32_H1[3] = {}, W32_M0adj[3] = {}, W32_A1[4] = {}, W32_Phi1adj[4] = {};
   bool tc32 = false;
   // 1: bf16 operands; 2: weights split hi + lo (x_hi W_hi + x_hi W_lo); 3: both
   // split (x_hi W_hi + x_lo W_hi + x_hi W_lo: close to float32 operand precision)
@@ -129,24 +129,47 @@ struct smx_engine {
     return reinterpret_cast<const __nv_bfloat16*>(upload(b));
   }
 
-  // does every weight have a split: finite, and its bf16 rounding finite too?
+  // does every weight have a split: finite, and its grid's end too (f32_operand)?
   static bool splittable(const std::vector<float>& W) {
     for (float w : W)
-      if (!(std::fabs(w) <= 3.3895313892515355e38f)) return false;  // bf16's largest
+      if (!(std::fabs(w) < 1.7014118346046923e38f)) return false;  // 2^127
     return true;
   }
 
-  // B operand of a float32 tensor-core GEMM from a row-major float [nrows][K] matrix: row n
-  // holds (W0 | W1 | W2), each the bf16 rounding of what the ones before it leave, padded
+  // B operand of a float32 tensor-core GEMM from a row-major float [nrows][K] matrix, its columns
+  // divided by the powers of two above their largest values (relative to the matrix's; 0: none):
+  // row n holds (W0 | W1 | W2), W0 rounded to 2^-7 of the power of two above the row's largest
+  // value (k_umma_f32's grid), the others the bf16 rounding of what the ones before leave, padded
   // with zeros to whole k-blocks
-  const __nv_bfloat16* f32_operand(const float* W, int nrows, int K) {
+  smx::F32Weights f32_operand(const float* W, int nrows, int K) {
     const size_t Kp = smx::umma_f32_kp(K);
-    std::vector<uint16_t> b(nrows * 3 * Kp, 0);
+    auto above = [](float v) {  // v < 2^above
+      int e = 0;
+      std::frexp(v, &e);
+      return e;
+    };
+    std::vector<float> most(K, 0.0f), scale(Kp, 0.0f);
     for (int n = 0; n < nrows; ++n)
+      for (int k = 0; k < K; ++k) most[k] = std::max(most[k], std::fabs(W[static_cast<size_t>(n) * K + k]));
+    const int top = above(*std::max_element(most.begin(), most.end()));
+    std::vector<int> shift(K, 0);
+    for (int k = 0; k < K; ++k)
+      if (most[k] > 0.0f) {
+        shift[k] = std::max(above(most[k]) - top, -120);
+        scale[k] = std::ldexp(1.0f, shift[k]);
+      }
+    std::vector<uint16_t> b(nrows * 3 * Kp, 0);
+    std::vector<float> row(K);
+    for (int n = 0; n < nrows; ++n) {
+      for (int k = 0; k < K; ++k) row[k] = std::ldexp(W[static_cast<size_t>(n) * K + k], -shift[k]);
+      float big = 0.0f;
+      for (float w : row) big = std::max(big, std::fabs(w));
+      const int e = above(big);
       for (int k = 0; k < K; ++k) {
-        float w = W[static_cast<size_t>(n) * K + k];
+        float w = row[k];
         for (int t = 0; t < 3; ++t) {
-          const uint16_t h = smx::bf16_bits(w);
+          const float v = t > 0 ? w : static_cast<float>(std::ldexp(std::rint(std::ldexp(static_cast<double>(w), 7 - e)), e - 7));
+          const uint16_t h = smx::bf16_bits(v);
           b[(static_cast<size_t>(n) * 3 + t) * Kp + k] = h;
           const uint32_t hu = static_cast<uint32_t>(h) << 16;
           float hf;
@@ -154,7 +177,8 @@ struct smx_engine {
           w -= hf;
         }
       }
-    return reinterpret_cast<const __nv_bfloat16*>(upload(b));
+    }
+    return {reinterpret_cast<const __nv_bfloat16*>(upload(b)), upload(scale)};
   }
 
   void setup_tc_weights() {
@@ -521,11 +545,11 @@ struct smx_engine {
     tc_tuned_us[gid] = best * 1000.0f / 3.0f;
   }
 
-  // float32 GEMMs: on the tensor cores (B: the segments' split weights) or the SIMT kernel
-  void gemm32(const smx::GemmBatch& b, const __nv_bfloat16* const* B, cudaStream_t s) {
+  // float32 GEMMs: on the tensor cores (W: the segments' split weights) or the SIMT kernel
+  void gemm32(const smx::GemmBatch& b, const smx::F32Weights* W, cudaStream_t s) {
     if (b.n == 0) return;
     if (tc32)
-      smx::launch_umma_f32(b, B, status_dev, s, test_timeout_due());
+      smx::launch_umma_f32(b, W, status_dev, s, test_timeout_due());
     else
       smx::launch_gemm(b, s);
   }
@@ -802,15 +826,15 @@ struct smx_engine {
         }
       run_tc(1, g, ng, true, s);
       smx::GemmBatch b{};
-      const __nv_bfloat16* B[4] = {};
+      smx::F32Weights W[4] = {};
       for (int l = 0; l < 4; ++l)
         if (dm.num_e[l] > 0 && !tc_A1[l]) {
-          B[b.n] = W32_A1[l];
+          W[b.n] = W32_A1[l];
           b.s[b.n++] = seg_rows(Phi1, A1, dm.A1W[l], N1, 2 * l + 1, dm.num_e[l] * C, C,
                                 static_cast<long>(dm.n_lme) * C, dm.lme_off[l] * C, dm.num_e[l] * C,
                                 16L * C, l * l * C, C);
         }
-      gemm32(b, B, s);
+      gemm32(b, W, s);
     }
     mark(4, s);
     smx::launch_node_tail(dm, in.node_type, N1, A1, H1, M1, H2, A1adj_out, H1_adj_fx, M1_adj, H2_adj,
@@ -831,14 +855,14 @@ struct smx_engine {
         }
       run_tc(2, g, ng, true, s);
       smx::GemmBatch b{};
-      const __nv_bfloat16* B[4] = {};
+      smx::F32Weights W[4] = {};
       for (int l = 0; l < 4; ++l)
         if (dm.num_e[l] > 0 && !tc_Phi1adj[l]) {
-          B[b.n] = W32_Phi1adj[l];
+          W[b.n] = W32_Phi1adj[l];
           b.s[b.n++] = seg_rows(A1_adj, Phi1_adj, dm.A1W_T[l], N1, 2 * l + 1, C, dm.num_e[l] * C, 16L * C, l * l * C,
                                 C, static_cast<long>(dm.n_lme) * C, dm.lme_off[l] * C, dm.num_e[l] * C);
         }
-      gemm32(b, B, s);
+      gemm32(b, W, s);
     }
     mark(6, s);
     smx::launch_layer1_rev(dm, in1, H1, Phi1_adj, H1_adj_fx, f1, s);

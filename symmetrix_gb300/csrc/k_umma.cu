@@ -204,23 +204,29 @@ __global__ void __launch_bounds__(128, 1) k_umma_gemm(const __grid_constant__ Um
 // ---------------------------------------------------------------------------
 // Float32 GEMMs:  Y[rows, N] = X[rows, K] . B[N, K]^T with float32 X, split in the kernel.
 //
-// x = x0 + x1 + x2 and w = w0 + w1 + w2 in bf16 (24 bits: what float32 holds), six products:
-// x0 w0 into accumulators of its own, x0 w1, x1 w0, x1 w1, x0 w2, x2 w0 into another that the
-// epilogue adds, so that the small products are not rounded at the size of the large one (the
-// products left out are 2^-27 of x w, root mean square, and below 2^-23; with x1 w2 and x2 w1,
-// 4096 x 5 x 384 x 128 35 -> 42 us).  The tensor core's running sum is cut towards zero at every
-// 16-wide step, where a chain of FMAs errs either way and grows with the root of K, so the steps
-// go round three accumulators of x0 w0.  (One, for two CTAs per SM up to K = 128: the 4096-atom
-// evaluation 1.9% shorter, its forces' error 3.3e-7 -> 4.1e-7.  Giving back the mean loss,
-// 1.2e-8 per step, makes exact sums and rows of few terms wrong by up to 4 ulp.)  Error against
-// float64, 2-norm, this kernel : the SIMT one, in 1e-8 (rows of random sign; of one sign; with
+// x = x0 + x1 + x2 and w = w0 + w1 + w2 in bf16, eight products (all but x2 w2, 2^-34).  The tensor
+// core's running sum is cut towards zero at every 16-wide step: what it loses has the sum's sign,
+// so it stays in sums over many results (total energies), where a chain of FMAs errs either way.
+// So the leading terms lie on a grid: x0 is x rounded to 2^-7 of the power of two above the largest
+// of its row's k-block, w0 the same over its row of B, both integers of at most 8 bits there.  Their
+// products add exactly up to K = 1024 (14 + 10 bits of the accumulator's 24; where a row's k-blocks
+// differ, their ratio comes out of the 9 or so bits that sums of either sign leave free), and the
+// other seven, 2^-7 and less of them, go into a second accumulator that the epilogue adds: what is
+// cut there is 2^-7 of what it was.  x1 and x2 hold what the grid leaves to 2^-26 of the block's
+// largest; so that this is 2^-26 of the largest contribution whatever the channels' units, x_k is
+// taken times the power of two above B's largest |w_nk| over n, and w_nk divided by it.
+// Error against float64, 2-norm, this kernel : the SIMT one, in 1e-8 (random rows; of one sign; with
 // one nonzero; with elements over 12 orders of magnitude; sums of integers are exact in both):
-//   K =  64, N =  64    4.8 : 14.4    4.8 : 12.1   2.6 : 2.6    7.1 :  9.2
-//   K = 128, N = 128    6.1 : 20.3    6.4 : 16.0   2.6 : 2.6    8.8 : 12.3
-//   K = 384, N = 128   12.6 : 35.2   16.4 : 29.0   2.6 : 2.5   18.6 : 21.0
-//   K = 640, N = 128   19.5 : 45.3   30.7 : 34.7   2.6 : 2.6   29.1 : 27.7
-//   K = 768, N = 256   23.3 : 49.3   37.3 : 40.7   2.6 : 2.5   34.2 : 30.1
-// Rows with values that have no split (infinities, NaN, values above bf16's largest) give what
+//   K =  64, N =  64   3.5 : 14.6   2.6 : 12.2   3.1 : 2.5   3.8 : 11.0
+//   K = 128, N = 128   3.7 : 20.2   2.3 : 16.0   3.2 : 2.5   4.0 : 15.9
+//   K = 384, N = 128   5.0 : 35.0   2.2 : 28.9   3.4 : 2.6   5.6 : 26.6
+//   K = 640, N = 128   7.2 : 45.1   2.8 : 34.6   3.6 : 2.5   8.2 : 34.5
+//   K = 768, N = 256   7.6 : 49.9   3.1 : 40.9   3.4 : 2.5   8.9 : 37.3
+// and no mean loss (its part along the results is below 0.1 in every random case).  Times, us: 28672 x
+// 128 x 384 36.0 : 80.1, 20480 x 384 x 128 37.2 : 69.9.  (Terms of each value's own 8 bits, six
+// products, the steps round three accumulators of x0 w0: 45.2 and 36.5 us; mean loss 1.8 at K = 64,
+// 9.5 at 384; total energies of 1000 to 3000 atoms of 128 channels 1.6-1.9e-7 off, now 3-5e-8.)
+// Rows with values that have no split (infinities, NaN, finite ones from 2^112 on) give what
 // chains of FMAs give: see plain_tile.  The weights all have one (checked where they are laid out).
 // Eight warps read the float32 rows where the producers left them (the row map of the SIMT
 // GEMM) and split them into the swizzled operand layout, a k-block ahead in registers; one
@@ -229,7 +235,8 @@ __global__ void __launch_bounds__(128, 1) k_umma_gemm(const __grid_constant__ Um
 struct F32SegDev {
   CUtensorMap tb;
   GemmSeg g;
-  int NT, tiles_m, tiles_n, mains, stages;  // mains: accumulators of x0 w0
+  const float* scale;  // F32Weights::scale
+  int NT, tiles_m, tiles_n, stages;
 };
 struct F32GroupDev {
   F32SegDev s[4];
@@ -238,17 +245,22 @@ struct F32GroupDev {
 };
 constexpr int kF32Split = 256;                // threads that split X and store Y
 constexpr int kF32Threads = kF32Split + 32;   // and a warp whose first lane issues TMA and MMAs
-constexpr int kF32Mains = 3;          // accumulators of x0 w0
 constexpr uint32_t kATerm = kTileM * kBoxK * 2;  // bytes of one X term of a k-block
 
+// 1.5 2^23 grid steps of a row's k-block, m the bits of its largest |x| (a NaN from 2^112 on)
+__device__ __forceinline__ float grid_magic(uint32_t m) {
+  m = min(m & 0x7f800000u, 238u << 23);
+  return __uint_as_float((m + (17u << 23)) | 0x400000u);
+}
+__device__ __forceinline__ float to_grid(float x, float magic) { return __fsub_rn(__fadd_rn(x, magic), magic); }
 __device__ __forceinline__ float bf16_lo(uint32_t p) { return __uint_as_float(p << 16); }
 __device__ __forceinline__ float bf16_hi(uint32_t p) { return __uint_as_float(p & 0xffff0000u); }
 __device__ __forceinline__ uint32_t bf16_pair(float a, float b) {
   const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
   return *reinterpret_cast<const uint32_t*>(&v);
 }
-// A tile with a value that has no split (an infinity, a NaN, or a finite value above bf16's
-// largest, whose leading term is infinite): its sums as the SIMT kernel forms them, chains of
+// A tile with a value that has no split (an infinity, a NaN, or a finite value from 2^112 on,
+// whose grid has no magic number): its sums as the SIMT kernel forms them, chains of
 // FMAs over k on the float32 weights.
 __device__ __forceinline__ void plain_tile(const GemmSeg& g, const long* x_row, int m0, int n0, int NT, int tid) {
   for (int t = tid; t < kTileM * NT; t += kF32Split) {
@@ -261,8 +273,8 @@ __device__ __forceinline__ void plain_tile(const GemmSeg& g, const long* x_row, 
   }
 }
 
-// Tiles of 64 columns up to K = 128: two CTAs per SM with one stage each (72 KB, 256 TMEM columns)
-// overlap one's splitting and stores with the other's MMAs; otherwise one CTA with two stages.
+// Up to K = 128 two CTAs per SM with one stage each (96 KB, 256 TMEM columns) overlap one's
+// splitting and stores with the other's MMAs; above, one CTA with two stages.
 __global__ void __launch_bounds__(kF32Threads, 2) k_umma_f32(const __grid_constant__ F32GroupDev grp,
                                                              unsigned* status) {
   pdl_begin();
@@ -280,7 +292,7 @@ __global__ void __launch_bounds__(kF32Threads, 2) k_umma_f32(const __grid_consta
   const uint32_t b_bytes = static_cast<uint32_t>(NT) * kBoxK * 2, stage_bytes = 3 * kATerm + 3 * b_bytes;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int m0 = tile_m * kTileM, n0 = tile_n * NT;
-  const uint32_t used = static_cast<uint32_t>((seg.mains + 1) * NT);
+  const uint32_t used = static_cast<uint32_t>(2 * NT);
   const uint32_t ncols = used <= 64 ? 64u : (used <= 128 ? 128u : (used <= 256 ? 256u : 512u));
   if (tid == 0) {
     for (int s = 0; s < S; ++s) {
@@ -308,9 +320,10 @@ __global__ void __launch_bounds__(kF32Threads, 2) k_umma_f32(const __grid_consta
   // a k-block row is 16 float4: a warp reads two rows at a time, 16 rows in all; this thread
   // has float4 c of rows warp * 16 + lane / 16 + 2 j
   const int c = lane & 15, row0 = warp * 16 + (lane >> 4);
-  float4 v[8];
+  float4 v[8], sc;
   auto load = [&](int kb) {
     const int k = kb * kBoxK + 4 * c;
+    sc = __ldg(reinterpret_cast<const float4*>(seg.scale + k));
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       const long o = x_row[row0 + 2 * j];
@@ -334,13 +347,20 @@ __global__ void __launch_bounds__(kF32Threads, 2) k_umma_f32(const __grid_consta
       for (int j = 0; j < 8; ++j) {
         const int row = row0 + 2 * j;
         uint8_t* a = st + row * 128 + ((c >> 1) ^ (row & 7)) * 16 + (c & 1) * 8;
-        float4 x = v[j];
+        float4 x = make_float4(v[j].x * sc.x, v[j].y * sc.y, v[j].z * sc.z, v[j].w * sc.w);
+        uint32_t big = max(max(__float_as_uint(fabsf(x.x)), __float_as_uint(fabsf(x.y))),
+                           max(__float_as_uint(fabsf(x.z)), __float_as_uint(fabsf(x.w))));
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) big = max(big, __shfl_xor_sync(0xffffffffu, big, o));
+        const float magic = grid_magic(big);
+        float4 y = make_float4(to_grid(x.x, magic), to_grid(x.y, magic), to_grid(x.z, magic), to_grid(x.w, magic));
 #pragma unroll
         for (int t = 0; t < 3; ++t) {
-          const uint2 w = make_uint2(bf16_pair(x.x, x.y), bf16_pair(x.z, x.w));
+          const uint2 w = make_uint2(bf16_pair(y.x, y.y), bf16_pair(y.z, y.w));
           *reinterpret_cast<uint2*>(a + t * kATerm) = w;
           if (t < 2)
             x = make_float4(x.x - bf16_lo(w.x), x.y - bf16_hi(w.x), x.z - bf16_lo(w.y), x.w - bf16_hi(w.y));
+          y = x;
         }
         low += (x.x + x.y) + (x.z + x.w);  // a value without a split: NaN from here on
       }
@@ -376,10 +396,11 @@ __global__ void __launch_bounds__(kF32Threads, 2) k_umma_f32(const __grid_consta
           sm100::umma_bf16(d, sm100::sdesc_sw128(x0 + xt * kATerm + k * 32),
                            sm100::sdesc_sw128(w0 + wt * b_bytes + k * 32), idesc, acc);
         };
-        const uint32_t corr = tmem + seg.mains * NT;
-        const int step = kb * (kBoxK / 16) + k;
-        mma(tmem + (step % seg.mains) * NT, 0, 0, step >= seg.mains ? 1u : 0u);
-        mma(corr, 0, 2, (kb | k) != 0 ? 1u : 0u);
+        const uint32_t corr = tmem + NT, more = (kb | k) != 0 ? 1u : 0u;
+        mma(tmem, 0, 0, more);
+        mma(corr, 1, 2, more);
+        mma(corr, 2, 1, 1u);
+        mma(corr, 0, 2, 1u);
         mma(corr, 2, 0, 1u);
         mma(corr, 1, 1, 1u);
         mma(corr, 0, 1, 1u);
@@ -416,12 +437,10 @@ __global__ void __launch_bounds__(kF32Threads, 2) k_umma_f32(const __grid_consta
     const uint32_t t0 = tmem + (static_cast<uint32_t>(quarter * 32) << 16);
     for (int c0 = (warp >> 2) * 32; c0 < NT; c0 += 64) {
       float a[32], b[32];
-      sm100::tmem_ld32(t0 + static_cast<uint32_t>(seg.mains * NT + c0), a);
-      for (int w = seg.mains - 1; w >= 0; --w) {
-        sm100::tmem_ld32(t0 + static_cast<uint32_t>(w * NT + c0), b);
+      sm100::tmem_ld32(t0 + static_cast<uint32_t>(c0), a);
+      sm100::tmem_ld32(t0 + static_cast<uint32_t>(NT + c0), b);
 #pragma unroll
-        for (int q = 0; q < 32; ++q) a[q] += b[q];
-      }
+      for (int q = 0; q < 32; ++q) a[q] += b[q];
 #pragma unroll
       for (int q = 0; q < 8; ++q)
         reinterpret_cast<float4*>(stg + lane * 32)[q ^ (lane & 7)] =
@@ -499,8 +518,8 @@ bool umma_supported(int K, int NT, int terms) {
 
 namespace {
 
-// ring stages (see k_umma_f32; two also where one CTA's TMEM columns are more than half)
-int f32_stages(int K, int NT) { return K > 2 * kBoxK || (kF32Mains + 1) * NT > 256 ? 2 : 1; }
+// ring stages (see k_umma_f32)
+int f32_stages(int K) { return K > 2 * kBoxK ? 2 : 1; }
 // N-tile: the widest of 128, 96, 64, 32 that divides the columns
 int f32_tile_n(int ncols) {
   for (int nt : {128, 96, 64})
@@ -512,11 +531,14 @@ size_t f32_smem_bytes(int NT, int stages) {
 }
 }  // namespace
 
-bool umma_f32_supported(int K, int ncols) { return K > 0 && K % 32 == 0 && ncols > 0 && ncols % 32 == 0; }
+// (K: the leading products' sums stay exact)
+bool umma_f32_supported(int K, int ncols) {
+  return K > 0 && K <= 1024 && K % 32 == 0 && ncols > 0 && ncols % 32 == 0;
+}
 
 int umma_f32_kp(int K) { return (K + kBoxK - 1) / kBoxK * kBoxK; }
 
-void launch_umma_f32(const GemmBatch& b, const __nv_bfloat16* const* B, unsigned* status, cudaStream_t s,
+void launch_umma_f32(const GemmBatch& b, const F32Weights* W, unsigned* status, cudaStream_t s,
                      bool test_timeout) {
   F32GroupDev grp;
   std::memset(&grp, 0, sizeof(grp));
@@ -532,9 +554,9 @@ void launch_umma_f32(const GemmBatch& b, const __nv_bfloat16* const* B, unsigned
     F32SegDev& d = grp.s[used++];
     d.g = g;
     d.NT = f32_tile_n(g.ncols);
-    d.mains = kF32Mains;
-    d.stages = f32_stages(g.K, d.NT);
-    d.tb = make_map(B[q], g.ncols, 3 * umma_f32_kp(g.K), d.NT);
+    d.stages = f32_stages(g.K);
+    d.scale = W[q].scale;
+    d.tb = make_map(W[q].terms, g.ncols, 3 * umma_f32_kp(g.K), d.NT);
     d.tiles_m = (g.rows + kTileM - 1) / kTileM;
     d.tiles_n = g.ncols / d.NT;
     gx = std::max(gx, static_cast<long>(d.tiles_m) * d.tiles_n);

@@ -114,11 +114,16 @@ struct UmmaGemm {
 // wait gives up after 2 ms: the launch records a timeout in *status and writes nothing)
 void launch_umma_gemms(const UmmaGemm* g, int n, unsigned* status, cudaStream_t s, bool test_timeout = false);
 
-// The batch's GEMMs in float32 on the tensor cores; B[q]: segment q's weights as three bf16
-// terms, [ncols][3][umma_f32_kp(K)], zero behind K (GemmSeg::B serves rows that have no such split).
+// The batch's GEMMs in float32 on the tensor cores; W[q]: segment q's weights, the columns k scaled
+// by 1 / scale[k], as three bf16 terms [ncols][3][umma_f32_kp(K)], zero behind K, and scale
+// [umma_f32_kp(K)], powers of two (GemmSeg::B serves rows that have no such split).
+struct F32Weights {
+  const __nv_bfloat16* terms;
+  const float* scale;
+};
 bool umma_f32_supported(int K, int ncols);
 int umma_f32_kp(int K);
-void launch_umma_f32(const GemmBatch& b, const __nv_bfloat16* const* B, unsigned* status, cudaStream_t s,
+void launch_umma_f32(const GemmBatch& b, const F32Weights* W, unsigned* status, cudaStream_t s,
                      bool test_timeout = false);
 
 // k_md.cu
