@@ -384,7 +384,7 @@ def time_md(eng, pos, species, masses, L, vel, args, dist, estream):
 
 # (workload, stage) -> (DRAM bytes per launch, the ncu summary it comes from)
 NCU_TRAFFIC = {
-    ("fp32_4096", "layer1_rev"): (165.6e6 + 11.5e6, "profiles/layer1_rev_fp32_4096.md (ncu --set full, 1 launch)"),
+    ("fp32_4096", "layer1_rev"): (161.4e6 + 17.6e6, "profiles/layer1_rev_fp32_4096.md (ncu, 1 launch, a box of this shape)"),
 }
 
 ATOM_KERNELS = ("layer0_fwd", "contract0_rev", "layer0_rev", "layer1_fwd", "layer1_rev", "node_tail")
@@ -394,7 +394,7 @@ def schedule_of(eng):
     """The autotuned schedule the engine ran with: per-atom kernels on persistent grids, GEMM tiles."""
     mask = eng.get_option("persistent")
     out = {"persistent_kernels": [k for b, k in enumerate(ATOM_KERNELS) if mask >> b & 1],
-           "species_order": eng.get_option("species_order"), "l2_channel_slices": eng.get_option("l2_split")}
+           "species_order": eng.get_option("species_order")}
     if eng.precision == "bfloat16":
         out["gemm"] = eng.gemm_schedule()
     return out

@@ -234,7 +234,9 @@ int smx_stage_times(smx_engine* eng, double* out_ms, int cap);
  * box_lengths[3] of an orthorhombic periodic cell (NULL = non-periodic).  Builds the
  * full neighbour list (r < r_cut) on the GPU, evaluates, and returns the total energy,
  * optionally node_energies[n], atomic forces[3n] and the virial[9] W_ab = sum_e xyz_a f_b
- * (row-major, float64).  Host pointers; synchronous. */
+ * (row-major, float64).  Host pointers; synchronous.  The engine keeps the call's device
+ * buffers for the next one (about 190 bytes per neighbour-list entry, up to 1 GiB) until it is
+ * destroyed or needs the memory itself. */
 int smx_compute_atoms(smx_engine* eng, int n_atoms, const double* positions, const int* species,
                       const double* box_lengths, double* energy, double* node_energies, double* forces,
                       double* virial);

@@ -9,7 +9,7 @@
 // block: no block barriers, all per-channel arithmetic on channel pairs with the packed FMA,
 // and the next edge's cubics loaded into the registers that this edge's have left.  What
 // bounds them is the L2 gather of the folded spline rows, 8 KB per edge at 128 channels
-// (0.09 ms for 213k edges at the 19.6 TB/s of a plain gather), and of the contraction's
+// (0.08 ms for 213k edges at the 21.9 TB/s of a plain gather), and of the contraction's
 // coefficients, 0.2 MB per node.  Against a block of two warp groups per node whose sums met
 // in shared memory, five-and-forty scalar FMAs per edge and channel for the force and
 // polynomials with the products of pairs in registers (255 of them): 4096 atoms, 128

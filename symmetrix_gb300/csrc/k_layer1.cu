@@ -11,7 +11,7 @@
 // molecule in a batch gives the bits that it gives alone.
 //
 // What bounds it: the L2 gather of the spline rows, 20 KB per edge at L_max = 1 and 128
-// channels, which a plain gather kernel of the same rows runs at 19.6 TB/s (0.22 ms for 213k
+// channels, which a plain gather kernel of as many rows runs at 21.9 TB/s (0.20 ms for 213k
 // edges).  One block of C threads per node, no prefetch, all paths and a table walk for the
 // Clebsch-Gordan rows took 0.373 ms on the 4096-atom box (213k edges), this form 0.250 ms;
 // L_max = 2, 2197 atoms, 178k edges 0.816 -> 0.435 ms; 64 atoms of 32 channels 37 -> 14.5 us.
@@ -394,7 +394,8 @@ void launch_layer1_fwd(const DevModel& m, const EdgeIn& in, const float* H1, flo
 }
 
 // resident blocks per SM of the persistent layer-1 kernels at this model's launch shapes
-// (DEPTH 2 runs where its items are fewer than this grid)
+// (the forward's at DEPTH 1; at DEPTH 2, up to deep_items items, 8 of the blocks are resident and
+// the others of the grid find few items left)
 void layer1_residency(const DevModel& m, int* per_sm) {
   dispatch_layer1(m, [&](auto lc, auto cc, auto nc) {
     constexpr int LM = decltype(lc)::value, CT = decltype(cc)::value;
